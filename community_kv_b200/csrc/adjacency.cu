@@ -10,15 +10,27 @@
 //
 // The reference sorts with torch.unique and adds with scatter_add_.  Here: the raw edges
 // are enumerated in the reference's order (all direct edges, then all co-attention edges),
-// sorted by their 64-bit key with a stable least-significant-digit radix sort (8 bits per
-// pass, only as many passes as the vertex count needs), and every run of equal keys is
-// summed front to back by one thread - a stable sort keeps equal keys in enumeration
-// order, so each weight is the same sequence of fp32 additions a sequential scatter-add
-// performs: the result is bit-exact and independent of scheduling.  HBM-bound integer work:
-// five passes over 12 bytes per raw edge; nothing here is shaped for the tensor cores.
+// sorted with a stable least-significant-digit radix sort (8 bits per pass), and every run
+// of equal keys is summed front to back by one thread - a stable sort keeps equal keys in
+// enumeration order, so each weight is the same sequence of fp32 additions a sequential
+// scatter-add performs: the result is bit-exact and independent of scheduling.
+//
+// What bounds it is the traffic of the sort, so it carries as few bytes as often as it can:
+//   * both ends of an edge lie in one graph, so the key is (graph, min, max) with the
+//     positions inside the graph: 31 bits and four passes for 32 graphs of 8192 positions
+//     instead of 36 bits and five, and a 4-byte key wherever it fits (else 8 bytes);
+//   * the raw edges are never written in enumeration order: the first pass makes them from
+//     the rows (16 bytes of neighbours and scores per 44 edges of 8 bytes);
+//   * a pass is one kernel: every tile publishes its digit counts and sums its
+//     predecessors' (decoupled look-back), and items leave in digit order through shared
+//     memory, so that a tile writes runs of consecutive items.
+// 32 graphs of 8192 positions, 11.5 M raw edges: 0.61 ms (105-115 us a pass, 85 us the runs);
+// five passes over enumerated 12-byte items with separate count and scan kernels took 1.1 ms.
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <type_traits>
 
 #include "../../include/ckv_b200.h"
 
@@ -26,15 +38,97 @@ namespace ckv {
 namespace {
 
 constexpr int kSortThreads = 256;
-constexpr int kSortItems = 8;                          // keys per thread and tile
-constexpr int kSortTile = kSortThreads * kSortItems;   // 2048
-constexpr int kScanThreads = 1024;
-constexpr int kScanItems = 4;
-constexpr int kScanTile = kScanThreads * kScanItems;   // 4096
-constexpr uint64_t kInvalidKey = ~0ull;
+constexpr int kSortWarps = kSortThreads / 32;
+constexpr int kDigits = 256;
+constexpr int kMaxPasses = 8;
+constexpr int kNarrowItems = 16;  // items per thread with 4-byte keys; half of it with 8-byte keys
 
-// ---- device-wide exclusive scan of uint32 (three small launches) ----
-__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t value, uint32_t* warp_total, uint32_t* total) {
+template <typename Key>
+struct Sort {
+  static constexpr int kItems = sizeof(Key) == 4 ? kNarrowItems : kNarrowItems / 2;
+  static constexpr int kTile = kSortThreads * kItems;
+};
+
+template <typename Key>
+struct Runs {
+  static constexpr int kItems = sizeof(Key) == 4 ? 8 : 4;
+  static constexpr int kTile = kSortThreads * kItems;
+};
+
+// The rows that the raw edges are made from.
+struct EdgeRows {
+  const int32_t* indices;     // [lines, kappa]
+  const float* scores;
+  const int64_t* positions;   // [lines]
+  uint32_t rows;              // lines per graph
+  uint32_t direct;            // direct edges in all: lines * kappa
+  uint32_t raw;               // raw edges in all
+  int kappa;
+  int seq_len;
+  int position_bits;          // a key is (graph, min, max): graph << 2 bits | min << bits | max
+  float direct_scale;
+  float co_scale;
+};
+
+template <typename Key>
+__device__ __forceinline__ Key edge_key(const EdgeRows& e, uint32_t graph, uint32_t a, uint32_t b) {
+  const uint32_t low = min(a, b);
+  const uint32_t high = max(a, b);
+  return (static_cast<Key>(graph) << (2 * e.position_bits)) | (static_cast<Key>(low) << e.position_bits) | high;
+}
+__device__ __forceinline__ bool in_graph(const EdgeRows& e, int64_t position) {
+  return static_cast<uint64_t>(position) < static_cast<uint64_t>(e.seq_len);
+}
+
+// ---- digit totals of every pass ----
+// One thread per line: it has the line's neighbours at hand and needs no index arithmetic.
+// The top digit (graph and the leading bits of min) is the same for most edges of a line, so
+// a thread counts runs of it in a register; the other digits go to shared memory one by one.
+template <typename Key>
+__global__ void __launch_bounds__(kSortThreads) digit_totals_kernel(const EdgeRows e, int passes, uint32_t* totals) {
+  __shared__ uint32_t count[kMaxPasses * kDigits];
+  for (int i = threadIdx.x; i < passes * kDigits; i += kSortThreads) count[i] = 0u;
+  __syncthreads();
+  const uint32_t lines = e.direct / e.kappa;
+  const uint32_t line = blockIdx.x * kSortThreads + threadIdx.x;
+  const int top = passes - 1;
+  uint32_t run_digit = 0u, run = 0u;
+  auto add = [&](Key key) {
+    for (int p = 0; p < top; ++p) {
+      atomicAdd(&count[p * kDigits + (static_cast<uint32_t>(key >> (8 * p)) & 255u)], 1u);
+    }
+    const uint32_t digit = static_cast<uint32_t>(key >> (8 * top)) & 255u;
+    if (digit != run_digit) {
+      if (run > 0u) atomicAdd(&count[top * kDigits + run_digit], run);
+      run_digit = digit;
+      run = 0u;
+    }
+    ++run;
+  };
+  if (line < lines) {
+    const uint32_t graph = line / e.rows;
+    const int32_t* own = e.indices + static_cast<int64_t>(line) * e.kappa;
+    const int64_t position = e.positions[line];
+    const bool co = e.raw > e.direct;
+    for (int a = 0; a < e.kappa; ++a) {
+      const int32_t u = own[a];
+      if (!in_graph(e, u)) continue;
+      if (in_graph(e, position)) add(edge_key<Key>(e, graph, u, static_cast<uint32_t>(position)));
+      for (int b = a; co && b < e.kappa; ++b) {
+        const int32_t v = own[b];
+        if (in_graph(e, v)) add(edge_key<Key>(e, graph, u, v));
+      }
+    }
+    if (run > 0u) atomicAdd(&count[top * kDigits + run_digit], run);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < passes * kDigits; i += kSortThreads) {
+    if (count[i] > 0u) atomicAdd(&totals[i], count[i]);
+  }
+}
+
+// Exclusive prefix over the 256 threads of a block; `warp_total` holds one word per warp.
+__device__ __forceinline__ uint32_t block_prefix(uint32_t value, uint32_t* warp_total, uint32_t* total) {
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   uint32_t inclusive = value;
@@ -45,265 +139,514 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t value, uint32_
   }
   if (lane == 31) warp_total[warp] = inclusive;
   __syncthreads();
-  if (warp == 0) {
-    uint32_t running = lane < (blockDim.x >> 5) ? warp_total[lane] : 0u;
+  uint32_t before = 0u, all = 0u;
 #pragma unroll
-    for (int delta = 1; delta < 32; delta <<= 1) {
-      const uint32_t other = __shfl_up_sync(0xffffffffu, running, delta);
-      if (lane >= delta) running += other;
-    }
-    warp_total[lane] = running;
+  for (int w = 0; w < kSortWarps; ++w) {
+    before += w < warp ? warp_total[w] : 0u;
+    all += warp_total[w];
   }
-  __syncthreads();
-  const uint32_t before = warp > 0 ? warp_total[warp - 1] : 0u;
-  if (total != nullptr) *total = warp_total[(blockDim.x >> 5) - 1];
-  __syncthreads();
+  *total = all;
   return before + inclusive - value;
 }
 
-__global__ void __launch_bounds__(kScanThreads) scan_tiles_kernel(const uint32_t* in, uint32_t* out, int64_t n,
-                                                                  uint32_t* tile_total) {
-  __shared__ uint32_t warp_total[32];
-  const int64_t base = static_cast<int64_t>(blockIdx.x) * kScanTile + threadIdx.x * kScanItems;
-  uint32_t item[kScanItems];
-  uint32_t sum = 0;
-#pragma unroll
-  for (int i = 0; i < kScanItems; ++i) {
-    item[i] = base + i < n ? in[base + i] : 0u;
-    sum += item[i];
-  }
+// One block per pass: digit totals -> where each digit begins, and the number of valid edges.
+__global__ void __launch_bounds__(kSortThreads) digit_bases_kernel(uint32_t* totals, uint32_t* valid) {
+  __shared__ uint32_t warp_total[kSortWarps];
+  uint32_t* row = totals + blockIdx.x * kDigits;
   uint32_t total;
-  uint32_t prefix = block_exclusive_scan(sum, warp_total, &total);
+  const uint32_t prefix = block_prefix(row[threadIdx.x], warp_total, &total);
+  row[threadIdx.x] = prefix;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *valid = total;
+}
+
+// ---- decoupled look-back ----
+// A tile publishes its count with kPartial, later the sum over all tiles up to it with kComplete;
+// flag and value are one 64-bit word.  Tiles take their numbers from a counter when they start, so
+// every predecessor is already running and a wait ends; the waits are bounded all the same, and one
+// that runs out is reported and yields a wrong sum (the stores that use it check their bounds).
+constexpr uint64_t kPartial = 1ull << 62;
+constexpr uint64_t kComplete = 2ull << 62;
+constexpr uint64_t kValueMask = (1ull << 62) - 1;
+constexpr uint32_t kLookPolls = 1u << 22;
+
+__device__ __forceinline__ uint64_t look(const uint64_t* word) {
+  uint64_t value;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(value) : "l"(word) : "memory");
+  return value;
+}
+__device__ __forceinline__ void publish(uint64_t* word, uint64_t value) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(word), "l"(value) : "memory");
+}
+
+// One thread, one chain: the sum over the tiles in front of `tile`; words of a chain are `stride` apart.
+// When a grid starts, a tile finds hundreds of partial words in front of it, so a thread reads
+// kLookWords of them at a time.
+constexpr int kLookWords = 8;
+
+__device__ __forceinline__ uint32_t look_back(const uint64_t* words, uint32_t tile, uint32_t stride, uint32_t* fault) {
+  uint64_t sum = 0;
+  uint32_t polls = 0;
+  int64_t t = static_cast<int64_t>(tile) - 1;
+  bool done = t < 0;
+  while (!done) {
+    uint64_t word[kLookWords];
 #pragma unroll
-  for (int i = 0; i < kScanItems; ++i) {
-    if (base + i < n) out[base + i] = prefix;
-    prefix += item[i];
-  }
-  if (threadIdx.x == 0) tile_total[blockIdx.x] = total;
-}
-
-// One CTA: exclusive scan of the tile totals in place, any length.
-__global__ void __launch_bounds__(kScanThreads) scan_totals_kernel(uint32_t* tile_total, int64_t tiles) {
-  __shared__ uint32_t warp_total[32];
-  __shared__ uint32_t carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (int64_t base = 0; base < tiles; base += kScanThreads) {
-    const int64_t index = base + threadIdx.x;
-    const uint32_t value = index < tiles ? tile_total[index] : 0u;
-    uint32_t total;
-    const uint32_t prefix = block_exclusive_scan(value, warp_total, &total);
-    if (index < tiles) tile_total[index] = carry + prefix;
-    __syncthreads();
-    if (threadIdx.x == 0) carry += total;
-    __syncthreads();
-  }
-}
-
-__global__ void __launch_bounds__(kScanThreads) scan_add_kernel(uint32_t* out, int64_t n, const uint32_t* tile_total) {
-  const int64_t base = static_cast<int64_t>(blockIdx.x) * kScanTile + threadIdx.x * kScanItems;
-  const uint32_t add = tile_total[blockIdx.x];
+    for (int i = 0; i < kLookWords; ++i) word[i] = t - i >= 0 ? look(words + (t - i) * stride) : kComplete;
+    const int64_t from = t;
 #pragma unroll
-  for (int i = 0; i < kScanItems; ++i) {
-    if (base + i < n) out[base + i] += add;
-  }
-}
-
-cudaError_t exclusive_scan(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* tile_total, cudaStream_t stream) {
-  const int64_t tiles = (n + kScanTile - 1) / kScanTile;
-  scan_tiles_kernel<<<static_cast<unsigned>(tiles), kScanThreads, 0, stream>>>(in, out, n, tile_total);
-  scan_totals_kernel<<<1, kScanThreads, 0, stream>>>(tile_total, tiles);
-  scan_add_kernel<<<static_cast<unsigned>(tiles), kScanThreads, 0, stream>>>(out, n, tile_total);
-  return cudaGetLastError();
-}
-
-// ---- raw edges in the reference's enumeration order ----
-// index < direct: (graph, row, k); else (graph, row, pair) with pairs in row-major upper-triangular order
-__global__ void __launch_bounds__(256) edge_keys_kernel(const int32_t* topk_indices, const float* topk_scores,
-                                                        const int64_t* query_positions, int64_t rows, int kappa,
-                                                        int seq_len, int64_t vertices, float direct_scale,
-                                                        float co_scale, int64_t direct, int64_t raw,
-                                                        uint64_t* keys, float* weights) {
-  const int pairs = kappa * (kappa + 1) / 2;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < raw;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    uint64_t key = kInvalidKey;
-    float weight = 0.f;
-    if (i < direct) {
-      const int64_t line = i / kappa;  // graph * rows + row
-      const int64_t graph = line / rows;
-      const int32_t neighbour = topk_indices[i];
-      if (neighbour >= 0 && neighbour < seq_len) {
-        const int64_t a = query_positions[line] + graph * seq_len;
-        const int64_t b = static_cast<int64_t>(neighbour) + graph * seq_len;
-        key = static_cast<uint64_t>((a < b ? a : b) * vertices + (a < b ? b : a));
-        weight = __fmul_rn(topk_scores[i], direct_scale);
-      }
-    } else {
-      const int64_t j = i - direct;
-      const int64_t line = j / pairs;
-      int pair = static_cast<int>(j - line * pairs);
-      int first = 0;
-      while (pair >= kappa - first) {  // row `first` of the upper triangle holds kappa - first pairs
-        pair -= kappa - first;
-        ++first;
-      }
-      const int second = first + pair;
-      const int64_t graph = line / rows;
-      const int32_t u = topk_indices[line * kappa + first];
-      const int32_t v = topk_indices[line * kappa + second];
-      if (u >= 0 && u < seq_len && v >= 0 && v < seq_len) {
-        const int64_t a = static_cast<int64_t>(u) + graph * seq_len;
-        const int64_t b = static_cast<int64_t>(v) + graph * seq_len;
-        key = static_cast<uint64_t>((a < b ? a : b) * vertices + (a < b ? b : a));
-        weight = __fmul_rn(__fmul_rn(topk_scores[line * kappa + first], topk_scores[line * kappa + second]), co_scale);
+    for (int i = 0; i < kLookWords; ++i) {
+      if (!done && from - i == t && word[i] != 0ull) {
+        sum += word[i] & kValueMask;
+        done = (word[i] & kComplete) != 0ull;
+        --t;
       }
     }
-    keys[i] = key;
-    weights[i] = weight;
-  }
-}
-
-// ---- one stable radix pass: digit = (key >> shift) & 255 ----
-// Tile t covers items [t * 2048, (t + 1) * 2048); item order inside a tile is round-major
-// (round r holds items r * 256 .. r * 256 + 255), which both kernels below walk in order.
-__global__ void __launch_bounds__(kSortThreads) radix_count_kernel(const uint64_t* keys, int64_t n, int shift,
-                                                                   int64_t tiles, uint32_t* table) {
-  __shared__ uint32_t count[256];
-  count[threadIdx.x] = 0;
-  __syncthreads();
-  const int64_t base = static_cast<int64_t>(blockIdx.x) * kSortTile;
-#pragma unroll
-  for (int r = 0; r < kSortItems; ++r) {
-    const int64_t index = base + r * kSortThreads + threadIdx.x;
-    if (index < n) {
-      atomicAdd(&count[(keys[index] >> shift) & 255u], 1u);
+    if (!done && t == from && ++polls > kLookPolls) {
+      atomicOr(fault, 1u);
+      done = true;
     }
   }
-  __syncthreads();
-  table[static_cast<int64_t>(threadIdx.x) * tiles + blockIdx.x] = count[threadIdx.x];  // digit-major
+  return static_cast<uint32_t>(sum);
 }
 
-__global__ void __launch_bounds__(kSortThreads) radix_scatter_kernel(const uint64_t* keys, const float* weights,
-                                                                     int64_t n, int shift, int64_t tiles,
-                                                                     const uint32_t* table, uint64_t* keys_out,
-                                                                     float* weights_out) {
-  __shared__ uint32_t digit_base[256];                     // where the tile's next item of a digit goes
-  __shared__ uint32_t round_base[256];                     // the same, at the start of the current round
-  __shared__ uint16_t warp_count[kSortThreads / 32][256];  // this sorting pass, per warp and digit
+// ---- one stable radix pass: digit = byte `pass` of the key ----
+// Item order inside a tile: warp w holds items [32 kItems w, 32 kItems (w + 1)), round i of the
+// warp 32 consecutive ones.  An item's rank among the tile's items of its digit is the count of
+// the warps before it, the rounds before it and the lanes before it.  The pass is bound by its
+// instructions once the traffic is down to 16 bytes per item, so the lanes of a warp that share a
+// digit find one another by OR-ing their lane bits into a word of shared memory (about 15
+// instructions whatever the digit's width; eight ballots take 40), and a full tile runs without
+// bounds checks.
+template <typename Key>
+__device__ __forceinline__ uint32_t digit_of(Key key, int pass) {
+  if constexpr (sizeof(Key) == 4) {
+    return __byte_perm(static_cast<uint32_t>(key), 0u, 0x4440u | static_cast<uint32_t>(pass));
+  } else {
+    return static_cast<uint32_t>(key >> (8 * pass)) & 255u;
+  }
+}
+
+template <typename Key, int kKappa, bool kFirst>
+__global__ void __launch_bounds__(kSortThreads, 3)
+    radix_pass_kernel(const EdgeRows e, const Key* keys, const float* weights, Key* keys_out, float* weights_out,
+                      const uint32_t* digit_base, const uint32_t* valid, int pass, uint64_t* words, uint32_t* ticket,
+                      uint32_t* fault) {
+  constexpr int kItems = Sort<Key>::kItems;
+  constexpr int kTile = Sort<Key>::kTile;
+  // counts per warp and digit, and the lane masks; the items in digit order reuse the masks' room
+  __shared__ uint32_t warp_count[kSortWarps][kDigits];
+  union Stage {
+    uint32_t lanes[kSortWarps][kDigits];
+    struct {
+      Key key[kTile];
+      float weight[kTile];
+    } out;
+  };
+  __shared__ Stage stage;
+  __shared__ uint32_t target_base[kDigits];
+  __shared__ uint32_t warp_total[kSortWarps];
+  __shared__ uint32_t tile_s;
+  __shared__ uint16_t pair_slots[kFirst ? 2080 : 1];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
-  digit_base[threadIdx.x] = table[static_cast<int64_t>(threadIdx.x) * tiles + blockIdx.x];
-  const int64_t base = static_cast<int64_t>(blockIdx.x) * kSortTile;
-  for (int r = 0; r < kSortItems; ++r) {
+  if (threadIdx.x == 0) tile_s = atomicAdd(ticket, 1u);
 #pragma unroll
-    for (int w = 0; w < kSortThreads / 32; ++w) {
-      warp_count[w][threadIdx.x] = 0;
-    }
-    __syncthreads();
-    const int64_t index = base + r * kSortThreads + threadIdx.x;
-    const bool live = index < n;
-    const uint64_t key = live ? keys[index] : 0ull;
-    const float weight = live ? weights[index] : 0.f;
-    const uint32_t digit = static_cast<uint32_t>(key >> shift) & 255u;
-    // lanes of this warp that hold the same digit (eight ballots instead of a match instruction)
-    unsigned peers = __ballot_sync(0xffffffffu, live);
-#pragma unroll
-    for (int bit = 0; bit < 8; ++bit) {
-      const unsigned votes = __ballot_sync(0xffffffffu, (digit >> bit) & 1u);
-      peers &= ((digit >> bit) & 1u) ? votes : ~votes;
-    }
-    const uint32_t rank_in_warp = __popc(peers & ((1u << lane) - 1u));
-    if (live && rank_in_warp == 0) {
-      warp_count[warp][digit] = static_cast<uint16_t>(__popc(peers));
-    }
-    __syncthreads();
-    {
-      // thread d: exclusive prefix of digit d's counts over the warps (warp order = item order)
-      const int d = threadIdx.x;
-      uint32_t sum = 0;
-#pragma unroll
-      for (int w = 0; w < kSortThreads / 32; ++w) {
-        const uint32_t count = warp_count[w][d];
-        warp_count[w][d] = static_cast<uint16_t>(sum);
-        sum += count;
+  for (int w = 0; w < kSortWarps; ++w) {
+    warp_count[w][threadIdx.x] = 0u;
+    stage.lanes[w][threadIdx.x] = 0u;
+  }
+  const uint32_t kappa = kKappa > 0 ? kKappa : static_cast<uint32_t>(e.kappa);
+  const uint32_t pairs = kappa * (kappa + 1) / 2;
+  if constexpr (kFirst) {
+    // pair number -> its two slots, row-major over the upper triangle
+    for (uint32_t p = threadIdx.x; p < pairs; p += kSortThreads) {
+      uint32_t first = 0, rest = p;
+      while (rest >= kappa - first) {
+        rest -= kappa - first;
+        ++first;
       }
-      round_base[d] = digit_base[d];
-      digit_base[d] += sum;
+      pair_slots[p] = static_cast<uint16_t>(first | ((first + rest) << 8));
+    }
+  }
+  __syncthreads();
+  const uint32_t tile = tile_s;
+  const uint32_t n = kFirst ? e.raw : *valid;
+  const uint64_t base = static_cast<uint64_t>(tile) * kTile;
+  if (base >= n) return;
+  const uint32_t item0 = static_cast<uint32_t>(base) + warp * (32 * kItems) + lane;
+  uint32_t* const my_count = warp_count[warp];
+  uint32_t* const my_lanes = stage.lanes[warp];
+
+  auto work = [&](auto full) {
+    constexpr bool kFull = decltype(full)::value;  // every item of the tile takes part
+    Key key[kItems];
+    float weight[kItems];
+    uint32_t live = 0u;  // bit i: item i takes part
+    if constexpr (!kFirst) {
+#pragma unroll
+      for (int i = 0; i < kItems; ++i) {
+        const bool here = kFull || item0 + i * 32 < n;
+        key[i] = here ? keys[item0 + i * 32] : 0;  // the weights follow: nothing before the look-back needs them
+        live |= (here ? 1u : 0u) << i;
+      }
+    } else {
+      uint32_t graph = 0u, next_graph = 0u;  // `next_graph`: first line of the graph after it
+      bool placed = false;
+      auto graph_of = [&](uint32_t line) {
+        if (!placed) {
+          graph = line / e.rows;
+          next_graph = (graph + 1u) * e.rows;
+          placed = true;
+        }
+        while (line >= next_graph) {
+          ++graph;
+          next_graph += e.rows;
+        }
+        return graph;
+      };
+#pragma unroll
+      for (int i = 0; i < kItems; ++i) {
+        const uint32_t index = item0 + i * 32;
+        key[i] = 0;
+        weight[i] = 0.f;
+        if (index >= n || index < item0) continue;
+        if (index < e.direct) {
+          const uint32_t line = index / kappa;
+          const int32_t u = e.indices[index];
+          const int64_t position = e.positions[line];
+          if (in_graph(e, u) && in_graph(e, position)) {
+            key[i] = edge_key<Key>(e, graph_of(line), u, static_cast<uint32_t>(position));
+            weight[i] = __fmul_rn(e.scores[index], e.direct_scale);
+            live |= 1u << i;
+          }
+        } else {
+          const uint32_t j = index - e.direct;
+          const uint32_t line = j / pairs;
+          const uint32_t slots = pair_slots[j - line * pairs];
+          const uint32_t own = line * kappa;  // below raw, which is below 2^32
+          const uint32_t first = own + (slots & 255u), second = own + (slots >> 8);
+          const int32_t u = e.indices[first], v = e.indices[second];
+          if (in_graph(e, u) && in_graph(e, v)) {
+            if (index - 32 * i < e.direct) placed = false;  // the direct edges' last line is behind this one's first
+            key[i] = edge_key<Key>(e, graph_of(line), u, v);
+            weight[i] = __fmul_rn(__fmul_rn(e.scores[first], e.scores[second]), e.co_scale);
+            live |= 1u << i;
+          }
+        }
+      }
+    }
+
+    uint32_t rank[kItems];
+#pragma unroll
+    for (int i = 0; i < kItems; ++i) {
+      const bool here = kFull || ((live >> i) & 1u);
+      const uint32_t digit = digit_of(key[i], pass);
+      if (here) atomicOr(&my_lanes[digit], 1u << lane);
+      __syncwarp();
+      const uint32_t peers = my_lanes[digit];
+      const uint32_t before = my_count[digit];
+      const uint32_t below = __popc(peers & ((1u << lane) - 1u));
+      __syncwarp();
+      if (here && below == 0u) {
+        my_count[digit] = before + __popc(peers);
+        my_lanes[digit] = 0u;
+      }
+      __syncwarp();
+      rank[i] = before + below;
     }
     __syncthreads();
-    if (live) {
-      const int64_t target = static_cast<int64_t>(round_base[digit]) + warp_count[warp][digit] + rank_in_warp;
-      keys_out[target] = key;
-      weights_out[target] = weight;
+
+    // thread d looks after digit d
+    {
+      const int d = threadIdx.x;
+      uint32_t count = 0u;
+#pragma unroll
+      for (int w = 0; w < kSortWarps; ++w) count += warp_count[w][d];
+      publish(words + static_cast<uint64_t>(tile) * kDigits + d, (tile == 0 ? kComplete : kPartial) | count);
+      if constexpr (!kFirst) {
+#pragma unroll
+        for (int i = 0; i < kItems; ++i) {
+          if (kFull || ((live >> i) & 1u)) weight[i] = weights[item0 + i * 32];
+        }
+      }
+      uint32_t total;
+      const uint32_t start = block_prefix(count, warp_total, &total);
+      uint32_t running = start;  // counts become places in the tile
+#pragma unroll
+      for (int w = 0; w < kSortWarps; ++w) {
+        const uint32_t c = warp_count[w][d];
+        warp_count[w][d] = running;
+        running += c;
+      }
+      const uint32_t ahead = look_back(words + d, tile, kDigits, fault);
+      if (tile > 0) {
+        publish(words + static_cast<uint64_t>(tile) * kDigits + d, kComplete | (static_cast<uint64_t>(ahead) + count));
+      }
+      target_base[d] = digit_base[d] + ahead - start;
+      if (d == 0) tile_s = total;
     }
     __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kItems; ++i) {
+      if (kFull || ((live >> i) & 1u)) {
+        const uint32_t slot = my_count[digit_of(key[i], pass)] + rank[i];
+        stage.out.key[slot] = key[i];
+        stage.out.weight[slot] = weight[i];
+      }
+    }
+    __syncthreads();
+    const uint32_t here = kFull ? kTile : tile_s;
+    const uint32_t limit = *valid;
+#pragma unroll
+    for (int i = 0; i < kItems; ++i) {
+      const uint32_t slot = threadIdx.x + i * kSortThreads;
+      if (kFull || slot < here) {
+        const Key k = stage.out.key[slot];
+        const uint32_t target = target_base[digit_of(k, pass)] + slot;
+        if (target < limit) {
+          keys_out[target] = k;
+          weights_out[target] = stage.out.weight[slot];
+        }
+      }
+    }
+  };
+  if (!kFirst && base + kTile <= n) {
+    work(std::true_type());
+  } else {
+    work(std::false_type());
   }
 }
 
-// ---- runs of equal keys ----
-__global__ void __launch_bounds__(256) run_heads_kernel(const uint64_t* keys, int64_t n, uint32_t* head) {
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const uint64_t key = keys[i];
-    head[i] = (key != kInvalidKey && (i == 0 || keys[i - 1] != key)) ? 1u : 0u;
+// ---- runs of equal keys -> edges ----
+// A thread holds kRunItems consecutive items; it sums every run that begins among them, reading on
+// where the last one goes beyond.  Items come and edges leave through shared memory.
+template <typename Key>
+__global__ void __launch_bounds__(kSortThreads)
+    run_edges_kernel(const Key* keys, const float* weights, const uint32_t* valid, int position_bits, int seq_len,
+                     int64_t capacity, uint64_t* words, uint32_t* ticket, uint32_t* fault, int32_t* edge_src,
+                     int32_t* edge_dst, float* edge_weight, int64_t* edge_count) {
+  constexpr int kItems = Runs<Key>::kItems;
+  constexpr int kTile = Runs<Key>::kTile;
+  __shared__ alignas(16) Key key_in[kTile];
+  __shared__ alignas(16) float weight_in[kTile];
+  __shared__ Key key_out[kTile];
+  __shared__ float weight_out[kTile];
+  __shared__ uint32_t warp_total[kSortWarps];
+  __shared__ uint32_t tile_s, ahead_s;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) tile_s = atomicAdd(ticket, 1u);
+  __syncthreads();
+  const uint32_t tile = tile_s;
+  const uint32_t n = *valid;
+  const uint64_t base = static_cast<uint64_t>(tile) * kTile;
+  if (base >= n) return;
+  const uint32_t here = n - base < kTile ? static_cast<uint32_t>(n - base) : kTile;
+  // four weights and their keys per thread and step
+  for (uint32_t i = 4 * threadIdx.x; i < kTile; i += 4 * kSortThreads) {
+    if (i + 4 <= here) {
+#pragma unroll
+      for (int v = 0; v < static_cast<int>(sizeof(Key) / 4); ++v) {
+        reinterpret_cast<uint4*>(key_in + i)[v] = reinterpret_cast<const uint4*>(keys + base + i)[v];
+      }
+      *reinterpret_cast<float4*>(weight_in + i) = *reinterpret_cast<const float4*>(weights + base + i);
+    } else {
+      for (uint32_t j = i; j < here; ++j) {
+        key_in[j] = keys[base + j];
+        weight_in[j] = weights[base + j];
+      }
+    }
   }
-}
-
-__global__ void __launch_bounds__(256) run_reduce_kernel(const uint64_t* keys, const float* weights,
-                                                         const uint32_t* head, const uint32_t* slot, int64_t n,
-                                                         int64_t vertices, int64_t capacity, int32_t* edge_src,
-                                                         int32_t* edge_dst, float* edge_weight, int64_t* edge_count) {
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const uint64_t key = keys[i];
-    if (i == n - 1) {
-      *edge_count = static_cast<int64_t>(slot[i]) + head[i];  // runs of valid keys
+  const Key before_tile = base > 0 ? keys[base - 1] : 0;
+  __syncthreads();
+  const uint32_t first = threadIdx.x * kItems;
+  Key key[kItems];
+  uint32_t heads = 0u;
+  Key previous = first > 0 ? key_in[first - 1] : before_tile;
+#pragma unroll
+  for (int i = 0; i < kItems; ++i) {
+    key[i] = key_in[first + i];
+    const bool head = first + i < here && ((first + i == 0 && base == 0) || key[i] != previous);
+    heads |= (head ? 1u : 0u) << i;
+    previous = key[i];
+  }
+  uint32_t total;
+  uint32_t slot = block_prefix(__popc(heads), warp_total, &total);
+  if (threadIdx.x < 32) {
+    // a warp looks back together: lane l at the l-th tile in front
+    if (lane == 0) publish(words + tile, (tile == 0 ? kComplete : kPartial) | total);
+    uint64_t sum = 0;
+    uint32_t polls = 0;
+    int64_t t = static_cast<int64_t>(tile) - 1;
+    while (t >= 0) {
+      const uint64_t word = t - lane >= 0 ? look(words + (t - lane)) : kComplete;
+      const unsigned ready = __ballot_sync(0xffffffffu, word != 0ull);
+      const unsigned done = __ballot_sync(0xffffffffu, (word & kComplete) != 0ull);
+      const int reach = done ? __ffs(done) : 32;  // lanes 0 .. reach - 1 are wanted
+      const unsigned wanted = reach == 32 ? 0xffffffffu : (1u << reach) - 1u;
+      if ((ready & wanted) != wanted) {
+        if (++polls > kLookPolls) {
+          if (lane == 0) atomicOr(fault, 1u);
+          break;
+        }
+        continue;
+      }
+      uint64_t part = lane < reach ? (word & kValueMask) : 0ull;
+#pragma unroll
+      for (int offset = 16; offset > 0; offset >>= 1) part += __shfl_xor_sync(0xffffffffu, part, offset);
+      sum += part;
+      if (done) break;
+      t -= 32;
     }
-    if (!head[i]) continue;
-    float sum = weights[i];
-    for (int64_t j = i + 1; j < n && keys[j] == key; ++j) {
-      sum = __fadd_rn(sum, weights[j]);
+    if (lane == 0) {
+      ahead_s = static_cast<uint32_t>(sum);
+      if (tile > 0) publish(words + tile, kComplete | (sum + total));
+      if (base + kTile >= n) {
+        *edge_count = *fault != 0u ? -1 : static_cast<int64_t>(sum + total);
+      }
     }
-    const int64_t out = slot[i];
+  }
+  if (heads != 0u) {
+    float sum = 0.f;
+    Key open = 0;
+    bool started = false;
+#pragma unroll
+    for (int i = 0; i < kItems; ++i) {
+      const float weight = weight_in[first + i];
+      if ((heads >> i) & 1u) {
+        if (started) {
+          key_out[slot] = open;
+          weight_out[slot] = sum;
+          ++slot;
+        }
+        started = true;
+        open = key[i];
+        sum = weight;
+      } else if (started && first + i < here) {
+        sum = __fadd_rn(sum, weight);
+      }
+    }
+    uint32_t j = first + kItems;
+    while (j < here && key_in[j] == open) {
+      sum = __fadd_rn(sum, weight_in[j]);
+      ++j;
+    }
+    if (j >= here) {
+      // the run may go on in the next tiles: four items in flight
+      bool more = true;
+      for (uint64_t at = base + here; more && at < n; at += 4) {
+        Key k[4];
+        float w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint64_t from = at + i < n ? at + i : n - 1;
+          k[i] = keys[from];
+          w[i] = weights[from];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          more = more && at + i < n && k[i] == open;
+          if (more) sum = __fadd_rn(sum, w[i]);
+        }
+      }
+    }
+    key_out[slot] = open;
+    weight_out[slot] = sum;
+  }
+  __syncthreads();
+  const Key mask = (static_cast<Key>(1) << position_bits) - 1;
+  for (uint32_t s = threadIdx.x; s < total; s += kSortThreads) {
+    const int64_t out = static_cast<int64_t>(ahead_s) + s;
     if (out < capacity) {
-      edge_src[out] = static_cast<int32_t>(key / static_cast<uint64_t>(vertices));
-      edge_dst[out] = static_cast<int32_t>(key % static_cast<uint64_t>(vertices));
-      edge_weight[out] = sum;
+      const Key k = key_out[s];
+      const int32_t vertex0 = static_cast<int32_t>(k >> (2 * position_bits)) * seq_len;
+      edge_src[out] = vertex0 + static_cast<int32_t>((k >> position_bits) & mask);
+      edge_dst[out] = vertex0 + static_cast<int32_t>(k & mask);
+      edge_weight[out] = weight_out[s];
     }
   }
 }
 
 int64_t align256(int64_t bytes) { return (bytes + 255) / 256 * 256; }
 
+// Scratch for `raw` edges.  The key width is not known when the size is asked for, so the layout
+// is the one of 8-byte keys; 4-byte keys use part of it.
 struct Scratch {
-  uint64_t* keys[2];
+  void* keys[2];
   float* weights[2];
-  uint32_t* table;       // radix digit counts [256][tiles]; also run heads / slots [raw]
-  uint32_t* table_scan;
-  uint32_t* tile_total;
+  uint32_t* control;  // cleared: digit totals [kMaxPasses][256], valid, fault, a ticket per kernel
+  uint64_t* words;    // cleared: look-back words, [pass][tile][256], then [tile] of the runs
   int64_t bytes;
 };
+constexpr int64_t kControlWords = kMaxPasses * kDigits + 2 + kMaxPasses + 1;
+
+template <typename Key>
+int64_t look_words(int64_t raw, int passes) {
+  return passes * ((raw + Sort<Key>::kTile - 1) / Sort<Key>::kTile) * kDigits +
+         (raw + Runs<Key>::kTile - 1) / Runs<Key>::kTile;
+}
 
 Scratch carve(void* base, int64_t raw) {
   Scratch s = {};
-  const int64_t tiles = (raw + kSortTile - 1) / kSortTile;
-  const int64_t table_items = raw > 256 * tiles ? raw : 256 * tiles;
   int64_t offset = 0;
   auto take = [&](int64_t bytes) {
     uint8_t* p = base ? static_cast<uint8_t*>(base) + offset : nullptr;
     offset += align256(bytes);
     return p;
   };
-  s.keys[0] = reinterpret_cast<uint64_t*>(take(raw * 8));
-  s.keys[1] = reinterpret_cast<uint64_t*>(take(raw * 8));
+  s.keys[0] = take(raw * 8);
+  s.keys[1] = take(raw * 8);
   s.weights[0] = reinterpret_cast<float*>(take(raw * 4));
   s.weights[1] = reinterpret_cast<float*>(take(raw * 4));
-  s.table = reinterpret_cast<uint32_t*>(take(table_items * 4));
-  s.table_scan = reinterpret_cast<uint32_t*>(take(table_items * 4));
-  s.tile_total = reinterpret_cast<uint32_t*>(take(((table_items + kScanTile - 1) / kScanTile + 1) * 4));
+  // `control` and `words` are cleared together
+  const int64_t words = look_words<uint64_t>(raw, kMaxPasses);
+  uint8_t* cleared = take(align256(kControlWords * 4) + words * 8);
+  s.control = reinterpret_cast<uint32_t*>(cleared);
+  s.words = reinterpret_cast<uint64_t*>(cleared + align256(kControlWords * 4));
   s.bytes = offset;
   return s;
+}
+
+template <typename Key, int kKappa>
+cudaError_t sort_and_merge(const EdgeRows& e, const Scratch& s, int bits, int64_t capacity, int32_t* edge_src,
+                           int32_t* edge_dst, float* edge_weight, int64_t* edge_count, cudaStream_t stream) {
+  const int passes = bits > 8 ? (bits + 7) / 8 : 1;
+  const unsigned tiles = static_cast<unsigned>((static_cast<int64_t>(e.raw) + Sort<Key>::kTile - 1) / Sort<Key>::kTile);
+  const unsigned run_tiles = static_cast<unsigned>((static_cast<int64_t>(e.raw) + Runs<Key>::kTile - 1) / Runs<Key>::kTile);
+  uint32_t* totals = s.control;
+  uint32_t* valid = totals + kMaxPasses * kDigits;
+  uint32_t* fault = valid + 1;
+  uint32_t* tickets = fault + 1;
+  cudaError_t err = cudaMemsetAsync(
+      s.control, 0, align256(kControlWords * 4) + static_cast<size_t>(look_words<Key>(e.raw, passes)) * 8, stream);
+  if (err != cudaSuccess) return err;
+  const unsigned lines = e.direct / e.kappa;
+  digit_totals_kernel<Key><<<(lines + kSortThreads - 1) / kSortThreads, kSortThreads, 0, stream>>>(e, passes, totals);
+  digit_bases_kernel<<<passes, kSortThreads, 0, stream>>>(totals, valid);
+  for (int p = 0; p < passes; ++p) {
+    Key* out = static_cast<Key*>(s.keys[p & 1]);
+    const Key* in = static_cast<const Key*>(s.keys[1 - (p & 1)]);
+    uint64_t* words = s.words + static_cast<int64_t>(p) * tiles * kDigits;
+    if (p == 0) {
+      radix_pass_kernel<Key, kKappa, true><<<tiles, kSortThreads, 0, stream>>>(
+          e, in, s.weights[1], out, s.weights[0], totals, valid, 0, words, tickets, fault);
+    } else {
+      radix_pass_kernel<Key, 0, false><<<tiles, kSortThreads, 0, stream>>>(
+          e, in, s.weights[1 - (p & 1)], out, s.weights[p & 1], totals + p * kDigits, valid, p, words, tickets + p,
+          fault);
+    }
+  }
+  const int last = (passes - 1) & 1;
+  run_edges_kernel<Key><<<run_tiles, kSortThreads, 0, stream>>>(
+      static_cast<const Key*>(s.keys[last]), s.weights[last], valid, e.position_bits, e.seq_len, capacity,
+      s.words + static_cast<int64_t>(passes) * tiles * kDigits, tickets + kMaxPasses, fault, edge_src, edge_dst,
+      edge_weight, edge_count);
+  return cudaGetLastError();
+}
+
+int bits_for(int64_t values) {
+  int bits = 0;
+  while ((1ll << bits) < values) ++bits;
+  return bits;
 }
 
 }  // namespace
@@ -342,37 +685,29 @@ int ckv_build_adjacency(const int32_t* topk_indices, const float* topk_scores, c
   if (scratch_bytes < s.bytes) return CKV_ERR_CAPACITY;
   if (reinterpret_cast<uintptr_t>(scratch) % 256) return CKV_ERR_ALIGN;
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
-  const int64_t direct = static_cast<int64_t>(graphs) * rows * kappa;
-  const unsigned wide = static_cast<unsigned>((raw + 255) / 256 > 148 * 16 ? 148 * 16 : (raw + 255) / 256);
   if (cudaMemsetAsync(edge_count, 0, sizeof(int64_t), stream) != cudaSuccess) return CKV_ERR_LAUNCH;
-  ckv::edge_keys_kernel<<<wide, 256, 0, stream>>>(topk_indices, topk_scores, query_positions, rows, kappa, seq_len,
-                                                  vertices, static_cast<float>(lam / 2.0), static_cast<float>(1.0 - lam), direct, raw,
-                                                  s.keys[0],
-                                                  s.weights[0]);
-  if (cudaGetLastError() != cudaSuccess) return CKV_ERR_LAUNCH;
-  // keys are below vertices^2 (the invalid key has every bit set and sorts last in every pass)
-  int vertex_bits = 0;
-  while ((1ll << vertex_bits) < vertices) ++vertex_bits;
-  const int bits = 2 * vertex_bits;
-  const int64_t tiles = (raw + ckv::kSortTile - 1) / ckv::kSortTile;
-  int from = 0;
-  for (int shift = 0; shift < bits; shift += 8) {
-    ckv::radix_count_kernel<<<static_cast<unsigned>(tiles), ckv::kSortThreads, 0, stream>>>(
-        s.keys[from], raw, shift, tiles, s.table);
-    if (ckv::exclusive_scan(s.table, s.table_scan, 256 * tiles, s.tile_total, stream) != cudaSuccess) {
-      return CKV_ERR_LAUNCH;
-    }
-    ckv::radix_scatter_kernel<<<static_cast<unsigned>(tiles), ckv::kSortThreads, 0, stream>>>(
-        s.keys[from], s.weights[from], raw, shift, tiles, s.table_scan, s.keys[1 - from], s.weights[1 - from]);
-    if (cudaGetLastError() != cudaSuccess) return CKV_ERR_LAUNCH;
-    from = 1 - from;
+  ckv::EdgeRows e = {};
+  e.indices = topk_indices;
+  e.scores = topk_scores;
+  e.positions = query_positions;
+  e.rows = static_cast<uint32_t>(rows);
+  e.direct = static_cast<uint32_t>(static_cast<int64_t>(graphs) * rows * kappa);
+  e.raw = static_cast<uint32_t>(raw);
+  e.kappa = kappa;
+  e.seq_len = seq_len;
+  e.position_bits = ckv::bits_for(seq_len);
+  e.direct_scale = static_cast<float>(lam / 2.0);
+  e.co_scale = static_cast<float>(1.0 - lam);
+  const int bits = ckv::bits_for(graphs) + 2 * e.position_bits;  // at most 62: the vertex count is below 2^31
+  auto run = [&](auto sorter) {
+    return sorter(e, s, bits, edge_capacity, edge_src, edge_dst, edge_weight, edge_count, stream) == cudaSuccess
+               ? CKV_OK
+               : CKV_ERR_LAUNCH;
+  };
+  if (bits <= 32 && 2 * e.position_bits < 32) {  // and no shift by the width of the key
+    return kappa == 8 ? run(ckv::sort_and_merge<uint32_t, 8>) : run(ckv::sort_and_merge<uint32_t, 0>);
   }
-  ckv::run_heads_kernel<<<wide, 256, 0, stream>>>(s.keys[from], raw, s.table);
-  if (ckv::exclusive_scan(s.table, s.table_scan, raw, s.tile_total, stream) != cudaSuccess) return CKV_ERR_LAUNCH;
-  ckv::run_reduce_kernel<<<wide, 256, 0, stream>>>(s.keys[from], s.weights[from], s.table, s.table_scan, raw,
-                                                   vertices, edge_capacity, edge_src, edge_dst, edge_weight,
-                                                   edge_count);
-  return cudaGetLastError() == cudaSuccess ? CKV_OK : CKV_ERR_LAUNCH;
+  return kappa == 8 ? run(ckv::sort_and_merge<uint64_t, 8>) : run(ckv::sort_and_merge<uint64_t, 0>);
 }
 
 }  // extern "C"
