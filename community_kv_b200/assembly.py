@@ -90,7 +90,8 @@ def compute_centroids(
     capacity = live + max_decode_tokens
     dim = keys.shape[-1]
     if community_ids.is_cuda and keys.dtype == torch.bfloat16 and dim == 128:
-        return _centroids_cuda(community_ids, keys, retrieval_to_graph, retrieval_to_kv, live, capacity, num_sink)
+        offsets, positions = _member_csr_cuda(community_ids, live, num_sink)
+        return _centroids_cuda(offsets, positions, keys, retrieval_to_graph, retrieval_to_kv, live, capacity)
     labels = community_ids[retrieval_to_graph.long(), num_sink:].long()
     rows = keys[retrieval_to_kv.long(), num_sink:].float()
     sums = torch.zeros((heads, capacity, dim), dtype=torch.float32, device=keys.device)
@@ -128,11 +129,9 @@ def _member_csr_cuda(community_ids: torch.Tensor, widest: int, num_sink: int) ->
     return offsets, positions
 
 
-def _centroids_cuda(community_ids, keys, retrieval_to_graph, retrieval_to_kv, live, capacity, num_sink):
+def _centroids_cuda(offsets, positions, keys, retrieval_to_graph, retrieval_to_kv, live, capacity):
     native = _native()
     device = keys.device
-    counts = torch.full((community_ids.shape[0],), live, dtype=torch.int32, device=device)
-    offsets, positions = build_member_csr(community_ids, counts, num_sink=num_sink)
     heads = retrieval_to_graph.numel()
     if keys.stride(-1) != 1:
         keys = keys.contiguous()
@@ -162,20 +161,25 @@ def init_modularity_state(
 
     graphs, length = community_ids.shape
     device = community_ids.device
-    weight = torch.zeros((graphs, community_capacity), dtype=torch.float32, device=device)
-    total = torch.zeros((graphs,), dtype=torch.float32, device=device)
-    if not edge_src.numel():
-        return weight, total
-    if community_ids.is_cuda:
+    if community_ids.is_cuda and edge_src.numel():
         native = _native()
+        weight = torch.empty((graphs, community_capacity), dtype=torch.float32, device=device)
+        total = torch.empty((graphs,), dtype=torch.float32, device=device)
         labels = community_ids.to(torch.int32).contiguous()
-        source, destination = edge_src.long().contiguous(), edge_dst.long().contiguous()
+        narrow = edge_src.dtype == edge_dst.dtype == torch.int32  # what build_adjacency returns
+        width = torch.int32 if narrow else torch.int64
+        source, destination = edge_src.to(width).contiguous(), edge_dst.to(width).contiguous()
         values = edge_weight.float().contiguous()
+        entry = native.library().ckv_assemble_modularity32 if narrow else native.library().ckv_assemble_modularity
         with torch.cuda.device(device):
-            _check(native.library().ckv_assemble_modularity(
+            _check(entry(
                 labels.data_ptr(), graphs, length, source.data_ptr(), destination.data_ptr(), values.data_ptr(),
                 source.numel(), community_capacity, weight.data_ptr(), total.data_ptr(),
                 native.current_stream(device)))
+        return weight, total
+    weight = torch.zeros((graphs, community_capacity), dtype=torch.float32, device=device)
+    total = torch.zeros((graphs,), dtype=torch.float32, device=device)
+    if not edge_src.numel():
         return weight, total
     source, destination = edge_src.long(), edge_dst.long()
     graph = source // length
@@ -255,13 +259,15 @@ def build_adjacency(
     source = torch.empty((raw,), dtype=torch.int32, device=device)
     destination = torch.empty((raw,), dtype=torch.int32, device=device)
     weight = torch.empty((raw,), dtype=torch.float32, device=device)
-    count = torch.zeros((1,), dtype=torch.int64, device=device)
+    count = torch.empty((1,), dtype=torch.int64, device=device)
     with torch.cuda.device(device):
         _check(lib.ckv_build_adjacency(
             indices.data_ptr(), scores.data_ptr(), positions.data_ptr(), graphs, rows, kappa, int(seq_len),
             float(lam), source.data_ptr(), destination.data_ptr(), weight.data_ptr(), raw, count.data_ptr(),
             scratch.data_ptr(), scratch.numel(), native.current_stream(device)))
     edges = int(count.item())
+    if edges < 0:
+        raise RuntimeError("the adjacency sort gave up a bounded wait; its edges are invalid")
     return source[:edges], destination[:edges], weight[:edges]
 
 
@@ -306,16 +312,22 @@ def assemble_layer(
     to_graph, to_kv = aggregation_mappings(
         aggregation, query_heads=query_heads, kv_heads=kv_heads, device=keys.device
     )
-    centroids, sizes = compute_centroids(
-        community_ids,
-        counts,
-        keys,
-        retrieval_to_graph=to_graph,
-        retrieval_to_kv=to_kv,
-        num_sink=num_sink,
-        max_decode_tokens=max_decode_tokens,
-    )
-    offsets, positions = build_member_csr(community_ids, counts, num_sink=num_sink)
+    if community_ids.is_cuda and keys.dtype == torch.bfloat16 and keys.shape[1:] == (length, 128):
+        # one pass over the labels serves the member lists and the centroids
+        live = int(counts.max())
+        offsets, positions = _member_csr_cuda(community_ids, live, num_sink)
+        centroids, sizes = _centroids_cuda(offsets, positions, keys, to_graph, to_kv, live, live + max_decode_tokens)
+    else:
+        centroids, sizes = compute_centroids(
+            community_ids,
+            counts,
+            keys,
+            retrieval_to_graph=to_graph,
+            retrieval_to_kv=to_kv,
+            num_sink=num_sink,
+            max_decode_tokens=max_decode_tokens,
+        )
+        offsets, positions = build_member_csr(community_ids, counts, num_sink=num_sink)
     capacity = centroids.shape[1]
     if community_weight is None:
         community_weight = torch.zeros((graphs, capacity), dtype=torch.float32, device=keys.device)

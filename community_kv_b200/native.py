@@ -192,6 +192,7 @@ ENTRY_POINTS = (
     "ckv_assemble_member_csr",
     "ckv_assemble_centroids",
     "ckv_assemble_modularity",
+    "ckv_assemble_modularity32",
     "ckv_adjacency_raw_edges",
     "ckv_adjacency_scratch_bytes",
     "ckv_build_adjacency",
@@ -236,8 +237,9 @@ def library() -> ctypes.CDLL:
     lib.ckv_assemble_member_csr.argtypes = [_p, _i, _i, _i, _i, _p, _p, _p, _i, _p]
     lib.ckv_assemble_centroids.restype = ctypes.c_int
     lib.ckv_assemble_centroids.argtypes = [_p, _p, _i, _i, _p, _l, _l, _p, _p, _i, _i, _i, _p, _p, _p]
-    lib.ckv_assemble_modularity.restype = ctypes.c_int
-    lib.ckv_assemble_modularity.argtypes = [_p, _i, _i, _p, _p, _p, _l, _i, _p, _p, _p]
+    for name in ("ckv_assemble_modularity", "ckv_assemble_modularity32"):
+        getattr(lib, name).restype = ctypes.c_int
+        getattr(lib, name).argtypes = [_p, _i, _i, _p, _p, _p, _l, _i, _p, _p, _p]
     for name in ("ckv_adjacency_raw_edges", "ckv_adjacency_scratch_bytes"):
         getattr(lib, name).restype = ctypes.c_int64
         getattr(lib, name).argtypes = [_l, _l, _i, ctypes.c_double]

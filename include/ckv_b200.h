@@ -361,6 +361,11 @@ int ckv_assemble_modularity(const int32_t* labels, int32_t graphs, int32_t lengt
                             const int64_t* edge_dst, const float* edge_weight, int64_t edges,
                             int32_t capacity, float* community_weight, float* total_weight,
                             void* cuda_stream);
+/* The same with int32 vertices, as ckv_build_adjacency writes them. */
+int ckv_assemble_modularity32(const int32_t* labels, int32_t graphs, int32_t length, const int32_t* edge_src,
+                              const int32_t* edge_dst, const float* edge_weight, int64_t edges,
+                              int32_t capacity, float* community_weight, float* total_weight,
+                              void* cuda_stream);
 
 /* Edge list -> coalesced adjacency: what the host partitioner consumes.  topk_indices int32 and
  * topk_scores fp32 are [graphs, rows, kappa] (neighbour position per row, -1 or >= seq_len:
@@ -371,7 +376,8 @@ int ckv_assemble_modularity(const int32_t* labels, int32_t graphs, int32_t lengt
  * their weights in enumeration order (the scale factors are lam / 2 and 1 - lam rounded to fp32
  * once, as a Python float times an fp32 tensor gives), output sorted by (min, max): edge_src / edge_dst int32,
  * edge_weight fp32, *edge_count the number of distinct edges (device int64; edges beyond
- * edge_capacity are counted but not stored).  scratch: ckv_adjacency_scratch_bytes() bytes,
+ * edge_capacity are counted but not stored; -1: a bounded wait inside the sort ran out and the
+ * edges are invalid).  scratch: ckv_adjacency_scratch_bytes() bytes,
  * 256-byte aligned.  Replaces build_adjacency (community_kv/graph/partition.py:168-249). */
 int64_t ckv_adjacency_raw_edges(int64_t graphs, int64_t rows, int32_t kappa, double lam);
 int64_t ckv_adjacency_scratch_bytes(int64_t graphs, int64_t rows, int32_t kappa, double lam);

@@ -175,3 +175,52 @@ def test_adjacency_against_the_cpu_restatement(graphs, rows, length, lam):
     got = build_adjacency(torch.from_numpy(indices).to(device), torch.from_numpy(scores).to(device),
                           torch.from_numpy(positions).to(device), seq_len=length, lam=lam)
     _adjacency_equal(got, want, f"{graphs}x{rows}")
+
+
+@pytest.mark.parametrize(
+    "graphs,rows,length,kappa,lam",
+    [
+        (1, 1, 9, 8, 0.5),            # fewer edges than a tile's first warp has lanes for
+        (3, 31, 4096, 8, 0.5),        # 4092 edges, a few short of a tile; 4-byte keys
+        (2, 47, 65536, 8, 0.5),       # two positions fill 4 bytes: 8-byte keys, two tiles and a bit
+        (1, 187, 256, 8, 0.25),       # 8228 edges, a few beyond two tiles
+        (1, 600, 5000, 8, 1.0),       # direct edges only
+        (5, 260, 3000, 3, 0.5),       # another row width, several graphs in a tile
+        (2, 900, 40, 8, 0.5),         # long runs of one edge, across tiles
+    ],
+)
+def test_adjacency_at_the_edges_of_tiles_and_keys(graphs, rows, length, kappa, lam):
+    from community_kv_b200.assembly import build_adjacency
+    from oracle.adjacency_oracle import build_adjacency as oracle_adjacency
+
+    device = torch.device("cuda", 0)
+    rng = np.random.default_rng(rows + length)
+    positions = rng.integers(0, length, size=(graphs, rows)).astype(np.int64)
+    indices = rng.integers(-1, length, size=(graphs, rows, kappa)).astype(np.int32)
+    scores = rng.uniform(0, 1, size=indices.shape).astype(np.float32)
+    want = oracle_adjacency(indices, scores, positions, seq_len=length, lam=lam)
+    got = build_adjacency(torch.from_numpy(indices).to(device), torch.from_numpy(scores).to(device),
+                          torch.from_numpy(positions).to(device), seq_len=length, lam=lam)
+    _adjacency_equal(got, want, f"{graphs}x{rows}x{kappa}")
+
+
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
+@pytest.mark.parametrize("edges", [1, 15, 16, 4097, 9001])
+def test_modularity_of_sorted_edges(edges, dtype):
+    """Runs of one source, a graph's end inside a thread's run, a ragged tail, unaligned edge arrays."""
+
+    device = torch.device("cuda", 0)
+    graphs, length, communities = 3, 700, 20
+    labels = _labels(graphs, length, communities, seed=11)
+    generator = torch.Generator().manual_seed(edges)
+    source = torch.randint(0, graphs * length, (edges + 1,), generator=generator).sort().values
+    destination = source // length * length + torch.randint(0, length, (edges + 1,), generator=generator)
+    weight = torch.rand((edges + 1,), generator=generator)
+    for begin in (0, 1):
+        part = [t[begin : begin + edges] for t in (source, destination, weight)]
+        want_weight, want_total = init_modularity_state(labels, *part, community_capacity=24)
+        moved = [t.to(device)[begin : begin + edges] for t in (source.to(dtype), destination.to(dtype), weight)]
+        got_weight, got_total = init_modularity_state(labels.to(device), *moved, community_capacity=24)
+        # positive terms in another order: n * 2^-24 relative with n below 1000 per community, 6000 per graph
+        torch.testing.assert_close(got_weight.cpu(), want_weight, rtol=6e-5, atol=1e-6)
+        torch.testing.assert_close(got_total.cpu(), want_total, rtol=4e-4, atol=1e-6)
