@@ -156,16 +156,6 @@ def convert_prefill_tensors(
     for mapping in (retrieval_to_graph, retrieval_to_kv):
         if mapping.dtype != torch.int32 or mapping.shape != (heads,):
             raise TypeError("aggregation mappings must be int32 retrieval-head vectors")
-    widest_kv = int(retrieval_to_kv.max()) + 1
-    query_heads = heads * group_size if query_heads is None else query_heads
-    kv_heads = widest_kv if kv_heads is None else kv_heads
-    if query_heads != heads * group_size:
-        raise ValueError("query-head count does not match retrieval-head geometry")
-    if kv_heads <= 0 or widest_kv > kv_heads:
-        raise ValueError("KV-head count does not cover retrieval mappings")
-    if token_communities.shape[1] < prefill_seq_len + max_decode_tokens:
-        raise ValueError("token_communities lacks requested decode headroom")
-    device = centroids.device
     for tensor in (
         member_offsets,
         member_positions,
@@ -177,11 +167,28 @@ def convert_prefill_tensors(
         retrieval_to_graph,
         retrieval_to_kv,
     ):
-        if tensor.device != device:
+        if tensor.device != centroids.device:
             raise ValueError("all converted tensors must share one device")
-
-    head_counts = num_communities[retrieval_to_graph.long()].contiguous()
-    initial = tuple(int(v) for v in head_counts.cpu().tolist())
+    # everything that the checks read comes to the host in one copy
+    if member_offsets.dtype != torch.int32 or member_offsets.ndim != 2:
+        raise TypeError("member_offsets must be a rank-two int32 tensor")
+    host = torch.cat(
+        (retrieval_to_graph, retrieval_to_kv, num_communities, member_offsets.reshape(-1))
+    ).cpu()
+    host_graph, host_kv, host_counts, host_offsets = host.split((heads, heads, graphs, member_offsets.numel()))
+    widest_kv = int(host_kv.max()) + 1
+    query_heads = heads * group_size if query_heads is None else query_heads
+    kv_heads = widest_kv if kv_heads is None else kv_heads
+    if query_heads != heads * group_size:
+        raise ValueError("query-head count does not match retrieval-head geometry")
+    if kv_heads <= 0 or widest_kv > kv_heads:
+        raise ValueError("KV-head count does not cover retrieval mappings")
+    if token_communities.shape[1] < prefill_seq_len + max_decode_tokens:
+        raise ValueError("token_communities lacks requested decode headroom")
+    device = centroids.device
+    if int(host_graph.min()) < 0 or int(host_graph.max()) >= graphs:
+        raise ValueError("retrieval mapping index is out of bounds")
+    initial = tuple(host_counts[host_graph.long()].tolist())
     if any(not 0 < count <= capacity for count in initial):
         raise ValueError("active community counts must fit centroid capacity")
     csr = PrefillCSR(
@@ -192,7 +199,7 @@ def convert_prefill_tensors(
     mutable = MutableGraphState(
         centroids=centroids.contiguous(),
         community_sizes=community_sizes.contiguous(),
-        community_counts=head_counts.clone(),
+        community_counts=num_communities.index_select(0, retrieval_to_graph),
         community_weight=community_weight.contiguous(),
         total_weight=total_weight.contiguous(),
         token_communities=token_communities.contiguous(),
@@ -205,8 +212,9 @@ def convert_prefill_tensors(
         retrieval_to_graph=retrieval_to_graph.contiguous(),
         retrieval_to_kv=retrieval_to_kv.contiguous(),
     )
-    csr.validate()
-    mutable.validate()
+    # the padding repeats a row's last offset, so the rows as they came say all there is to check
+    csr.validate(offsets=host_offsets.view(graphs, -1), counts=host_counts)
+    mutable.validate(retrieval_to_graph=host_graph, retrieval_to_kv=host_kv)
     return ConvertedPrefillState(
         csr=csr,
         mutable=mutable,

@@ -14,6 +14,7 @@ from __future__ import annotations
 
 from collections.abc import Sequence
 from dataclasses import dataclass, fields
+from math import prod
 
 import torch
 
@@ -30,6 +31,29 @@ def _lead(batch: int | None) -> tuple[int, ...]:
     if batch <= 0:
         raise ValueError("batch must be positive")
     return (batch,)
+
+
+def _carve(
+    shapes: Sequence[tuple[tuple[int, ...], torch.dtype]], device: torch.device | str, *, ones: bool = False
+) -> list[torch.Tensor]:
+    """Tensors of the given shapes in one allocation cleared by one fill: all zero, or all bits set (integer -1).
+
+    A layer's workspaces and pools are some thirty small tensors, and a fill of its own for each
+    costs more than anything else in preparing a layer.  Every tensor starts on a 256-byte boundary.
+    """
+
+    sizes = [prod(shape) * dtype.itemsize for shape, dtype in shapes]
+    starts = [0]
+    for size in sizes:
+        starts.append(starts[-1] + (size + 255) // 256 * 256)
+    if ones:
+        storage = torch.full((starts[-1],), 255, dtype=torch.uint8, device=device)
+    else:
+        storage = torch.zeros((starts[-1],), dtype=torch.uint8, device=device)
+    return [
+        storage[start : start + size].view(dtype).view(shape)
+        for start, size, (shape, dtype) in zip(starts, sizes, shapes)
+    ]
 
 
 def _int32(name: str, tensor: torch.Tensor) -> None:
@@ -77,7 +101,9 @@ class PrefillCSR:
     def community_capacity(self) -> int:
         return self.member_offsets.shape[-1] - 1
 
-    def validate(self) -> None:
+    def validate(self, *, offsets: torch.Tensor | None = None, counts: torch.Tensor | None = None) -> None:
+        """``offsets``, ``counts``: host copies of the two tensors, where the caller has them already."""
+
         for item in fields(self):
             _int32(item.name, getattr(self, item.name))
         if self.member_offsets.ndim != 2 or self.member_positions.ndim != 2:
@@ -87,18 +113,16 @@ class PrefillCSR:
             raise ValueError("community_counts must have one entry per graph")
         if self.member_positions.shape[0] != graphs:
             raise ValueError("member_positions must have one row per graph")
-        offsets = self.member_offsets.cpu().long()
-        counts = self.community_counts.cpu().long()
-        width = self.member_positions.shape[1]
-        for graph in range(graphs):
-            count = int(counts[graph])
-            if not 0 <= count < offsets.shape[1]:
-                raise ValueError("community count exceeds offset capacity")
-            row = offsets[graph, : count + 1]
-            if int(row[0]) != 0 or bool((row[1:] < row[:-1]).any()):
-                raise ValueError("active CSR offsets must start at zero and be monotonic")
-            if int(row[-1]) > width:
-                raise ValueError("CSR offsets exceed member-position capacity")
+        offsets = self.member_offsets.cpu() if offsets is None else offsets
+        counts = (self.community_counts.cpu() if counts is None else counts).long().unsqueeze(1)
+        if bool(((counts < 0) | (counts >= self.member_offsets.shape[1])).any()):
+            raise ValueError("community count exceeds offset capacity")
+        counts = counts.clamp(max=offsets.shape[1] - 1)  # the host copy may lack the padding
+        falls = (offsets[:, 1:] < offsets[:, :-1]) & (torch.arange(offsets.shape[1] - 1) < counts)
+        if bool(offsets[:, 0].any()) or bool(falls.any()):
+            raise ValueError("active CSR offsets must start at zero and be monotonic")
+        if bool((offsets.gather(1, counts) > self.member_positions.shape[1]).any()):
+            raise ValueError("CSR offsets exceed member-position capacity")
 
     def members(self, graph: int, community: int) -> torch.Tensor:
         if not 0 <= graph < self.graph_count:
@@ -149,15 +173,11 @@ class DecodeDeltaChunks:
         shapes.update({name: (graph_count, max_decode_tokens) for name in _DELTA_CHUNK_FIELDS})
         shapes.update({name: (graph_count, community_capacity) for name in _DELTA_TABLE_FIELDS})
         shapes.update({name: (graph_count,) for name in _DELTA_CURSOR_FIELDS})
-        tensors = {
-            name: torch.full(
-                lead + shape,
-                -1 if name in _DELTA_MINUS_ONE else 0,
-                dtype=torch.int32,
-                device=device,
-            )
-            for name, shape in shapes.items()
-        }
+        tensors = {}
+        for ones in (False, True):
+            names = [name for name in shapes if (name in _DELTA_MINUS_ONE) == ones]
+            pool = _carve([(lead + shapes[name], torch.int32) for name in names], device, ones=ones)
+            tensors.update(zip(names, pool))
         return cls(**tensors)
 
     @property
@@ -283,7 +303,11 @@ class MutableGraphState:
         own = [getattr(self, item.name) for item in fields(self) if item.name != "deltas"]
         return own + [getattr(self.deltas, item.name) for item in fields(self.deltas)]
 
-    def validate(self) -> None:
+    def validate(
+        self, *, retrieval_to_graph: torch.Tensor | None = None, retrieval_to_kv: torch.Tensor | None = None
+    ) -> None:
+        """``retrieval_to_graph``, ``retrieval_to_kv``: host copies, where the caller has them already."""
+
         if self.centroids.ndim != 3:
             raise ValueError("centroids must have shape [graphs, communities, dim]")
         if self.centroids.dtype not in (torch.float8_e4m3fn, torch.float32):
@@ -317,11 +341,9 @@ class MutableGraphState:
             _int32(name, mapping)
             if mapping.shape != (heads,):
                 raise ValueError(f"{name} must have one entry per retrieval head")
-        if (
-            int(self.retrieval_to_graph.min()) < 0
-            or int(self.retrieval_to_graph.max()) >= graphs
-            or int(self.retrieval_to_kv.min()) < 0
-        ):
+        to_graph = self.retrieval_to_graph.cpu() if retrieval_to_graph is None else retrieval_to_graph
+        to_kv = self.retrieval_to_kv.cpu() if retrieval_to_kv is None else retrieval_to_kv
+        if int(to_graph.min()) < 0 or int(to_graph.max()) >= graphs or int(to_kv.min()) < 0:
             raise ValueError("retrieval mapping index is out of bounds")
         device = self.centroids.device
         if any(tensor.device != device for tensor in self.tensors()):
@@ -397,17 +419,27 @@ class CentroidSelectionWorkspace:
             )
         selected = token_budget - num_sink - 1
         heads = lead + (kv_heads,)
+        scores, ends, counts, tiles = _carve(
+            [
+                (heads + (community_capacity,), torch.float16),
+                (heads + (selected,), torch.int32),
+                (heads, torch.int32),
+                (heads + (token_budget // ATTENTION_TILE,), torch.int32),
+            ],
+            device,
+        )
+        threshold, communities, positions = _carve(
+            [(heads + (width,), torch.int32) for width in (4, selected, token_budget)], device, ones=True
+        )
         return cls(
-            scores=torch.zeros(heads + (community_capacity,), dtype=torch.float16, device=device),
+            scores=scores,
             score_cover=cover,
-            native_threshold=torch.full(heads + (4,), -1, dtype=torch.int32, device=device),
-            communities=torch.full(heads + (selected,), -1, dtype=torch.int32, device=device),
-            cumulative_ends=torch.zeros(heads + (selected,), dtype=torch.int32, device=device),
-            descriptor_counts=torch.zeros(heads, dtype=torch.int32, device=device),
-            tile_descriptors=torch.zeros(
-                heads + (token_budget // ATTENTION_TILE,), dtype=torch.int32, device=device
-            ),
-            positions=torch.full(heads + (token_budget,), -1, dtype=torch.int32, device=device),
+            native_threshold=threshold,
+            communities=communities,
+            cumulative_ends=ends,
+            descriptor_counts=counts,
+            tile_descriptors=tiles,
+            positions=positions,
             token_budget=token_budget,
             num_sink=num_sink,
             max_communities=max_communities,
@@ -478,18 +510,28 @@ class SegmentedAttentionWorkspace:
         lead = _lead(batch)
         heads = lead + (kv_heads,)
         query_heads = lead + (kv_heads * group_size,)
+        partials, packed, output, lse, scores, positions, status = _carve(
+            [
+                (heads + (splits, group_size, PARTIAL_STRIDE), torch.float32),
+                (heads + (splits, KAPPA), torch.int64),
+                (query_heads + (HEAD_DIM,), dtype),
+                (query_heads, torch.float32),
+                (heads + (KAPPA,), torch.float32),
+                (heads + (KAPPA,), torch.int32),
+                ((1,), torch.int32),
+            ],
+            device,
+        )
         return cls(
             group_size=group_size,
             splits=splits,
-            partials=torch.zeros(
-                heads + (splits, group_size, PARTIAL_STRIDE), dtype=torch.float32, device=device
-            ),
-            partial_topk_packed=torch.zeros(heads + (splits, KAPPA), dtype=torch.int64, device=device),
-            output=torch.zeros(query_heads + (HEAD_DIM,), dtype=dtype, device=device),
-            lse=torch.zeros(query_heads, dtype=torch.float32, device=device),
-            topk_scores=torch.zeros(heads + (KAPPA,), dtype=torch.float32, device=device),
-            topk_positions=torch.zeros(heads + (KAPPA,), dtype=torch.int32, device=device),
-            status=torch.zeros((1,), dtype=torch.int32, device=device),
+            partials=partials,
+            partial_topk_packed=packed,
+            output=output,
+            lse=lse,
+            topk_scores=scores,
+            topk_positions=positions,
+            status=status,
         )
 
 
@@ -511,10 +553,8 @@ class OnlineUpdateWorkspace:
         if graph_count <= 0:
             raise ValueError("graph_count must be positive")
         shape = _lead(batch) + (graph_count,)
-        return cls(
-            assigned_communities=torch.zeros(shape, dtype=torch.int32, device=device),
-            overflow=torch.zeros(shape, dtype=torch.int32, device=device),
-        )
+        assigned, overflow = _carve([(shape, torch.int32)] * 2, device)
+        return cls(assigned_communities=assigned, overflow=overflow)
 
 
 @dataclass(slots=True)
