@@ -169,13 +169,10 @@ def convert_prefill_tensors(
     ):
         if tensor.device != centroids.device:
             raise ValueError("all converted tensors must share one device")
-    # everything that the checks read comes to the host in one copy
     if member_offsets.dtype != torch.int32 or member_offsets.ndim != 2:
         raise TypeError("member_offsets must be a rank-two int32 tensor")
-    host = torch.cat(
-        (retrieval_to_graph, retrieval_to_kv, num_communities, member_offsets.reshape(-1))
-    ).cpu()
-    host_graph, host_kv, host_counts, host_offsets = host.split((heads, heads, graphs, member_offsets.numel()))
+    host = torch.cat((retrieval_to_graph, retrieval_to_kv, num_communities)).cpu()
+    host_graph, host_kv, host_counts = host.split((heads, heads, graphs))
     widest_kv = int(host_kv.max()) + 1
     query_heads = heads * group_size if query_heads is None else query_heads
     kv_heads = widest_kv if kv_heads is None else kv_heads
@@ -212,8 +209,7 @@ def convert_prefill_tensors(
         retrieval_to_graph=retrieval_to_graph.contiguous(),
         retrieval_to_kv=retrieval_to_kv.contiguous(),
     )
-    # the padding repeats a row's last offset, so the rows as they came say all there is to check
-    csr.validate(offsets=host_offsets.view(graphs, -1), counts=host_counts)
+    csr.validate()
     mutable.validate(retrieval_to_graph=host_graph, retrieval_to_kv=host_kv)
     return ConvertedPrefillState(
         csr=csr,

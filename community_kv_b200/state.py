@@ -101,9 +101,7 @@ class PrefillCSR:
     def community_capacity(self) -> int:
         return self.member_offsets.shape[-1] - 1
 
-    def validate(self, *, offsets: torch.Tensor | None = None, counts: torch.Tensor | None = None) -> None:
-        """``offsets``, ``counts``: host copies of the two tensors, where the caller has them already."""
-
+    def validate(self) -> None:
         for item in fields(self):
             _int32(item.name, getattr(self, item.name))
         if self.member_offsets.ndim != 2 or self.member_positions.ndim != 2:
@@ -113,15 +111,21 @@ class PrefillCSR:
             raise ValueError("community_counts must have one entry per graph")
         if self.member_positions.shape[0] != graphs:
             raise ValueError("member_positions must have one row per graph")
-        offsets = self.member_offsets.cpu() if offsets is None else offsets
-        counts = (self.community_counts.cpu() if counts is None else counts).long().unsqueeze(1)
-        if bool(((counts < 0) | (counts >= self.member_offsets.shape[1])).any()):
+        # compared where the tensors are: on the host a comparison of this size is shared out over
+        # every core, and waking those costs milliseconds
+        offsets, width = self.member_offsets, self.community_capacity
+        counts = self.community_counts.unsqueeze(1)
+        outside = (counts < 0) | (counts > width)
+        falls = (offsets[:, 1:] < offsets[:, :-1]) & (torch.arange(width, device=offsets.device) < counts)
+        beyond = offsets.gather(1, counts.clamp(0, width).long()) > self.member_positions.shape[1]
+        outside, starts, falls, beyond = torch.stack(
+            (outside.any(), offsets[:, 0].any(), falls.any(), beyond.any())
+        ).tolist()
+        if outside:
             raise ValueError("community count exceeds offset capacity")
-        counts = counts.clamp(max=offsets.shape[1] - 1)  # the host copy may lack the padding
-        falls = (offsets[:, 1:] < offsets[:, :-1]) & (torch.arange(offsets.shape[1] - 1) < counts)
-        if bool(offsets[:, 0].any()) or bool(falls.any()):
+        if starts or falls:
             raise ValueError("active CSR offsets must start at zero and be monotonic")
-        if bool((offsets.gather(1, counts) > self.member_positions.shape[1]).any()):
+        if beyond:
             raise ValueError("CSR offsets exceed member-position capacity")
 
     def members(self, graph: int, community: int) -> torch.Tensor:
