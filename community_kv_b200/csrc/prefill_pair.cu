@@ -156,24 +156,74 @@ __device__ __forceinline__ uint32_t quantised_key_fma(float raw) {
   return __float_as_uint(scaled + 12582912.0f) & 0x7fffu;
 }
 
-// Insertion into a descending list by position: every slot decides by two comparisons
-// whether it keeps its entry, takes the candidate or takes its left neighbour's entry.
+// Insertion into a descending list: slot k becomes the median of its entry, its left
+// neighbour's entry and the candidate (two operations per slot, all slots side by side).
 template <int kDepth>
 __device__ __forceinline__ void sorted_insert(uint32_t (&queue)[kDepth], uint32_t candidate) {
-  bool keeps[kDepth];
 #pragma unroll
-  for (int k = 0; k < kDepth; ++k) {
-    keeps[k] = queue[k] >= candidate;
+  for (int k = kDepth - 1; k > 0; --k) {
+    queue[k] = max(queue[k], min(queue[k - 1], candidate));
   }
-  uint32_t next[kDepth];
-  next[0] = keeps[0] ? queue[0] : candidate;
+  queue[0] = max(queue[0], candidate);
+}
+
+// Minimum that does not lose a NaN
+__device__ __forceinline__ float min_nan(float a, float b) {
+  float y;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+  return y;
+}
+
+// Candidates of one column class (32 of the 128 columns): the columns that reach the gate
+// as a bit mask, then insertion in rounds - every lane with a pending column inserts its
+// next one per round, the others zero, without a branch.  The mask is collected from the
+// sign of score - gate, one shift each.  The pick of the column's score (a binary tree over
+// the index bits) and the insertion are shallow: two warps share a scheduler, so the
+// depth of the dependency chain is what a round costs.  A score that is not a number
+// passes the sign test and is turned away by the comparison behind the pick.
+// `sinks`: that many columns at the front are no candidates.
+template <int kClass>
+__device__ __forceinline__ void take_candidates(const float (&s)[128], float gate, int key0, int sinks,
+                                                uint32_t (&queue)[kLocalK]) {
+  const uint64_t minus_gate = pack_pair(-gate, -gate);
+  uint32_t below[4] = {0u, 0u, 0u, 0u};  // sign bits of eight columns each
 #pragma unroll
-  for (int k = 1; k < kDepth; ++k) {
-    next[k] = keeps[k] ? queue[k] : (keeps[k - 1] ? candidate : queue[k - 1]);
+  for (int byte = 0; byte < 4; ++byte) {
+#pragma unroll
+    for (int j = 6; j >= 0; j -= 2) {
+      const int c = ((byte * 8 + j) >> 1) * 8 + kClass * 2;
+      float lo, hi;
+      unpack_pair(add_pair(pack_pair(s[c], s[c + 1]), minus_gate), lo, hi);
+      below[byte] = __funnelshift_l(__float_as_uint(hi), below[byte], 1);
+      below[byte] = __funnelshift_l(__float_as_uint(lo), below[byte], 1);
+    }
   }
+  uint32_t takers = ~(below[0] | (below[1] << 8) | (below[2] << 16) | (below[3] << 24));
+  if (sinks > 0) {
+    // the pairs of whole groups of eight columns, and up to two columns of the next group
+    const int pairs = min(sinks >> 3, 15);
+    const int more = sinks >= 128 ? 2 : min(max((sinks & 7) - 2 * kClass, 0), 2);
+    takers &= ~(((1u << (2 * pairs)) - 1u) | (((1u << more) - 1u) << (2 * pairs)));
+  }
+  while (__any_sync(0xffffffffu, takers != 0u)) {
+    const int i = __ffs(takers) - 1;  // -1: nothing left in this lane
+    float pick[16];
 #pragma unroll
-  for (int k = 0; k < kDepth; ++k) {
-    queue[k] = next[k];
+    for (int m = 0; m < 16; ++m) {
+      pick[m] = (i & 1) ? s[m * 8 + kClass * 2 + 1] : s[m * 8 + kClass * 2];
+    }
+#pragma unroll
+    for (int width = 8, bit = 2; width >= 1; width >>= 1, bit <<= 1) {
+#pragma unroll
+      for (int m = 0; m < width; ++m) {
+        pick[m] = (i & bit) ? pick[2 * m + 1] : pick[2 * m];
+      }
+    }
+    const int c = (i >> 1) * 8 + kClass * 2 + (i & 1);
+    const uint32_t candidate =
+        (quantised_key_fma(pick[0]) << 17) | (static_cast<uint32_t>(key0 + c) & 0x1ffffu);
+    sorted_insert<kLocalK>(queue, takers != 0u && pick[0] >= gate ? candidate : 0u);
+    takers &= takers - 1;
   }
 }
 
@@ -421,26 +471,28 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       // the row of O in tensor memory, once the product that still adds to it is done.
       const float new_max = fmaxf(run_max, tile_max);
       const bool move = new_max > run_max && (new_max - run_max) * scale_log2 > 8.0f;
-      float corr = 1.f;
-      if (move) {
-        corr = run_max == -INFINITY ? 0.f : exp2_fast((run_max - new_max) * scale_log2);
-        run_max = new_max;
-        run_sum *= corr;
-      }
-      if (block > 0 && __any_sync(0xffffffffu, move)) {
-        // P.V of the last block is done: this block's S was committed after it
-#pragma unroll
-        for (int part = 0; part < 4; ++part) {
-          uint32_t o[32];
-          tmem_load32_issue(o_addr + part * 32u, o);
-          tmem_wait_load();
-#pragma unroll
-          for (int c = 0; c < 32; ++c) {
-            o[c] = __float_as_uint(__uint_as_float(o[c]) * corr);
-          }
-          tmem_store32_issue(o_addr + part * 32u, o);
+      if (__any_sync(0xffffffffu, move)) {
+        float corr = 1.f;
+        if (move) {
+          corr = run_max == -INFINITY ? 0.f : exp2_fast((run_max - new_max) * scale_log2);
+          run_max = new_max;
+          run_sum *= corr;
         }
-        tmem_wait_store();
+        if (block > 0) {
+          // P.V of the last block is done: this block's S was committed after it.  Rare, so
+          // rolled and in narrow steps: 32 columns at a time spilled registers of the loop.
+#pragma unroll 1
+          for (int part = 0; part < 8; ++part) {
+            uint32_t o[16];
+            tmem_load16_issue(o_addr + part * 16u, o);
+            tmem_wait_load();
+#pragma unroll
+            for (int c = 0; c < 16; ++c) {
+              o[c] = __float_as_uint(__uint_as_float(o[c]) * corr);
+            }
+            tmem_store16_issue(o_addr + part * 16u, o);
+          }
+        }
       }
       // ---- probabilities, bf16 pairs, over the first 64 columns of this S buffer ----
       const float offset = (run_max == -INFINITY ? 0.f : run_max) * scale_log2;
@@ -448,11 +500,11 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       const uint64_t offset_pair = pack_pair(-offset, -offset);
       uint64_t sum_pair[2] = {0ull, 0ull};
 #pragma unroll
-      for (int part = 0; part < 2; ++part) {
-        uint32_t packed[32];
+      for (int quarter = 0; quarter < 4; ++quarter) {
+        uint32_t packed[16];
 #pragma unroll
-        for (int e = 0; e < 32; ++e) {
-          const int c = part * 64 + 2 * e;
+        for (int e = 0; e < 16; ++e) {
+          const int c = quarter * 32 + 2 * e;
           float x0, x1;
           unpack_pair(fma_pair(pack_pair(s[c], s[c + 1]), scale_pair, offset_pair), x0, x1);
           const float p0 = exp2_fast(x0);
@@ -460,7 +512,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
           sum_pair[e & 1] = add_pair(sum_pair[e & 1], pack_pair(p0, p1));
           packed[e] = pack_bf16(p0, p1);
         }
-        tmem_store32_issue(s_addr + part * 32u, packed);
+        tmem_store16_issue(s_addr + quarter * 16u, packed);
       }
       {
         float a0, a1, b0, b1;
@@ -476,78 +528,52 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         mbar_arrive(bar_p_full + 8 * t);
       }
 
-      // The candidate bookkeeping runs from the scores still in registers while the tensor
-      // cores work on this tile's P.V and next S: it is off the path between two blocks.
+      // The candidate bookkeeping is bound by the ALU and by its rounds of insertion, one at least
+      // in most blocks and classes; the gates keep their number down.  32 query on 8 KV heads,
+      // against a gate from the lists alone, rounds with a branch, and the rows behind the
+      // end taking part: 517 tokens 117 -> 39 us, 6001 tokens 1560 -> 530 us, 16384 tokens
+      // 3250 -> 2620 us (attention alone: 20, 326 and 1820 us).
+      // It runs from the scores still in registers while the tensor cores work on this
+      // tile's P.V and next S: it is off the path between two blocks.
       if constexpr (kMode == 1) {
-        if (key0 >= a.num_sink) {
-          // A key that is below eight keys already held can never reach the output:
-          // the second-best entries of the four classes are eight such keys, and so
-          // are the top four of the two best classes.
-          const uint32_t third0 = q32[0][3], third1 = q32[1][3], third2 = q32[2][3], third3 = q32[3][3];
-          const uint32_t second_of_fourths =
-              max(min(max(third0, third1), max(third2, third3)),
-                  max(min(third0, third1), min(third2, third3)));
-          const uint32_t row_floor = max(min(min(q32[0][1], q32[1][1]), min(q32[2][1], q32[3][1])),
-                                         second_of_fourths);
-          // smallest raw score whose quantised key can reach the floor, a little low
-          const float gate = (row_floor >> 17) == 0u
-                                 ? -3.0e38f
-                                 : (static_cast<float>(row_floor >> 17) - 0.75f) * (1.0f / 256.0f) - 48.0f;
-          // Class by class (32 of the 128 columns each; the larger of two partial maxima
-          // is the class maximum, so a class without a taker in any row of the warp costs
-          // one vote): the columns that reach the gate as a bit mask, then insertion in
-          // rounds - every lane with a pending column inserts its next one per round.
-          // Both the pick of the column's score (a binary tree over the index bits) and
-          // the insertion (position by comparison) are shallow: one warp runs this alone
-          // on its scheduler, so the depth of the dependency chain is what it costs.
+        const int sinks = a.num_sink - key0;  // columns of this block that are no candidates
+        if (sinks > 0) {
+          // the groups' maxima without them: the upper 64 columns, if that is far enough
 #pragma unroll
-          for (int cls = 0; cls < 4; ++cls) {
-            if (!__any_sync(0xffffffffu, fmaxf(part_max[2 * cls], part_max[2 * cls + 1]) >= gate)) {
-              continue;
-            }
-            uint32_t takers = 0u;
+          for (int i = 0; i < 8; ++i) {
+            part_max[i] = s[64 + i];
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const int c = (i >> 1) * 8 + cls * 2 + (i & 1);
-              takers |= (s[c] >= gate ? 1u : 0u) << i;
-            }
-            while (__any_sync(0xffffffffu, takers != 0u)) {
-              if (takers != 0u) {
-                const int i = __ffs(takers) - 1;
-                takers &= takers - 1;
-                float pick[16];
-#pragma unroll
-                for (int m = 0; m < 16; ++m) {
-                  pick[m] = (i & 1) ? s[m * 8 + cls * 2 + 1] : s[m * 8 + cls * 2];
-                }
-#pragma unroll
-                for (int width = 8, bit = 2; width >= 1; width >>= 1, bit <<= 1) {
-#pragma unroll
-                  for (int m = 0; m < width; ++m) {
-                    pick[m] = (i & bit) ? pick[2 * m + 1] : pick[2 * m];
-                  }
-                }
-                const int c = (i >> 1) * 8 + cls * 2 + (i & 1);
-                const uint32_t candidate =
-                    (quantised_key_fma(pick[0]) << 17) | (static_cast<uint32_t>(key0 + c) & 0x1ffffu);
-                sorted_insert<kLocalK>(q32[cls], candidate);
-              }
-            }
-          }
-        } else {
-#pragma unroll
-          for (int c = 0; c < 128; ++c) {
-            const int j = key0 + c;
-            if (s[c] > -INFINITY && j >= a.num_sink) {
-              const uint32_t candidate =
-                  (quantised_key(s[c]) << 17) | (static_cast<uint32_t>(j) & 0x1ffffu);
-              uint32_t(&queue)[kLocalK] = q32[(c & 7) >> 1];
-              if (candidate > queue[kLocalK - 1]) {
-                queue_insert<kLocalK>(queue, candidate);
-              }
+            for (int c = 72 + i; c < 128; c += 8) {
+              part_max[i] = fmaxf(part_max[i], s[c]);
             }
           }
         }
+        // A key that is below two keys of every class can never reach the output (the class
+        // lists then hold at least eight keys above it), nor one below the top four of two
+        // classes.  Two keys of every class: the second-best entries of the lists, or the
+        // maxima of this block's two column groups of every class.
+        const uint32_t third0 = q32[0][3], third1 = q32[1][3], third2 = q32[2][3], third3 = q32[3][3];
+        const uint32_t second_of_fourths =
+            max(min(max(third0, third1), max(third2, third3)),
+                max(min(third0, third1), min(third2, third3)));
+        const uint32_t row_floor = max(min(min(q32[0][1], q32[1][1]), min(q32[2][1], q32[3][1])),
+                                       second_of_fourths);
+        float block_floor =
+            min_nan(min_nan(min_nan(part_max[0], part_max[1]), min_nan(part_max[2], part_max[3])),
+                    min_nan(min_nan(part_max[4], part_max[5]), min_nan(part_max[6], part_max[7])));
+        block_floor = sinks > 64 ? -INFINITY : block_floor;
+        const uint32_t floor_key = max(row_floor >> 17, quantised_key_fma(block_floor));
+        // smallest raw score whose quantised key can reach the floor, a little low
+        float gate = floor_key == 0u
+                         ? -3.0e38f
+                         : (static_cast<float>(floor_key) - 0.75f) * (1.0f / 256.0f) - 48.0f;
+        // rows behind the end of a ragged prompt score 0 everywhere: ties that all reach the gate
+        gate = row_live ? gate : INFINITY;
+        // (no vote in front of a class: in most blocks some row of the warp has a taker)
+        take_candidates<0>(s, gate, key0, sinks, q32[0]);
+        take_candidates<1>(s, gate, key0, sinks, q32[1]);
+        take_candidates<2>(s, gate, key0, sinks, q32[2]);
+        take_candidates<3>(s, gate, key0, sinks, q32[3]);
       }
     }
 
@@ -586,30 +612,21 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         if constexpr (kMode == 1) {
           const int skip = a.num_sink + kKappa - 1;
           if (row_pos >= skip) {
-            // merge the four sorted class queues: eight rounds of "largest head wins"
-            int cursor[4] = {0, 0, 0, 0};
+            // merge the four sorted class queues: eight times the largest head, which then
+            // leaves its queue (a cursor per queue would put the queues into local memory)
             const int64_t base =
                 ((batch * heads_total + row_head) * (length - skip) + (row_pos - skip)) * kKappa;
             const float lse_log2 = lse * kLog2e;
 #pragma unroll
             for (int rank = 0; rank < kKappa; ++rank) {
-              uint32_t best = 0u;
-              int winner = 0;
+              const uint32_t best = max(max(q32[0][0], q32[1][0]), max(q32[2][0], q32[3][0]));
 #pragma unroll
               for (int c = 0; c < 4; ++c) {
-                uint32_t head = 0u;
+                const bool leaves = q32[c][0] == best;
 #pragma unroll
                 for (int k = 0; k < kLocalK; ++k) {
-                  head = cursor[c] == k ? q32[c][k] : head;
+                  q32[c][k] = leaves ? (k + 1 < kLocalK ? q32[c][k + 1] : 0u) : q32[c][k];
                 }
-                if (head > best) {
-                  best = head;
-                  winner = c;
-                }
-              }
-#pragma unroll
-              for (int c = 0; c < 4; ++c) {
-                cursor[c] += (c == winner) ? 1 : 0;
               }
               const float dequant = static_cast<float>(best >> 17) / 256.0f - 48.0f;
               a.topk_val[base + rank] = exp2f(dequant * scale_log2 - lse_log2);

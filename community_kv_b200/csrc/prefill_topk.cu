@@ -904,16 +904,6 @@ __device__ __forceinline__ uint32_t instruction_descriptor_n64() {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((kEdgeSub >> 3) << 17) | ((kPfRows >> 4) << 24);
 }
 
-__device__ __forceinline__ void tmem_load16_issue(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-}
-
 // Insertion into a descending list by position: every slot decides from two comparisons
 // whether it keeps its entry, takes the candidate or takes its left neighbour's entry, so
 // the dependency chain is two operations deep whatever the length.  Returns what fell off
