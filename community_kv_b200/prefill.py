@@ -118,8 +118,9 @@ def prefill_attention_topk(
         query, key, value, softmax_scale=softmax_scale, num_sink=num_sink, mode=1 if rows else 0, status=status
     )
     batch, length, heads, _ = out.shape
-    topk_val = torch.zeros((batch, heads, rows, TOPK), dtype=torch.float32, device=out.device)
-    topk_idx = torch.zeros((batch, heads, rows, TOPK), dtype=torch.int32, device=out.device)
+    # the kernel writes every entry
+    topk_val = torch.empty((batch, heads, rows, TOPK), dtype=torch.float32, device=out.device)
+    topk_idx = torch.empty((batch, heads, rows, TOPK), dtype=torch.int32, device=out.device)
     if rows:
         args.topk_val = topk_val.data_ptr()
         args.topk_idx = topk_idx.data_ptr()
