@@ -14,6 +14,7 @@ cudaError_t launch_append_kv(void* key_cache, void* value_cache, const void* new
 cudaError_t launch_wait_peers(uint32_t* flag, uint32_t expected, uint32_t* status, cudaStream_t stream);
 cudaError_t launch_nearest_centroid(const ckv_layer_args& a, int32_t* forced, cudaStream_t stream);
 bool fused_layer_supported(const ckv_layer_args& a);
+int fused_layer_clusters(int device, int splits, int group_size);
 cudaError_t launch_fused_layer(const ckv_layer_args& a, cudaStream_t stream);
 int attention_smem_bytes();
 cudaError_t launch_prefill(const ckv_prefill_args& a, cudaStream_t stream);
@@ -181,6 +182,16 @@ int ckv_decode_layer(const ckv_layer_args* args, void* cuda_stream) {
   status = ckv::launched(ckv::launch_attention(*args, stream));
   if (status != CKV_OK) return status;
   return ckv::launched(ckv::launch_merge_update(*args, stream));
+}
+
+int ckv_layer_clusters(int device, int splits, int group_size) {
+  if (splits < 1 || splits > 16 || group_size < 1 || group_size > 16) return 0;
+  int current = -1;
+  if (cudaGetDevice(&current) != cudaSuccess) return 0;
+  if (current != device && cudaSetDevice(device) != cudaSuccess) return 0;
+  const int clusters = ckv::fused_layer_clusters(device, splits, group_size);
+  if (current != device) cudaSetDevice(current);
+  return clusters;
 }
 
 int ckv_append_kv(void* key_cache, void* value_cache, const void* new_key, const void* new_value,

@@ -141,7 +141,7 @@ __device__ __forceinline__ float centroid_mean(float old_value, int old_size, fl
 
 // Optional phase timestamps of the single-launch decode path (see ckv_layer_args).
 __device__ __forceinline__ void phase_stamp(const ckv_layer_args& a, int flat, int rank, int slot) {
-  if (a.phase_times != nullptr && threadIdx.x == 0) {
+  if (a.phase_times != nullptr && threadIdx.x == 0 && rank < 8) {
     unsigned long long now;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
     a.phase_times[(static_cast<int64_t>(flat) * 8 + rank) * 16 + slot] = now;

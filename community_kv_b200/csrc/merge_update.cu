@@ -15,7 +15,7 @@ __global__ void __launch_bounds__(kMergeThreads + 32) merge_update_kernel(const 
   __shared__ float lse_s;
   pdl_release_dependents();
   pdl_wait_for_predecessor();  // partials and candidates come from the attention kernel
-  merge_update_unit(a, blockIdx.x, kMergeThreads / 32, decision, lse_s);
+  merge_update_unit<8>(a, blockIdx.x, kMergeThreads / 32, decision, lse_s);
   if (blockIdx.x == 0) {
     wait_for_peer_rows(a);
   }

@@ -7,7 +7,6 @@
 namespace ckv {
 
 constexpr int kMergeThreads = 128;
-constexpr int kMaxSplitsInFlight = 8;  // split rows a merging lane fetches at once
 
 struct UpdateDecision {
   int assigned;      // community id the new token joins (clamped to capacity-1)
@@ -42,6 +41,8 @@ __device__ __forceinline__ void wait_for_peer_rows(const ckv_layer_args& a) {
   }
 }
 
+// kInFlight: split rows that a merging lane fetches at once (eight in the stand-alone kernel: the
+// registers of sixteen would keep its CTAs from running beside the next layer's launch).
 // Warps 0 .. merge_warps-1 merge the split partials; warp `merge_warps` is the update
 // warp: it merges the neighbour candidates and fetches everything the online
 // assignment needs while the other warps are still merging, then applies the
@@ -49,6 +50,7 @@ __device__ __forceinline__ void wait_for_peer_rows(const ckv_layer_args& a) {
 // 128 threads and (merge_warps + 1) warps; `decision` and `lse_s` live in shared
 // memory.  Partials are read past the L1 cache: in the fused kernel other CTAs of
 // the cluster have just written them.
+template <int kInFlight>
 __device__ __forceinline__ void merge_update_unit(const ckv_layer_args& a, int flat, int merge_warps,
                                                   UpdateDecision& decision, float& lse_s) {
   const Unit u = make_unit(a, flat);
@@ -114,9 +116,9 @@ __device__ __forceinline__ void merge_update_unit(const ckv_layer_args& a, int f
                             static_cast<int64_t>(flat) * group * kHeadDim;
     for (int g = warp; g < group && !update_only; g += merge_warps) {
       // the accumulator rows do not depend on the (max, sum) pairs: fetch both at once
-      float4 rows[kMaxSplitsInFlight];
+      float4 rows[kInFlight];
 #pragma unroll
-      for (int s = 0; s < kMaxSplitsInFlight; ++s) {
+      for (int s = 0; s < kInFlight; ++s) {
         if (s < splits) {
           rows[s] = __ldcg(reinterpret_cast<const float4*>(
               partial + s * split_stride + g * kPartialStride + 4 * lane));
@@ -144,7 +146,7 @@ __device__ __forceinline__ void merge_update_unit(const ckv_layer_args& a, int f
       }
       float4 numerator = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int s = 0; s < kMaxSplitsInFlight; ++s) {
+      for (int s = 0; s < kInFlight; ++s) {
         if (s < splits) {
           const float w = __shfl_sync(0xffffffffu, weight, s);
           numerator.x += rows[s].x * w;
@@ -153,7 +155,7 @@ __device__ __forceinline__ void merge_update_unit(const ckv_layer_args& a, int f
           numerator.w += rows[s].w * w;
         }
       }
-      for (int s = kMaxSplitsInFlight; s < splits; ++s) {
+      for (int s = kInFlight; s < splits; ++s) {
         const float w = __shfl_sync(0xffffffffu, weight, s);
         const float4 v = __ldcg(reinterpret_cast<const float4*>(
             partial + s * split_stride + g * kPartialStride + 4 * lane));

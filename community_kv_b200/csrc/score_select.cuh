@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cstddef>
+#include <type_traits>
 
 #include "ckv_device.cuh"
 
@@ -888,6 +889,7 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+constexpr int kMaxCluster = 16;  // CTAs of a cluster, more than eight with the non-portable attribute
 constexpr int kClusterStageBytes = 2 * 16 * kHeadDim * 4 + 2 * kDescStash * 4;  // 32 KB
 
 struct ClusterSelectSmem {
@@ -987,8 +989,8 @@ __device__ __forceinline__ void select_cluster(const ckv_layer_args& a, int flat
   // Sum a pair of 256-bin histograms over the cluster.  Each thread owns 256 / kThreads
   // bins and reads every slice's values (all loads in flight together); it writes the sum
   // over all slices and the sum over the slices in front of this one.
-  constexpr int kMaxRanks = 8;
-  auto gather = [&](const int* mass, const int* count) {
+  auto gather_from = [&](auto max_ranks, const int* mass, const int* count) {
+    constexpr int kMaxRanks = decltype(max_ranks)::value;
     int part_mass[kBins][kMaxRanks];
     int part_count[kBins][kMaxRanks];
 #pragma unroll
@@ -1018,6 +1020,13 @@ __device__ __forceinline__ void select_cluster(const ckv_layer_args& a, int flat
       sm.before_count[tid + k * kThreads] = before_count;
     }
     __syncthreads();
+  };
+  auto gather = [&](const int* mass, const int* count) {
+    if (ranks <= 8) {
+      gather_from(std::integral_constant<int, 8>{}, mass, count);
+    } else {
+      gather_from(std::integral_constant<int, kMaxCluster>{}, mass, count);
+    }
   };
   // Warp 0: the threshold bin of the summed histogram, the totals above it, and the totals
   // above it of the slices in front of this one.

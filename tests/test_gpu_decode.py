@@ -95,6 +95,18 @@ def test_unfused_kernels_give_the_same_result(monkeypatch):
     _run_sequence(layer, config, steps=4, seed=100)
 
 
+@pytest.mark.parametrize("kv_heads,splits,expected", [(2, None, 16), (3, 11, 11), (1, 9, 9)])
+def test_more_than_eight_ctas_in_one_launch(kv_heads, splits, expected):
+    """A budget above 4096 on few heads: the launch uses a cluster of more than eight CTAs."""
+
+    layer = make_layer(seed=51, seq_len=12007, communities=301, kv_heads=kv_heads, max_decode_tokens=6,
+                       zipf_exponent=1.1)
+    config = CommunityKVConfig(token_budget=8192, num_sink=10, lam=0.5, aggregation="query_group")
+    state, twin = _run_sequence(layer, config, steps=4, seed=5100, splits=splits)
+    assert state.workspace.attention.splits == expected
+    assert native.library().ckv_decode_layer_kernels(ctypes.byref(state.args)) == 1
+
+
 @pytest.mark.parametrize("unfused", [False, True])
 def test_fixed_order_scores_are_bit_exact(monkeypatch, unfused):
     """``CKV_TENSOR_SCORES=0``: the CUDA-core scoring path sums in the fixed order the CPU restatement
