@@ -224,18 +224,14 @@ __device__ __forceinline__ uint32_t pack_bf16(float low, float high) {
   return *reinterpret_cast<const uint32_t*>(&pair);
 }
 
-__device__ __forceinline__ uint64_t shfl_xor_u64(uint64_t value, int mask) {
-  const uint32_t lo = __shfl_xor_sync(0xffffffffu, static_cast<uint32_t>(value), mask);
-  const uint32_t hi = __shfl_xor_sync(0xffffffffu, static_cast<uint32_t>(value >> 32), mask);
-  return (static_cast<uint64_t>(hi) << 32) | lo;
-}
+// Largest value of the warp: the high words, then the low words of those that hold it (two
+// warp reductions where ten shuffles stood; the top-8 merges of a layer do sixteen of these in
+// a chain: 31.3 -> 30.6 us for a layer of 8 heads, budget 2048).
 __device__ __forceinline__ uint64_t warp_max_u64(uint64_t value) {
-#pragma unroll
-  for (int offset = 16; offset > 0; offset >>= 1) {
-    const uint64_t other = shfl_xor_u64(value, offset);
-    value = other > value ? other : value;
-  }
-  return value;
+  const uint32_t mine = static_cast<uint32_t>(value >> 32);
+  const uint32_t high = __reduce_max_sync(0xffffffffu, mine);
+  const uint32_t low = __reduce_max_sync(0xffffffffu, mine == high ? static_cast<uint32_t>(value) : 0u);
+  return (static_cast<uint64_t>(high) << 32) | low;
 }
 
 // Newest-first member of a community's decode-delta chain, or 0 when the chain
