@@ -636,12 +636,12 @@ __global__ void __launch_bounds__(kPfThreads, 1)
 }
 
 // ---- exact top-m from the candidate lists (mode 2, second kernel) ----
-// One warp per (batch, KV head, position).  The G x 16 candidate keys are
-// re-scored as max over the group of scale * (q . k) in the fixed fp32 order
+// One warp per (batch, KV head, position).  The 16 candidate keys of each of its lists (two
+// from edge_candidates_kernel, one per head of the group otherwise) are re-scored as max over the group of scale * (q . k) in the fixed fp32 order
 // and ranked by (score descending, key index ascending).  A row is flagged when
 // a key that was turned away could still belong to the top-m: the best
 // approximate score among the dropped keys is within `slack` of the exact m-th.
-__global__ void __launch_bounds__(128) exact_edges_kernel(const ckv_prefill_args a, int group) {
+__global__ void __launch_bounds__(128) exact_edges_kernel(const ckv_prefill_args a, int group, int lists) {
   const int warps_per_block = 4;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -658,13 +658,13 @@ __global__ void __launch_bounds__(128) exact_edges_kernel(const ckv_prefill_args
   const int batch = static_cast<int>(item / (static_cast<int64_t>(rows) * a.kv_heads));
   const uint64_t* list = a.candidates +
                          ((static_cast<int64_t>(batch) * a.kv_heads + kv_head) * length + pos) *
-                             group * (kExactKeep + 1);
+                             lists * (kExactKeep + 1);
   const __nv_bfloat16* q_base = reinterpret_cast<const __nv_bfloat16*>(a.query) +
                                 batch * a.q_batch_stride + static_cast<int64_t>(pos) * a.q_row_stride +
                                 kv_head * group * a.q_head_stride;
   const __nv_bfloat16* k_base = reinterpret_cast<const __nv_bfloat16*>(a.key) +
                                 batch * a.k_batch_stride + kv_head * a.k_head_stride;
-  const int candidates = group * kExactKeep;  // <= 128
+  const int candidates = lists * kExactKeep;  // <= 128
   // the position's query rows, staged once per warp (every candidate reuses them)
   __shared__ uint4 q_stage[4][8 * 16];
   for (int index = lane; index < group * 16; index += 32) {
@@ -674,7 +674,7 @@ __global__ void __launch_bounds__(128) exact_edges_kernel(const ckv_prefill_args
   __syncwarp();
   uint64_t best_key[4];
   float best_dropped = -INFINITY;  // best approximate score among the keys turned away
-  if (lane < group) {
+  if (lane < lists) {
     const uint64_t lost = list[lane * (kExactKeep + 1) + kExactKeep];
     if (lost != 0ull) {
       best_dropped = key32_to_float(static_cast<uint32_t>(lost >> 32));
@@ -692,6 +692,9 @@ __global__ void __launch_bounds__(128) exact_edges_kernel(const ckv_prefill_args
       continue;
     }
     const int j = static_cast<int>(0xffffffffu - static_cast<uint32_t>(packed));
+    if (j < 0 || j > pos) {
+      continue;  // the lists of a launch that gave up a wait may hold anything
+    }
     const uint4* k_row = reinterpret_cast<const uint4*>(k_base + static_cast<int64_t>(j) * a.k_row_stride);
     uint4 k_reg[16];
 #pragma unroll
@@ -897,6 +900,10 @@ __global__ void __launch_bounds__(256) exact_rescan_kernel(const ckv_prefill_arg
 // each other their 16th score through shared memory (the position's 16th best is at
 // least the larger of the two, so anything clearly below it is turned away at once);
 // the two lists go to the candidate array that exact_edges_kernel re-scores.
+// Bound by the rounds of insertion (the product alone is a quarter of the time).  Their
+// number fell with the floor that both lists give together (8th of both: about the 16th of
+// the position, where either 16th is about its 32nd) and with halves of 32 columns where
+// pieces of 16 stood; 32 query on 8 KV heads, 6001 tokens: 1127 -> 1050 us for the whole call.
 constexpr int kEdgeThreads = 288;
 constexpr int kEdgeSub = 64;  // keys per sub-block
 
@@ -929,9 +936,14 @@ __device__ __forceinline__ uint64_t list_insert(uint64_t (&list)[kKeep], uint64_
   return lost;
 }
 
+// Score of a list entry, below everything for an empty one
+__device__ __forceinline__ float list_score(uint64_t entry) {
+  return entry == 0ull ? -INFINITY : key32_to_float(static_cast<uint32_t>(entry >> 32));
+}
+
 struct EdgeSmem {
   static constexpr int kQ = 0;                       // kGroup tiles
-  static constexpr int kBarBytes = 128 + 2 * kPfRows * 4;  // barriers, then the floors
+  static constexpr int kBarBytes = 128 + 4 * kPfRows * 4;  // barriers, then the floors
   static constexpr int total(int group) { return (group + 2) * kTileBytes + kBarBytes; }
 };
 
@@ -947,7 +959,7 @@ __global__ void __launch_bounds__(kEdgeThreads, 1)
   uint8_t* s_k = smem + kGroup * kTileBytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (kGroup + 2) * kTileBytes);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
-  volatile float* floors = reinterpret_cast<volatile float*>(bars + 16);  // [2][128]
+  volatile float* floors = reinterpret_cast<volatile float*>(bars + 16);  // [16th, 8th][list][128]
   const uint32_t bar_q = smem_u32(bars);           // Q tiles landed
   const uint32_t bar_k_full = smem_u32(bars + 1);  // two: K buffer filled
   const uint32_t bar_k_free = smem_u32(bars + 3);  // two: every MMA reading the K buffer is done
@@ -967,6 +979,7 @@ __global__ void __launch_bounds__(kEdgeThreads, 1)
 
   if (tid < 2 * kPfRows) {
     floors[tid] = -INFINITY;
+    floors[2 * kPfRows + tid] = -INFINITY;
   }
   if (tid == 0) {
     mbar_init(bar_q, 1);
@@ -1077,24 +1090,26 @@ __global__ void __launch_bounds__(kEdgeThreads, 1)
       tc_fence_after();
       const int key0 = sb * kEdgeSub;
       const bool plain = key0 + kEdgeSub - 1 <= pos0 && key0 >= a.num_sink;  // no mask, no sinks
-      const uint64_t last = list[kKeep - 1];
-      const float own_floor =
-          last == 0ull ? -INFINITY : key32_to_float(static_cast<uint32_t>(last >> 32));
+      // A key clearly below 16 keys already held at this position (in either list) cannot be
+      // one of its 16 best: below either list's 16th, or below the 8th of both.  The partner's
+      // values are read a little low; any earlier value of theirs is also valid.
+      const float own_floor = list_score(list[kKeep - 1]);
+      const float own_middle = list_score(list[kKeep / 2 - 1]);
       floors[wg * kPfRows + row] = own_floor;
-      // the other list's 16th score, a little low (any earlier value is also valid)
-      const float partner_floor = floors[(wg ^ 1) * kPfRows + row] - 2.0f * a.exact_slack;
-      float floor_score = fmaxf(own_floor, partner_floor);
-      // the next chunk's scores are requested before this chunk's list work and waited
-      // for after it
-      uint32_t raw[kGroup][16];
+      floors[(2 + wg) * kPfRows + row] = own_middle;
+      const float margin = 2.0f * a.exact_slack;
+      const float shared_floor = fmaxf(floors[(wg ^ 1) * kPfRows + row],
+                                       fminf(own_middle, floors[(2 + (wg ^ 1)) * kPfRows + row])) - margin;
+      float floor_score = fmaxf(own_floor, shared_floor);
+      float best[kEdgeSub];
 #pragma unroll
-      for (int h = 0; h < kGroup; ++h) {
-        tmem_load16_issue(lane_base + h * kEdgeSub, raw[h]);
-      }
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll 1
       for (int c0 = 0; c0 < kEdgeSub; c0 += 16) {
-        float best[16];
+        uint32_t raw[kGroup][16];
+#pragma unroll
+        for (int h = 0; h < kGroup; ++h) {
+          tmem_load16_issue(lane_base + h * kEdgeSub + c0, raw[h]);
+        }
+        tmem_wait_load();
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           float m = __uint_as_float(raw[0][i]);
@@ -1102,69 +1117,69 @@ __global__ void __launch_bounds__(kEdgeThreads, 1)
           for (int h = 1; h < kGroup; ++h) {
             m = fmaxf(m, __uint_as_float(raw[h][i]));
           }
-          const int j = key0 + c0 + i;
-          const bool visible = plain || (j <= row_pos && j >= a.num_sink);
-          best[i] = visible ? m * a.softmax_scale : -INFINITY;
+          best[c0 + i] = m * a.softmax_scale;
         }
-        if (c0 + 16 < kEdgeSub) {
+      }
+      // the scores are in registers: the next product may overwrite the buffer
+      tc_fence_before();
+      mbar_arrive(bar_s_free + 8 * wg);
+      if (!plain) {
 #pragma unroll
-          for (int h = 0; h < kGroup; ++h) {
-            tmem_load16_issue(lane_base + h * kEdgeSub + c0 + 16, raw[h]);
-          }
+        for (int i = 0; i < kEdgeSub; ++i) {
+          const int j = key0 + i;
+          best[i] = j <= row_pos && j >= a.num_sink ? best[i] : -INFINITY;
         }
-        // Columns that beat the floor, as a bit mask.  The lanes then insert in
-        // rounds: in every round each lane that still has such a column inserts its
-        // next one, so a chunk costs as many passes over the insertion code as the
-        // busiest lane has columns, not as many as there are columns with a taker.
+      }
+      // Columns that beat the floor, as a bit mask, 32 at a time.  The lanes then insert in
+      // rounds: in every round each lane that still has such a column inserts its
+      // next one, so a half costs as many passes over the insertion code as the
+      // busiest lane has columns, not as many as there are columns with a taker.
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
         uint32_t takers = 0u;
         float rejected = -INFINITY;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const bool take = row_live && best[i] > floor_score;
+        for (int i = 0; i < 32; ++i) {
+          const bool take = row_live && best[half * 32 + i] > floor_score;
           takers |= (take ? 1u : 0u) << i;
-          rejected = fmaxf(rejected, take ? -INFINITY : best[i]);
+          rejected = fmaxf(rejected, take ? -INFINITY : best[half * 32 + i]);
         }
         dropped = fmaxf(dropped, rejected);
         while (__any_sync(0xffffffffu, takers != 0u)) {
-          if (takers != 0u) {
-            const int i = __ffs(takers) - 1;
-            takers &= takers - 1;
-            // the column's score by a binary tree over the index bits (four selects deep)
-            float pick[8];
+          // every lane runs the same instructions: one without a column inserts zero
+          const int i = __ffs(takers) - 1;
+          const bool pending = takers != 0u;
+          takers &= takers - 1;
+          // the column's score by a binary tree over the index bits (five selects deep)
+          float pick[16];
 #pragma unroll
-            for (int m = 0; m < 8; ++m) pick[m] = (i & 1) ? best[2 * m + 1] : best[2 * m];
+          for (int m = 0; m < 16; ++m) {
+            pick[m] = (i & 1) ? best[half * 32 + 2 * m + 1] : best[half * 32 + 2 * m];
+          }
 #pragma unroll
-            for (int m = 0; m < 4; ++m) pick[m] = (i & 2) ? pick[2 * m + 1] : pick[2 * m];
+          for (int width = 8, bit = 2; width >= 1; width >>= 1, bit <<= 1) {
 #pragma unroll
-            for (int m = 0; m < 2; ++m) pick[m] = (i & 4) ? pick[2 * m + 1] : pick[2 * m];
-            const float v = (i & 8) ? pick[1] : pick[0];
-            if (v > floor_score) {
-              const uint64_t candidate = (static_cast<uint64_t>(ordered_key32(v)) << 32) |
-                                         (0xffffffffu - static_cast<uint32_t>(key0 + c0 + i));
-              const uint64_t lost = list_insert<kKeep>(list, candidate);
-              if (lost != 0ull) {
-                dropped = fmaxf(dropped, key32_to_float(static_cast<uint32_t>(lost >> 32)));
-              }
-              const uint64_t tail = list[kKeep - 1];
-              floor_score = fmaxf(
-                  partner_floor,
-                  tail == 0ull ? -INFINITY : key32_to_float(static_cast<uint32_t>(tail >> 32)));
-            } else {
-              dropped = fmaxf(dropped, v);
+            for (int m = 0; m < width; ++m) {
+              pick[m] = (i & bit) ? pick[2 * m + 1] : pick[2 * m];
             }
           }
+          const float v = pick[0];
+          const bool enters = pending && v > floor_score;
+          const uint64_t candidate =
+              enters ? (static_cast<uint64_t>(ordered_key32(v)) << 32) |
+                           (0xffffffffu - static_cast<uint32_t>(key0 + half * 32 + i))
+                     : 0ull;
+          const uint64_t lost = list_insert<kKeep>(list, candidate);
+          dropped = fmaxf(dropped, pending && !enters ? v : list_score(lost));
+          floor_score = fmaxf(shared_floor, list_score(list[kKeep - 1]));
         }
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       }
-      tc_fence_before();
-      mbar_arrive(bar_s_free + 8 * wg);
     }
     if (row_live && !failed) {
-      // [batch, kv head, position, G lanes, 16 kept + best dropped]: this thread's list
-      // is lane `wg` (the other lanes stay empty)
+      // [batch, kv head, position, 2 lists, 16 kept + best dropped]: this thread's is list `wg`
       uint64_t* out = a.candidates +
                       ((static_cast<int64_t>(batch) * gridDim.y + kv_head) * length + row_pos) *
-                          kGroup * (kExactKeep + 1);
+                          2 * (kExactKeep + 1);
 #pragma unroll
       for (int k = 0; k < kKeep; ++k) {
         out[wg * (kExactKeep + 1) + k] = list[k];
@@ -1305,7 +1320,8 @@ cudaError_t launch_prefill(const ckv_prefill_args& a, cudaStream_t stream) {
     return cudaSuccess;
   }
   const int64_t items = static_cast<int64_t>(a.batch) * a.kv_heads * rows;
-  exact_edges_kernel<<<static_cast<unsigned>((items + 3) / 4), 128, 0, stream>>>(a, group);
+  const int lists = group == 2 || group == 4 ? 2 : group;
+  exact_edges_kernel<<<static_cast<unsigned>((items + 3) / 4), 128, 0, stream>>>(a, group, lists);
   err = cudaGetLastError();
   if (err != cudaSuccess || a.edge_flags == nullptr) {
     return err;

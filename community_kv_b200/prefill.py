@@ -165,11 +165,13 @@ def prefill_attention_edges(
     kv_heads = keep[1].shape[2]
     group = heads // kv_heads
     device = out.device
-    candidates = torch.zeros((batch, kv_heads, length, group, EXACT_KEEP + 1), dtype=torch.int64, device=device)
-    edge_idx = torch.full((batch, kv_heads, rows, edges_per_row), -1, dtype=torch.int32, device=device)
-    edge_score = torch.zeros((batch, kv_heads, rows, edges_per_row), dtype=torch.float32, device=device)
-    flags = torch.zeros((batch, kv_heads, rows), dtype=torch.int32, device=device)
-    rescan_list = torch.zeros((1 + batch * kv_heads * rows,), dtype=torch.int32, device=device)
+    # the kernels write every entry that they or the caller read; only the queue starts empty
+    candidates = torch.empty((batch, kv_heads, length, group, EXACT_KEEP + 1), dtype=torch.int64, device=device)
+    edge_idx = torch.empty((batch, kv_heads, rows, edges_per_row), dtype=torch.int32, device=device)
+    edge_score = torch.empty((batch, kv_heads, rows, edges_per_row), dtype=torch.float32, device=device)
+    flags = torch.empty((batch, kv_heads, rows), dtype=torch.int32, device=device)
+    rescan_list = torch.empty((1 + batch * kv_heads * rows,), dtype=torch.int32, device=device)
+    rescan_list[:1].zero_()
     if rows:
         native.fill(
             args,

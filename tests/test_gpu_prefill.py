@@ -270,3 +270,48 @@ def test_full_size_reference_topk_rule():
         want_val = torch.exp(chosen * SCALE - lse[0, :, row].unsqueeze(1))
         torch.testing.assert_close(got_val, want_val, rtol=3e-2, atol=1e-9)
     assert exact_rows / (len(rows) * heads) > 0.9, exact_rows / (len(rows) * heads)
+
+
+@pytest.mark.parametrize("length,heads,kv_heads,sinks", [(517, 4, 1, 10), (385, 2, 1, 0), (300, 4, 2, 70), (401, 8, 2, 150)])
+def test_reference_topk_rule_with_ties(length, heads, kv_heads, sinks):
+    """Whole-number scores: every product and sum is exact, so the neighbours are the oracle's without any
+    allowance.  Most keys tie, so the gates in front of the insertion and the order among equal keys decide
+    every row; the sinks end inside the first key block, in its upper half and in the second block."""
+
+    generator = torch.Generator().manual_seed(length)
+    q = torch.randint(-1, 2, (1, length, heads, 128), generator=generator).to(torch.bfloat16)
+    k = torch.randint(-1, 2, (1, length, kv_heads, 128), generator=generator).to(torch.bfloat16)
+    v = torch.randint(-1, 2, (1, length, kv_heads, 128), generator=generator).to(torch.bfloat16)
+    *_, idx = prefill_attention_topk(q.cuda(), k.cuda(), v.cuda(), softmax_scale=SCALE, num_sink=sinks)
+    _, want_lse, raw = oracle.causal_attention(q[0].float().numpy(), k[0].float().numpy(), v[0].float().numpy(), SCALE)
+    for head in range(heads):
+        want_idx = oracle.reference_topk(raw[head], want_lse[head], SCALE, sinks)[1]
+        assert np.array_equal(idx[0, head].cpu().numpy(), want_idx), head
+
+
+@pytest.mark.parametrize("room,shift", [(0, 0), (24, 0), (24, 4)])
+def test_plugin_prefill_reads_the_cache_where_it_lies(room, shift):
+    """``[B, H, S, D]`` tensors with unused rows, and off the 16-byte boundary that the tile copies need."""
+
+    from types import SimpleNamespace
+
+    from community_kv_b200 import CommunityKVAttention, CommunityKVConfig, CommunityKVRuntime, PartitionConfig
+
+    length, heads, kv_heads = 200, 4, 2
+    q, k, v = _inputs(8, length, heads, kv_heads)
+    want = prefill_attention_topk(q.cuda(), k.cuda(), v.cuda(), softmax_scale=SCALE, num_sink=10)
+
+    def placed(tensor, rows):
+        whole = torch.zeros((tensor.shape[2] * rows * 128 + shift,), dtype=torch.bfloat16, device="cuda")
+        view = whole[shift:].view(1, tensor.shape[2], rows, 128)
+        view[:, :, :length] = tensor.cuda().transpose(1, 2)
+        return view
+
+    edges = {}
+    runtime = CommunityKVRuntime(config=CommunityKVConfig(num_sink=10), partition=PartitionConfig(), num_layers=1,
+                                 max_decode_tokens=8, partitioner=lambda **found: edges.update(found))
+    runtime.start_request()
+    out, _ = CommunityKVAttention(runtime).forward(
+        SimpleNamespace(layer_idx=0), placed(q, length), placed(k, length + room), placed(v, length + room), None, SCALE)
+    assert torch.equal(out, want[0])
+    assert torch.equal(edges["topk_indices"], want[5][0]) and torch.equal(edges["topk_scores"], want[4][0])
