@@ -78,7 +78,8 @@ def choose_splits(token_budget: int, units: int, requested: int | None = None) -
         wanted = requested
     else:
         wanted = max(1, RESIDENT_ATTENTION_CTAS // max(units, 1))
-        # Up to eight splits the whole layer is one cluster launch; more only pay off when
+        # Up to eight splits (sixteen where the device allows it, see ops.layer_splits) the whole
+        # layer is one cluster launch; more only pay off when
         # a split would otherwise have to walk through more than 512 tokens.
         if wanted > 8 and token_budget // 8 <= 512:
             wanted = 8
