@@ -172,6 +172,16 @@ def test_nearest_centroid_assignment_variant(aggregation, defer):
         CommunityKVConfig(online_assignment="nearest")
 
 
+@pytest.mark.parametrize("communities", [255, 257, 1301])
+def test_nearest_centroid_over_many_communities(communities):
+    """Around one row per lane group of the cluster (256 rows), and more rows than are in flight at once."""
+
+    layer = make_layer(seed=communities, seq_len=8192, communities=communities, kv_heads=2, max_decode_tokens=6)
+    config = CommunityKVConfig(token_budget=512, num_sink=10, lam=0.5, aggregation="query_group",
+                               online_assignment="nearest_centroid")
+    _run_sequence(layer, config, steps=4, seed=2400)
+
+
 @pytest.mark.parametrize("aggregation", [GraphAggregation.QUERY_GROUP, GraphAggregation.LAYER_WISE])
 def test_fp32_centroid_table(aggregation):
     """Not the reference's layout: the centroid table in fp32.  The scores (fixed-order sum of products
