@@ -112,9 +112,13 @@ class PrefillCSR:
             raise ValueError("community_counts must have one entry per graph")
         if self.member_positions.shape[0] != graphs:
             raise ValueError("member_positions must have one row per graph")
-        # compared where the tensors are: on the host a comparison of this size is shared out over
-        # every core, and waking those costs milliseconds
         offsets, width = self.member_offsets, self.community_capacity
+        if graphs == 0:
+            return
+        if width < 0:
+            raise ValueError("community count exceeds offset capacity")
+        # compared where the offsets are: on the host a comparison of this size is shared out over
+        # every core, and waking those costs milliseconds
         counts = self.community_counts.unsqueeze(1)
         outside = (counts < 0) | (counts > width)
         falls = (offsets[:, 1:] < offsets[:, :-1]) & (torch.arange(width, device=offsets.device) < counts)

@@ -26,6 +26,7 @@ from community_kv_b200.state import (
     CentroidSelectionWorkspace,
     DecodeDeltaChunks,
     DecodeLayerWorkspace,
+    PrefillCSR,
     choose_splits,
 )
 from community_kv_b200.synthetic import make_layer
@@ -158,6 +159,27 @@ def test_delta_chunks_grow_geometrically():
     small.append(0, 0, 5)
     with pytest.raises(RuntimeError, match="exhausted"):
         small.append(0, 1, 6)
+
+
+def test_member_lists_are_checked():
+    def csr(offsets, counts, width=6):
+        return PrefillCSR(torch.tensor(offsets, dtype=torch.int32), torch.zeros((len(counts), width), dtype=torch.int32),
+                          torch.tensor(counts, dtype=torch.int32))
+
+    csr([[0, 2, 5, 1], [0, 0, 6, 6]], [2, 3]).validate()  # behind a graph's own count anything goes
+    csr([[0], [0]], [0, 0]).validate()
+    PrefillCSR(torch.zeros((0, 0), dtype=torch.int32), torch.zeros((0, 4), dtype=torch.int32),
+               torch.zeros((0,), dtype=torch.int32)).validate()
+    for offsets, counts, message in (
+        ([[0, 2], [0, 2]], [1, 2], "count exceeds"),
+        ([[0, 2], [0, 2]], [-1, 1], "count exceeds"),
+        ([[], []], [0, 0], "count exceeds"),
+        ([[1, 2], [0, 2]], [0, 1], "start at zero"),
+        ([[0, 3, 2], [0, 1, 2]], [2, 2], "start at zero"),
+        ([[0, 3, 7], [0, 1, 2]], [2, 2], "member-position capacity"),
+    ):
+        with pytest.raises(ValueError, match=message):
+            csr(offsets, counts).validate()
 
 
 # ---- conversion and runtime bookkeeping (reference test_runtime.py:205-319) --------------------
