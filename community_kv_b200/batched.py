@@ -155,8 +155,7 @@ def stack_sequences(
         score_community_counts=counts,
         score_headroom=first.decode_capacity,
         batch=batch,
-        splits=ops.layer_splits(token_budget=budget, state=mutable, group_size=first.group_size, batch=batch,
-                                requested=splits),
+        splits=splits,
         max_communities=max_communities,
     )
     return BatchedLayerState(

@@ -13,9 +13,8 @@ cudaError_t launch_append_kv(void* key_cache, void* value_cache, const void* new
                              int64_t row_index_stride, int64_t row, cudaStream_t stream);
 cudaError_t launch_wait_peers(uint32_t* flag, uint32_t expected, uint32_t* status, cudaStream_t stream);
 cudaError_t launch_nearest_centroid(const ckv_layer_args& a, int32_t* forced, cudaStream_t stream);
-bool fused_layer_supported(const ckv_layer_args& a);
-int fused_layer_clusters(int device, int splits, int group_size);
-cudaError_t launch_fused_layer(const ckv_layer_args& a, cudaStream_t stream);
+int fused_layer_ctas(const ckv_layer_args& a);
+cudaError_t launch_fused_layer(const ckv_layer_args& a, int ctas, cudaStream_t stream);
 int attention_smem_bytes();
 cudaError_t launch_prefill(const ckv_prefill_args& a, cudaStream_t stream);
 
@@ -168,9 +167,10 @@ int ckv_decode_layer(const ckv_layer_args* args, void* cuda_stream) {
   status = ckv::select_device(args);
   if (status != CKV_OK) return status;
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
-  if (ckv::fused_layer_supported(*args)) {
+  const int ctas = ckv::fused_layer_ctas(*args);
+  if (ctas > 0) {
     // one cluster launch per layer: scoring, selection, attention, merge and update
-    if (ckv::launch_fused_layer(*args, stream) == cudaSuccess) return CKV_OK;
+    if (ckv::launch_fused_layer(*args, ctas, stream) == cudaSuccess) return CKV_OK;
     // the cluster shape could not be scheduled on this device: clear the error and
     // run the four kernels instead (same results)
     (void)cudaGetLastError();
@@ -182,16 +182,6 @@ int ckv_decode_layer(const ckv_layer_args* args, void* cuda_stream) {
   status = ckv::launched(ckv::launch_attention(*args, stream));
   if (status != CKV_OK) return status;
   return ckv::launched(ckv::launch_merge_update(*args, stream));
-}
-
-int ckv_layer_clusters(int device, int splits, int group_size) {
-  if (splits < 1 || splits > 16 || group_size < 1 || group_size > 16) return 0;
-  int current = -1;
-  if (cudaGetDevice(&current) != cudaSuccess) return 0;
-  if (current != device && cudaSetDevice(device) != cudaSuccess) return 0;
-  const int clusters = ckv::fused_layer_clusters(device, splits, group_size);
-  if (current != device) cudaSetDevice(current);
-  return clusters;
 }
 
 int ckv_append_kv(void* key_cache, void* value_cache, const void* new_key, const void* new_value,
@@ -234,7 +224,7 @@ int ckv_nearest_centroid(const ckv_layer_args* args, int32_t* forced_community, 
 
 int ckv_decode_layer_kernels(const ckv_layer_args* args) {
   if (args == nullptr) return CKV_ERR_NULL;
-  if (ckv::fused_layer_supported(*args)) return 1;
+  if (ckv::fused_layer_ctas(*args) > 0) return 1;
   return (args->retrieval_heads != args->graphs && !(args->flags & CKV_FLAG_SKIP_UPDATE)) ? 5 : 4;
 }
 

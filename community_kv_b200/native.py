@@ -180,7 +180,6 @@ ENTRY_POINTS = (
     "ckv_select_descriptors",
     "ckv_segmented_attention",
     "ckv_decode_layer",
-    "ckv_layer_clusters",
     "ckv_decode_layer_kernels",
     "ckv_attention_smem_bytes",
     "ckv_segmented_attention_static",
@@ -228,8 +227,6 @@ def library() -> ctypes.CDLL:
         function = getattr(lib, name)
         function.restype = ctypes.c_int
         function.argtypes = [ctypes.POINTER(LayerArgs), ctypes.c_void_p]
-    lib.ckv_layer_clusters.restype = ctypes.c_int
-    lib.ckv_layer_clusters.argtypes = [ctypes.c_int] * 3
     lib.ckv_decode_layer_kernels.restype = ctypes.c_int
     lib.ckv_decode_layer_kernels.argtypes = [ctypes.POINTER(LayerArgs)]
     lib.ckv_append_kv.restype = ctypes.c_int
@@ -255,13 +252,6 @@ def library() -> ctypes.CDLL:
     lib.ckv_prefill_topk.restype = ctypes.c_int
     lib.ckv_prefill_topk.argtypes = [ctypes.POINTER(PrefillArgs), ctypes.c_void_p]
     return lib
-
-
-@functools.cache
-def layer_clusters(device: int, splits: int, group_size: int) -> int:
-    """Units one decode-layer launch works on at a time with ``splits`` CTAs each (0: impossible)."""
-
-    return library().ckv_layer_clusters(device, splits, group_size)
 
 
 def pointer(tensor: torch.Tensor | None) -> int | None:
@@ -305,7 +295,6 @@ __all__ = [
     "call",
     "current_stream",
     "fill",
-    "layer_clusters",
     "library",
     "pointer",
 ]

@@ -27,11 +27,7 @@ from community_kv_b200.state import (
     PackedSegments,
     PrefillCSR,
     SegmentedAttentionWorkspace,
-    choose_splits,
 )
-
-MAX_CLUSTER = 16  # CTAs of a thread-block cluster (above eight: not on every device)
-CLUSTER_ROWS = 4608  # communities whose keys and sizes one CTA of the launch can hold
 
 
 def _require_cuda(*tensors: torch.Tensor) -> torch.device:
@@ -496,32 +492,6 @@ def segmented_attention_static(
     return workspace.output, workspace.lse, workspace.topk_scores, workspace.topk_positions
 
 
-def layer_splits(
-    *, token_budget: int, state: MutableGraphState, group_size: int, batch: int = 1, requested: int | None = None
-) -> int:
-    """Attention CTAs per retrieval head of a layer that ``ckv_decode_layer`` runs.
-
-    ``choose_splits`` goes beyond eight CTAs for budgets above 4096 on few heads.  Where the layer
-    can be one launch, a cluster of up to sixteen then does better than 32 CTAs and four kernels
-    (8 heads, budget 8192, a million tokens: 56 us against 65 us a layer); the size is the largest
-    of which all heads' clusters are resident at once.  Up to budget 4096 eight CTAs are as
-    good as sixteen (37.8 us against 37.1 us, and 31.3 us against 32.8 us at budget 2048).
-    """
-
-    units = batch * state.retrieval_head_count
-    splits = choose_splits(token_budget, units, requested)
-    device = state.centroids.device
-    if requested or splits <= 8 or device.type != "cuda":
-        return splits
-    if state.graph_count != state.retrieval_head_count or state.centroids.dtype != torch.float8_e4m3fn:
-        return splits  # four kernels in any case
-    for wanted in range(MAX_CLUSTER, 8, -1):
-        rows = 16 * -(-state.community_capacity // (16 * wanted))
-        if rows <= CLUSTER_ROWS and native.layer_clusters(device.index or 0, wanted, group_size) >= units:
-            return wanted
-    return splits
-
-
 def tensor_scores_enabled() -> bool:
     """Centroid scoring on the tensor cores (the default); ``CKV_TENSOR_SCORES=0`` selects the
     fixed-order CUDA-core sum, which a CPU can reproduce bit for bit."""
@@ -735,7 +705,6 @@ __all__ = [
     "append_kv",
     "build_layer_args",
     "decode_layer",
-    "layer_splits",
     "score_and_select",
     "score_centroids",
     "segmented_attention",

@@ -305,8 +305,7 @@ class DecodeRuntime:
                 device=device,
                 score_community_counts=converted.initial_community_counts,
                 score_headroom=converted.decode_capacity,
-                splits=ops.layer_splits(
-                    token_budget=budget, state=mutable, group_size=converted.group_size, requested=self.splits),
+                splits=self.splits,
                 max_communities=self.max_communities,
             ),
             sink_positions=torch.arange(self.config.num_sink, dtype=torch.int32, device=device),

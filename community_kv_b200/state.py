@@ -65,21 +65,21 @@ RESIDENT_ATTENTION_CTAS = 3 * 148  # three attention CTAs fit one SM; a B200 has
 
 
 def choose_splits(token_budget: int, units: int, requested: int | None = None) -> int:
-    """Attention CTAs per retrieval head.
+    """Pieces that a retrieval head's tokens are cut into for the attention.
 
-    By default the (sequence, head) units of one launch share a single wave of
-    resident CTAs; a head's tokens are cut into 16-token steps, so at most
-    ``token_budget // 16`` (and never more than 32) CTAs can work on one head.
-    With few units the default stops at eight, the largest thread-block cluster,
-    so that ``ckv_decode_layer`` stays a single launch.
+    The partial results of the pieces are merged in order, so this number fixes every bit of a
+    layer's output; how many CTAs share them is up to the library.  By default the
+    (sequence, head) units of one launch share a single wave of resident CTAs; a head's tokens
+    are cut into 16-token steps, so at most ``token_budget // 16`` (and never more than 32)
+    pieces are possible.  With few units the default stops at eight, the largest portable
+    thread-block cluster, so that ``ckv_decode_layer`` is a single launch with one piece per CTA.
     """
 
     if requested:
         wanted = requested
     else:
         wanted = max(1, RESIDENT_ATTENTION_CTAS // max(units, 1))
-        # Up to eight splits (sixteen where the device allows it, see ops.layer_splits) the whole
-        # layer is one cluster launch; more only pay off when
+        # Up to eight splits the whole layer is one cluster launch; more only pay off when
         # a split would otherwise have to walk through more than 512 tokens.
         if wanted > 8 and token_budget // 8 <= 512:
             wanted = 8

@@ -275,16 +275,14 @@ int ckv_select_descriptors(const ckv_layer_args* args, void* cuda_stream);
 int ckv_segmented_attention(const ckv_layer_args* args, void* cuda_stream);
 
 /* A1..A5 back to back: the whole per-layer decode transition.  With one graph per
- * retrieval head, at most sixteen splits and descriptors that fit the selection's
- * shared-memory list, this is ONE launch: a thread-block cluster per (sequence,
+ * retrieval head, at most eight splits and communities that fit the selection's
+ * shared-memory stash, this is ONE launch: a thread-block cluster per (sequence,
  * retrieval head) scores, selects, attends, merges and updates, synchronising
- * through cluster barriers.  Otherwise (or with CKV_FLAG_UNFUSED) the four
- * stand-alone kernels run back to back.  Results are identical either way. */
+ * through cluster barriers.  With more splits it is one launch of up to sixteen CTAs
+ * per unit where that was measured to be the faster route.  Otherwise (or with
+ * CKV_FLAG_UNFUSED) the four stand-alone kernels run back to back.  Results are
+ * identical either way. */
 int ckv_decode_layer(const ckv_layer_args* args, void* cuda_stream);
-
-/* How many (sequence, retrieval head) units that one launch works on at a time when
- * every unit has `splits` CTAs; 0 if a cluster of that size cannot run at all. */
-int ckv_layer_clusters(int device, int splits, int group_size);
 
 /* Writes the decoded token's K and V rows into the caches: cache[u, row, :] = new[u, :]
  * for u < units, where the caches are bf16 [units, rows, 128] with `unit_stride`

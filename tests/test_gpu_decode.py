@@ -95,16 +95,61 @@ def test_unfused_kernels_give_the_same_result(monkeypatch):
     _run_sequence(layer, config, steps=4, seed=100)
 
 
-@pytest.mark.parametrize("kv_heads,splits,expected", [(2, None, 16), (3, 11, 11), (1, 9, 9)])
-def test_more_than_eight_ctas_in_one_launch(kv_heads, splits, expected):
-    """A budget above 4096 on few heads: the launch uses a cluster of more than eight CTAs."""
+@pytest.mark.parametrize("kv_heads,splits,expected,kernels", [(2, None, 32, 4), (3, 11, 11, 1), (1, 9, 9, 1)])
+def test_more_than_eight_splits(kv_heads, splits, expected, kernels):
+    """A budget above 4096 on few heads: the default number of splits, and a cluster of more than eight CTAs."""
 
     layer = make_layer(seed=51, seq_len=12007, communities=301, kv_heads=kv_heads, max_decode_tokens=6,
                        zipf_exponent=1.1)
     config = CommunityKVConfig(token_budget=8192, num_sink=10, lam=0.5, aggregation="query_group")
     state, twin = _run_sequence(layer, config, steps=4, seed=5100, splits=splits)
     assert state.workspace.attention.splits == expected
-    assert native.library().ckv_decode_layer_kernels(ctypes.byref(state.args)) == 1
+    assert native.library().ckv_decode_layer_kernels(ctypes.byref(state.args)) == kernels
+
+
+@pytest.mark.parametrize(
+    "batch,kv_heads,group,splits,communities,kernels",
+    [
+        (1, 2, 4, None, 20000, 1),  # the default of 32 splits over sixteen CTAs
+        (1, 1, 1, 17, 20000, 1),    # nine CTAs, two splits but for one
+        (1, 2, 8, 31, 20000, 1),    # sixteen CTAs, two splits but for one
+        (1, 2, 4, 32, 300, 4),      # few communities: four kernels
+        (1, 20, 2, 16, 300, 1),     # 320 of 444 CTA slots
+        (1, 21, 2, 16, 300, 4),     # 336: no room for the next launch
+        (1, 2, 16, 16, 300, 4),     # two blocks of query heads
+        (3, 4, 4, 13, 300, 1),      # a batch
+        (3, 9, 4, None, 300, 4),    # 27 units: sixteen splits, all the slots
+    ],
+)
+def test_splits_alone_decide_the_bits(monkeypatch, batch, kv_heads, group, splits, communities, kernels):
+    """However many CTAs share the splits, output and state are those of the four stand-alone kernels."""
+
+    device = torch.device("cuda", 0)
+    config = CommunityKVConfig(token_budget=8192, num_sink=10, lam=0.5, aggregation="query_group")
+    length = 40000 if communities > 1000 else 9001
+    layers = [make_layer(seed=70 + b, seq_len=length, communities=communities, kv_heads=kv_heads, group_size=group,
+                         max_decode_tokens=6) for b in range(batch)]
+    key = torch.stack([layer.key for layer in layers]).to(device)
+    value = torch.stack([layer.value for layer in layers]).to(device)
+
+    def run(unfused):
+        monkeypatch.setenv("CKV_UNFUSED", unfused)
+        runtime = BatchedDecodeRuntime(config, splits=splits)
+        state = runtime.prepare_layer(0, [convert_prefill_tensors(**layer.to(device).prepare_kwargs()) for layer in layers])
+        outputs = []
+        for step in range(4):
+            query = torch.stack([make_query(seed=80 + 10 * step + b, query_heads=kv_heads * group) for b in range(batch)])
+            outputs.append(runtime.decode(layer_idx=0, query=query.to(device), key=key, value=value,
+                                          softmax_scale=SCALE).clone())
+        ws = state.workspace.attention
+        launched = native.library().ckv_decode_layer_kernels(ctypes.byref(state.args))
+        return launched, [*outputs, ws.lse, ws.topk_scores, ws.topk_positions, *state.mutable.tensors()]
+
+    four, want = run("1")
+    launched, got = run("0")
+    assert (four, launched) == (4, kernels)
+    for first, second in zip(got, want):
+        assert torch.equal(first.contiguous().view(torch.uint8), second.contiguous().view(torch.uint8))
 
 
 @pytest.mark.parametrize("unfused", [False, True])
