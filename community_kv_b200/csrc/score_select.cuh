@@ -3,7 +3,6 @@
 #pragma once
 
 #include <cstddef>
-#include <type_traits>
 
 #include "ckv_device.cuh"
 
@@ -936,7 +935,8 @@ __device__ __forceinline__ void cluster_select_begin(ClusterSelectSmem& sm) {
 // this; on return sm.desc_* hold all descriptors and the logical tokens
 // [token_begin, token_end) are resolved to cache rows.
 // `guess_bin`: the high-byte bin score_groups counted the low bytes of (-1: none).
-template <int kThreads>
+// kMaxRanks: the cluster has at most that many CTAs (registers of the histogram exchange).
+template <int kThreads, int kMaxRanks>
 __device__ __forceinline__ void select_cluster(const ckv_layer_args& a, int flat, ClusterSelectSmem& sm,
                                                int rank, int ranks, int row0, int rows,
                                                int token_begin, int token_end, int guess_bin) {
@@ -980,17 +980,12 @@ __device__ __forceinline__ void select_cluster(const ckv_layer_args& a, int flat
   cluster_sync_all();  // every slice's first-pass histogram is complete
   phase_stamp(a, flat, rank, 2);
 
-  // Sum a pair of 256-bin histograms over the cluster.  Each thread owns
-  // 256 / kThreads bins and keeps every slice's values in registers: once the
-  // threshold bin is known they also give the totals above it, for all slices and
-  // for the slices before this one, without another exchange.
   constexpr int kBins = 256 / kThreads;
   static_assert(kBins * kThreads == 256, "thread count must divide 256");
   // Sum a pair of 256-bin histograms over the cluster.  Each thread owns 256 / kThreads
   // bins and reads every slice's values (all loads in flight together); it writes the sum
   // over all slices and the sum over the slices in front of this one.
-  auto gather_from = [&](auto max_ranks, const int* mass, const int* count) {
-    constexpr int kMaxRanks = decltype(max_ranks)::value;
+  auto gather = [&](const int* mass, const int* count) {
     int part_mass[kBins][kMaxRanks];
     int part_count[kBins][kMaxRanks];
 #pragma unroll
@@ -1020,13 +1015,6 @@ __device__ __forceinline__ void select_cluster(const ckv_layer_args& a, int flat
       sm.before_count[tid + k * kThreads] = before_count;
     }
     __syncthreads();
-  };
-  auto gather = [&](const int* mass, const int* count) {
-    if (ranks <= 8) {
-      gather_from(std::integral_constant<int, 8>{}, mass, count);
-    } else {
-      gather_from(std::integral_constant<int, kMaxCluster>{}, mass, count);
-    }
   };
   // Warp 0: the threshold bin of the summed histogram, the totals above it, and the totals
   // above it of the slices in front of this one.
