@@ -119,7 +119,7 @@ class PrefillCSR:
             raise ValueError("community count exceeds offset capacity")
         # compared where the offsets are: on the host a comparison of this size is shared out over
         # every core, and waking those costs milliseconds
-        counts = self.community_counts.unsqueeze(1)
+        counts = self.community_counts.to(offsets.device).unsqueeze(1)
         outside = (counts < 0) | (counts > width)
         falls = (offsets[:, 1:] < offsets[:, :-1]) & (torch.arange(width, device=offsets.device) < counts)
         beyond = offsets.gather(1, counts.clamp(0, width).long()) > self.member_positions.shape[1]

@@ -204,6 +204,22 @@ def test_adjacency_at_the_edges_of_tiles_and_keys(graphs, rows, length, kappa, l
     _adjacency_equal(got, want, f"{graphs}x{rows}x{kappa}")
 
 
+@pytest.mark.parametrize("host", ["member_offsets", "member_positions", "community_counts"])
+def test_member_lists_on_the_host_and_the_device(host):
+    """``PrefillCSR.validate`` takes tensors that are not all on one device."""
+
+    from community_kv_b200.state import PrefillCSR
+
+    tensors = {"member_offsets": torch.tensor([[0, 2, 3], [0, 1, 9]], dtype=torch.int32),
+               "member_positions": torch.zeros((2, 4), dtype=torch.int32),
+               "community_counts": torch.tensor([2, 1], dtype=torch.int32)}
+    placed = {name: tensor if name == host else tensor.cuda() for name, tensor in tensors.items()}
+    PrefillCSR(**placed).validate()
+    placed["community_counts"] = placed["community_counts"] + 1
+    with pytest.raises(ValueError, match="count exceeds"):
+        PrefillCSR(**placed).validate()
+
+
 @pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
 @pytest.mark.parametrize("edges", [1, 15, 16, 4097, 9001])
 def test_modularity_of_sorted_edges(edges, dtype):
