@@ -253,11 +253,15 @@ __global__ void __launch_bounds__(256) modularity_kernel(const int32_t* labels, 
     for (int i = 0; i < kAhead; ++i) {
       const bool inside = source[i] >= 0 && source[i] < vertices;
       from[i] = inside ? __ldg(labels + source[i]) : -1;
-      // the destination counts for the source's graph, whichever graph its own number says
-      Index there = destination[i];
+      // the destination counts for the source's graph, whichever graph its own number says (a negative
+      // one counts from that graph's end); 64 bits: a graph of int32 vertices may end beyond 2^31
+      int64_t there = destination[i];
       if (inside) {
         const Index begin = source[i] - source[i] % length;
-        if (there < begin || there - begin >= length) there = begin + there % length;
+        if (destination[i] < begin || destination[i] - begin >= length) {
+          const Index at = destination[i] % length;
+          there = static_cast<int64_t>(begin) + (at < 0 ? at + length : at);
+        }
       }
       to[i] = inside ? __ldg(labels + there) : -1;
     }

@@ -221,6 +221,21 @@ def test_member_lists_on_the_host_and_the_device(host):
 
 
 @pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
+def test_modularity_counts_destinations_in_the_sources_graph(dtype):
+    """Destinations numbered in another graph, and negative ones: position modulo the length, as on the host."""
+
+    graphs, length, communities = 3, 50, 7
+    labels = _labels(graphs, length, communities, seed=12)
+    source = torch.tensor([60, 61, 110, 120, 149, 99, 55])
+    destination = torch.tensor([3, 149, -1, -50, -51, -99, 60])
+    weight = torch.tensor([1.0, 2.0, 4.0, 8.0, 16.0, 32.0, 64.0])
+    want = init_modularity_state(labels, source, destination, weight, community_capacity=8)
+    got = init_modularity_state(labels.cuda(), source.to(dtype).cuda(), destination.to(dtype).cuda(), weight.cuda(),
+                                community_capacity=8)
+    assert torch.equal(got[0].cpu(), want[0]) and torch.equal(got[1].cpu(), want[1])
+
+
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
 @pytest.mark.parametrize("edges", [1, 15, 16, 4097, 9001])
 def test_modularity_of_sorted_edges(edges, dtype):
     """Runs of one source, a graph's end inside a thread's run, a ragged tail, unaligned edge arrays."""
