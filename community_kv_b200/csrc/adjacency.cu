@@ -162,8 +162,9 @@ __global__ void __launch_bounds__(kSortThreads) digit_bases_kernel(uint32_t* tot
 // ---- decoupled look-back ----
 // A tile publishes its count with kPartial, later the sum over all tiles up to it with kComplete;
 // flag and value are one 64-bit word.  Tiles take their numbers from a counter when they start, so
-// every predecessor is already running and a wait ends; the waits are bounded all the same, and one
-// that runs out is reported and yields a wrong sum (the stores that use it check their bounds).
+// every predecessor is already running and a wait ends; the waits are bounded all the same (`polls`
+// looks without progress), and one that runs out is reported and yields a wrong sum (the stores that
+// use it check their bounds).
 constexpr uint64_t kPartial = 1ull << 62;
 constexpr uint64_t kComplete = 2ull << 62;
 constexpr uint64_t kValueMask = (1ull << 62) - 1;
@@ -183,9 +184,10 @@ __device__ __forceinline__ void publish(uint64_t* word, uint64_t value) {
 // kLookWords of them at a time.
 constexpr int kLookWords = 8;
 
-__device__ __forceinline__ uint32_t look_back(const uint64_t* words, uint32_t tile, uint32_t stride, uint32_t* fault) {
+__device__ __forceinline__ uint32_t look_back(const uint64_t* words, uint32_t tile, uint32_t stride, uint32_t polls,
+                                              uint32_t* fault) {
   uint64_t sum = 0;
-  uint32_t polls = 0;
+  uint32_t polled = 0;
   int64_t t = static_cast<int64_t>(tile) - 1;
   bool done = t < 0;
   while (!done) {
@@ -201,7 +203,7 @@ __device__ __forceinline__ uint32_t look_back(const uint64_t* words, uint32_t ti
         --t;
       }
     }
-    if (!done && t == from && ++polls > kLookPolls) {
+    if (!done && t == from && ++polled > polls) {
       atomicOr(fault, 1u);
       done = true;
     }
@@ -230,7 +232,7 @@ template <typename Key, int kKappa, bool kFirst>
 __global__ void __launch_bounds__(kSortThreads, 3)
     radix_pass_kernel(const EdgeRows e, const Key* keys, const float* weights, Key* keys_out, float* weights_out,
                       const uint32_t* digit_base, const uint32_t* valid, int pass, uint64_t* words, uint32_t* ticket,
-                      uint32_t* fault) {
+                      uint32_t polls, uint32_t* fault) {
   constexpr int kItems = Sort<Key>::kItems;
   constexpr int kTile = Sort<Key>::kTile;
   // counts per warp and digit, and the lane masks; the items in digit order reuse the masks' room
@@ -378,7 +380,7 @@ __global__ void __launch_bounds__(kSortThreads, 3)
         warp_count[w][d] = running;
         running += c;
       }
-      const uint32_t ahead = look_back(words + d, tile, kDigits, fault);
+      const uint32_t ahead = look_back(words + d, tile, kDigits, polls, fault);
       if (tile > 0) {
         publish(words + static_cast<uint64_t>(tile) * kDigits + d, kComplete | (static_cast<uint64_t>(ahead) + count));
       }
@@ -423,8 +425,9 @@ __global__ void __launch_bounds__(kSortThreads, 3)
 template <typename Key>
 __global__ void __launch_bounds__(kSortThreads)
     run_edges_kernel(const Key* keys, const float* weights, const uint32_t* valid, int position_bits, int seq_len,
-                     int64_t capacity, uint64_t* words, uint32_t* ticket, uint32_t* fault, int32_t* edge_src,
-                     int32_t* edge_dst, float* edge_weight, int64_t* edge_count) {
+                     int64_t capacity, uint64_t* words, uint32_t* ticket, uint32_t polls, uint32_t* fault,
+                     uint32_t* finished, int32_t* edge_src, int32_t* edge_dst, float* edge_weight,
+                     int64_t* edge_count) {
   constexpr int kItems = Runs<Key>::kItems;
   constexpr int kTile = Runs<Key>::kTile;
   __shared__ alignas(16) Key key_in[kTile];
@@ -475,7 +478,7 @@ __global__ void __launch_bounds__(kSortThreads)
     // a warp looks back together: lane l at the l-th tile in front
     if (lane == 0) publish(words + tile, (tile == 0 ? kComplete : kPartial) | total);
     uint64_t sum = 0;
-    uint32_t polls = 0;
+    uint32_t polled = 0;
     int64_t t = static_cast<int64_t>(tile) - 1;
     while (t >= 0) {
       const uint64_t word = t - lane >= 0 ? look(words + (t - lane)) : kComplete;
@@ -484,7 +487,7 @@ __global__ void __launch_bounds__(kSortThreads)
       const int reach = done ? __ffs(done) : 32;  // lanes 0 .. reach - 1 are wanted
       const unsigned wanted = reach == 32 ? 0xffffffffu : (1u << reach) - 1u;
       if ((ready & wanted) != wanted) {
-        if (++polls > kLookPolls) {
+        if (++polled > polls) {
           if (lane == 0) atomicOr(fault, 1u);
           break;
         }
@@ -500,8 +503,13 @@ __global__ void __launch_bounds__(kSortThreads)
     if (lane == 0) {
       ahead_s = static_cast<uint32_t>(sum);
       if (tile > 0) publish(words + tile, kComplete | (sum + total));
-      if (base + kTile >= n) {
-        *edge_count = *fault != 0u ? -1 : static_cast<int64_t>(sum + total);
+      if (base + kTile >= n) *edge_count = static_cast<int64_t>(sum + total);
+      // Any tile may be the one whose wait ran out, also after the last tile has its sum: the tile
+      // that comes through last has every other's word on it behind the fences, and passes it on.
+      __threadfence();
+      if (atomicAdd(finished, 1u) == (n - 1u) / kTile) {
+        __threadfence();
+        if (atomicOr(fault, 0u) != 0u) *edge_count = -1;
       }
     }
   }
@@ -573,11 +581,11 @@ int64_t align256(int64_t bytes) { return (bytes + 255) / 256 * 256; }
 struct Scratch {
   void* keys[2];
   float* weights[2];
-  uint32_t* control;  // cleared: digit totals [kMaxPasses][256], valid, fault, a ticket per kernel
+  uint32_t* control;  // cleared: digit totals [kMaxPasses][256], valid, fault, finished, a ticket per kernel
   uint64_t* words;    // cleared: look-back words, [pass][tile][256], then [tile] of the runs
   int64_t bytes;
 };
-constexpr int64_t kControlWords = kMaxPasses * kDigits + 2 + kMaxPasses + 1;
+constexpr int64_t kControlWords = kMaxPasses * kDigits + 3 + kMaxPasses + 1;
 
 template <typename Key>
 int64_t look_words(int64_t raw, int passes) {
@@ -607,15 +615,17 @@ Scratch carve(void* base, int64_t raw) {
 }
 
 template <typename Key, int kKappa>
-cudaError_t sort_and_merge(const EdgeRows& e, const Scratch& s, int bits, int64_t capacity, int32_t* edge_src,
-                           int32_t* edge_dst, float* edge_weight, int64_t* edge_count, cudaStream_t stream) {
+cudaError_t sort_and_merge(const EdgeRows& e, const Scratch& s, int bits, uint32_t polls, int64_t capacity,
+                           int32_t* edge_src, int32_t* edge_dst, float* edge_weight, int64_t* edge_count,
+                           cudaStream_t stream) {
   const int passes = bits > 8 ? (bits + 7) / 8 : 1;
   const unsigned tiles = static_cast<unsigned>((static_cast<int64_t>(e.raw) + Sort<Key>::kTile - 1) / Sort<Key>::kTile);
   const unsigned run_tiles = static_cast<unsigned>((static_cast<int64_t>(e.raw) + Runs<Key>::kTile - 1) / Runs<Key>::kTile);
   uint32_t* totals = s.control;
   uint32_t* valid = totals + kMaxPasses * kDigits;
   uint32_t* fault = valid + 1;
-  uint32_t* tickets = fault + 1;
+  uint32_t* finished = fault + 1;
+  uint32_t* tickets = finished + 1;
   cudaError_t err = cudaMemsetAsync(
       s.control, 0, align256(kControlWords * 4) + static_cast<size_t>(look_words<Key>(e.raw, passes)) * 8, stream);
   if (err != cudaSuccess) return err;
@@ -628,18 +638,18 @@ cudaError_t sort_and_merge(const EdgeRows& e, const Scratch& s, int bits, int64_
     uint64_t* words = s.words + static_cast<int64_t>(p) * tiles * kDigits;
     if (p == 0) {
       radix_pass_kernel<Key, kKappa, true><<<tiles, kSortThreads, 0, stream>>>(
-          e, in, s.weights[1], out, s.weights[0], totals, valid, 0, words, tickets, fault);
+          e, in, s.weights[1], out, s.weights[0], totals, valid, 0, words, tickets, polls, fault);
     } else {
       radix_pass_kernel<Key, 0, false><<<tiles, kSortThreads, 0, stream>>>(
           e, in, s.weights[1 - (p & 1)], out, s.weights[p & 1], totals + p * kDigits, valid, p, words, tickets + p,
-          fault);
+          polls, fault);
     }
   }
   const int last = (passes - 1) & 1;
   run_edges_kernel<Key><<<run_tiles, kSortThreads, 0, stream>>>(
       static_cast<const Key*>(s.keys[last]), s.weights[last], valid, e.position_bits, e.seq_len, capacity,
-      s.words + static_cast<int64_t>(passes) * tiles * kDigits, tickets + kMaxPasses, fault, edge_src, edge_dst,
-      edge_weight, edge_count);
+      s.words + static_cast<int64_t>(passes) * tiles * kDigits, tickets + kMaxPasses, polls, fault, finished, edge_src,
+      edge_dst, edge_weight, edge_count);
   return cudaGetLastError();
 }
 
@@ -665,10 +675,11 @@ int64_t ckv_adjacency_scratch_bytes(int64_t graphs, int64_t rows, int32_t kappa,
   return raw > 0 ? ckv::carve(nullptr, raw).bytes : 0;
 }
 
-int ckv_build_adjacency(const int32_t* topk_indices, const float* topk_scores, const int64_t* query_positions,
-                        int32_t graphs, int64_t rows, int32_t kappa, int32_t seq_len, double lam,
-                        int32_t* edge_src, int32_t* edge_dst, float* edge_weight, int64_t edge_capacity,
-                        int64_t* edge_count, void* scratch, int64_t scratch_bytes, void* cuda_stream) {
+int ckv_build_adjacency_polls(const int32_t* topk_indices, const float* topk_scores, const int64_t* query_positions,
+                              int32_t graphs, int64_t rows, int32_t kappa, int32_t seq_len, double lam,
+                              int32_t* edge_src, int32_t* edge_dst, float* edge_weight, int64_t edge_capacity,
+                              int64_t* edge_count, void* scratch, int64_t scratch_bytes, uint32_t look_polls,
+                              void* cuda_stream) {
   if (!topk_indices || !topk_scores || !query_positions || !edge_src || !edge_dst || !edge_weight ||
       !edge_count || !scratch) {
     return CKV_ERR_NULL;
@@ -700,7 +711,8 @@ int ckv_build_adjacency(const int32_t* topk_indices, const float* topk_scores, c
   e.co_scale = static_cast<float>(1.0 - lam);
   const int bits = ckv::bits_for(graphs) + 2 * e.position_bits;  // at most 62: the vertex count is below 2^31
   auto run = [&](auto sorter) {
-    return sorter(e, s, bits, edge_capacity, edge_src, edge_dst, edge_weight, edge_count, stream) == cudaSuccess
+    return sorter(e, s, bits, look_polls, edge_capacity, edge_src, edge_dst, edge_weight, edge_count, stream) ==
+                   cudaSuccess
                ? CKV_OK
                : CKV_ERR_LAUNCH;
   };
@@ -708,6 +720,15 @@ int ckv_build_adjacency(const int32_t* topk_indices, const float* topk_scores, c
     return kappa == 8 ? run(ckv::sort_and_merge<uint32_t, 8>) : run(ckv::sort_and_merge<uint32_t, 0>);
   }
   return kappa == 8 ? run(ckv::sort_and_merge<uint64_t, 8>) : run(ckv::sort_and_merge<uint64_t, 0>);
+}
+
+int ckv_build_adjacency(const int32_t* topk_indices, const float* topk_scores, const int64_t* query_positions,
+                        int32_t graphs, int64_t rows, int32_t kappa, int32_t seq_len, double lam,
+                        int32_t* edge_src, int32_t* edge_dst, float* edge_weight, int64_t edge_capacity,
+                        int64_t* edge_count, void* scratch, int64_t scratch_bytes, void* cuda_stream) {
+  return ckv_build_adjacency_polls(topk_indices, topk_scores, query_positions, graphs, rows, kappa, seq_len, lam,
+                                   edge_src, edge_dst, edge_weight, edge_capacity, edge_count, scratch,
+                                   scratch_bytes, ckv::kLookPolls, cuda_stream);
 }
 
 }  // extern "C"

@@ -196,6 +196,7 @@ ENTRY_POINTS = (
     "ckv_adjacency_raw_edges",
     "ckv_adjacency_scratch_bytes",
     "ckv_build_adjacency",
+    "ckv_build_adjacency_polls",
 )
 
 
@@ -245,6 +246,9 @@ def library() -> ctypes.CDLL:
         getattr(lib, name).argtypes = [_l, _l, _i, ctypes.c_double]
     lib.ckv_build_adjacency.restype = ctypes.c_int
     lib.ckv_build_adjacency.argtypes = [_p, _p, _p, _i, _l, _i, _i, ctypes.c_double, _p, _p, _p, _l, _p, _p, _l, _p]
+    lib.ckv_build_adjacency_polls.restype = ctypes.c_int
+    lib.ckv_build_adjacency_polls.argtypes = [
+        _p, _p, _p, _i, _l, _i, _i, ctypes.c_double, _p, _p, _p, _l, _p, _p, _l, ctypes.c_uint32, _p]
     lib.ckv_nearest_centroid.restype = ctypes.c_int
     lib.ckv_nearest_centroid.argtypes = [ctypes.POINTER(LayerArgs), ctypes.c_void_p, ctypes.c_void_p]
     lib.ckv_wait_peers.restype = ctypes.c_int

@@ -387,6 +387,13 @@ int ckv_build_adjacency(const int32_t* topk_indices, const float* topk_scores, c
                         int32_t graphs, int64_t rows, int32_t kappa, int32_t seq_len, double lam,
                         int32_t* edge_src, int32_t* edge_dst, float* edge_weight, int64_t edge_capacity,
                         int64_t* edge_count, void* scratch, int64_t scratch_bytes, void* cuda_stream);
+/* The same with a bound of the caller's on the waits inside the sort: a wait gives up after look_polls
+ * looks without progress (ckv_build_adjacency: 2^22).  For testing how a wait that ran out is reported. */
+int ckv_build_adjacency_polls(const int32_t* topk_indices, const float* topk_scores, const int64_t* query_positions,
+                              int32_t graphs, int64_t rows, int32_t kappa, int32_t seq_len, double lam,
+                              int32_t* edge_src, int32_t* edge_dst, float* edge_weight, int64_t edge_capacity,
+                              int64_t* edge_count, void* scratch, int64_t scratch_bytes, uint32_t look_polls,
+                              void* cuda_stream);
 
 /* P1.  Causal attention (output + lse) that also emits each row's strongest
  * Q.K neighbours: the reference's top-8 rule (mode 1) or exact top-m per KV head

@@ -204,6 +204,40 @@ def test_adjacency_at_the_edges_of_tiles_and_keys(graphs, rows, length, kappa, l
     _adjacency_equal(got, want, f"{graphs}x{rows}x{kappa}")
 
 
+def test_adjacency_reports_a_wait_that_ran_out():
+    """Waits inside the sort that give up at their first look: the count says so, or the edges are right.
+    More tiles than run at a time, so that some tile does find its predecessors unfinished."""
+
+    from community_kv_b200 import native
+    from community_kv_b200.assembly import build_adjacency
+
+    graphs, rows, kappa, length, lam = 4, 12000, 8, 8192, 0.5
+    generator = torch.Generator().manual_seed(5)
+    indices = torch.randint(0, length, (graphs, rows, kappa), generator=generator, dtype=torch.int32).cuda()
+    scores = torch.rand((graphs, rows, kappa), generator=generator).cuda()
+    positions = torch.randint(0, length, (graphs, rows), generator=generator).cuda()
+    want = build_adjacency(indices, scores, positions, seq_len=length, lam=lam)
+    lib = native.library()
+    raw = lib.ckv_adjacency_raw_edges(graphs, rows, kappa, lam)
+    reported = 0
+    for _ in range(20):
+        scratch = torch.zeros((lib.ckv_adjacency_scratch_bytes(graphs, rows, kappa, lam),), dtype=torch.uint8,
+                              device="cuda")
+        source, destination = (torch.empty((raw,), dtype=torch.int32, device="cuda") for _ in range(2))
+        weight = torch.empty((raw,), device="cuda")
+        count = torch.empty((1,), dtype=torch.int64, device="cuda")
+        assert lib.ckv_build_adjacency_polls(
+            indices.data_ptr(), scores.data_ptr(), positions.data_ptr(), graphs, rows, kappa, length, lam,
+            source.data_ptr(), destination.data_ptr(), weight.data_ptr(), raw, count.data_ptr(),
+            scratch.data_ptr(), scratch.numel(), 0, native.current_stream(indices.device)) == 0
+        edges = int(count)
+        reported += edges == -1
+        if edges != -1:
+            for got, expected in zip((source, destination, weight), want):
+                assert torch.equal(got[:edges], expected)
+    assert reported > 0
+
+
 @pytest.mark.parametrize("host", ["member_offsets", "member_positions", "community_counts"])
 def test_member_lists_on_the_host_and_the_device(host):
     """``PrefillCSR.validate`` takes tensors that are not all on one device."""
