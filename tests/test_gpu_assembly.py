@@ -204,6 +204,33 @@ def test_adjacency_at_the_edges_of_tiles_and_keys(graphs, rows, length, kappa, l
     _adjacency_equal(got, want, f"{graphs}x{rows}x{kappa}")
 
 
+def test_adjacency_leaves_out_direct_edges_of_rows_outside_the_graph():
+    """A row's own position beyond its graph, or negative: no direct edge; its neighbours' edges stay."""
+
+    from community_kv_b200.assembly import build_adjacency
+    from oracle.adjacency_oracle import build_adjacency as oracle_adjacency
+
+    length, kappa = 100, 8
+    rng = np.random.default_rng(3)
+    indices = rng.integers(0, length, size=(2, 40, kappa)).astype(np.int32)
+    scores = rng.uniform(0.01, 1, size=indices.shape).astype(np.float32)
+    positions = rng.integers(0, length, size=(2, 40)).astype(np.int64)
+    outside = rng.uniform(size=positions.shape) < 0.3
+    moved = np.where(outside, rng.choice([-1, -length, length, length + 7, 2**40], size=positions.shape), positions)
+    device = torch.device("cuda", 0)
+
+    def run(lam):
+        return build_adjacency(*(torch.from_numpy(a).to(device) for a in (indices, scores, moved)), seq_len=length, lam=lam)
+
+    # direct edges alone: as if those rows had no neighbours
+    want = oracle_adjacency(np.where(outside[..., None], -1, indices), scores, positions, seq_len=length, lam=1.0)
+    _adjacency_equal(run(1.0), want, "direct")
+    # lam = 0: direct edges weigh nothing, and every other edge is there
+    got = [t.cpu().numpy() for t in run(0.0)]
+    want = oracle_adjacency(indices, scores, positions, seq_len=length, lam=0.0)
+    _adjacency_equal([torch.from_numpy(a[got[2] > 0]) for a in got], [a[want[2] > 0] for a in want], "co-attention")
+
+
 def test_adjacency_reports_a_wait_that_ran_out():
     """Waits inside the sort that give up at their first look: the count says so, or the edges are right.
     More tiles than run at a time, so that some tile does find its predecessors unfinished."""
@@ -280,12 +307,11 @@ def test_modularity_of_sorted_edges(edges, dtype):
     generator = torch.Generator().manual_seed(edges)
     source = torch.randint(0, graphs * length, (edges + 1,), generator=generator).sort().values
     destination = source // length * length + torch.randint(0, length, (edges + 1,), generator=generator)
-    weight = torch.rand((edges + 1,), generator=generator)
+    # sixteenths: every sum below 2^20 is exact in fp32, in any order
+    weight = torch.randint(1, 17, (edges + 1,), generator=generator) / 16
     for begin in (0, 1):
         part = [t[begin : begin + edges] for t in (source, destination, weight)]
         want_weight, want_total = init_modularity_state(labels, *part, community_capacity=24)
         moved = [t.to(device)[begin : begin + edges] for t in (source.to(dtype), destination.to(dtype), weight)]
         got_weight, got_total = init_modularity_state(labels.to(device), *moved, community_capacity=24)
-        # positive terms in another order: n * 2^-24 relative with n below 1000 per community, 6000 per graph
-        torch.testing.assert_close(got_weight.cpu(), want_weight, rtol=6e-5, atol=1e-6)
-        torch.testing.assert_close(got_total.cpu(), want_total, rtol=4e-4, atol=1e-6)
+        assert torch.equal(got_weight.cpu(), want_weight) and torch.equal(got_total.cpu(), want_total)

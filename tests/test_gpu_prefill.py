@@ -289,6 +289,33 @@ def test_reference_topk_rule_with_ties(length, heads, kv_heads, sinks):
         assert np.array_equal(idx[0, head].cpu().numpy(), want_idx), head
 
 
+@pytest.mark.parametrize("kind", ["nan", "inf"])
+@pytest.mark.parametrize("heads,kv_heads", [(4, 1), (2, 2)])
+def test_reference_topk_rule_with_odd_scores(kind, heads, kv_heads):
+    """Whole-number scores with a few keys that make a row's scores infinite or not a number: a NaN or
+    -inf is never a neighbour (every row has eight others), a +inf is one and saturates the candidate key."""
+
+    length, sinks = 333, 10
+    generator = torch.Generator().manual_seed(length)
+    q = torch.randint(0, 2, (1, length, heads, 128), generator=generator).mul(2).sub(1).to(torch.bfloat16)
+    k = torch.randint(-1, 2, (1, length, kv_heads, 128), generator=generator).to(torch.bfloat16)
+    v = torch.randn((1, length, kv_heads, 128), generator=generator).to(torch.bfloat16)
+    if kind == "nan":
+        k[0, 45] = float("nan")
+        k[0, 200, :, 3] = float("nan")
+    else:
+        k[0, 77, :, 0] = float("inf")
+        k[0, 130, :, 0] = float("inf")
+        k[0, 300, :, 5] = float("-inf")
+    *_, idx = prefill_attention_topk(q.cuda(), k.cuda(), v.cuda(), softmax_scale=SCALE, num_sink=sinks)
+    group = heads // kv_heads
+    for head in range(heads):
+        raw = q[0, :, head].double().numpy() @ k[0, :, head // group].double().numpy().T
+        raw = np.where(np.isnan(raw), -1000.0, raw).astype(np.float32)  # quantises to the least key, as -inf does
+        want_idx = oracle.reference_topk(raw, np.zeros(length, np.float32), SCALE, sinks)[1]
+        assert np.array_equal(idx[0, head].cpu().numpy(), want_idx), head
+
+
 @pytest.mark.parametrize("room,shift", [(0, 0), (24, 0), (24, 4)])
 def test_plugin_prefill_reads_the_cache_where_it_lies(room, shift):
     """``[B, H, S, D]`` tensors with unused rows, and off the 16-byte boundary that the tile copies need."""
