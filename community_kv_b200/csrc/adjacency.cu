@@ -15,15 +15,23 @@
 // enumeration order, so each weight is the same sequence of fp32 additions a sequential
 // scatter-add performs: the result is bit-exact and independent of scheduling.
 //
-// What bounds it is the traffic of the sort, so it carries as few bytes as often as it can:
+// The sort is a one-sweep radix sort (Adinets and Merrill, "Onesweep", 2022: digit totals of all
+// passes up front, one kernel per pass with the decoupled look-back of Merrill and Garland, 2016)
+// and carries as few bytes as often as it can:
 //   * both ends of an edge lie in one graph, so the key is (graph, min, max) with the
 //     positions inside the graph: 31 bits and four passes for 32 graphs of 8192 positions
 //     instead of 36 bits and five, and a 4-byte key wherever it fits (else 8 bytes);
 //   * the raw edges are never written in enumeration order: the first pass makes them from
-//     the rows (16 bytes of neighbours and scores per 44 edges of 8 bytes);
+//     the rows (64 bytes of neighbours and scores per 44 edges of 8 bytes);
 //   * a pass is one kernel: every tile publishes its digit counts and sums its
-//     predecessors' (decoupled look-back), and items leave in digit order through shared
-//     memory, so that a tile writes runs of consecutive items.
+//     predecessors', and items leave in digit order through shared memory, so that a
+//     tile writes runs of consecutive items.
+// What bounds a pass now is not the traffic (16 bytes an item, 28 us of 11.5 M items at the copy
+// rate; DRAM is busy 15-20 %) but the latency of its chain - shared-memory atomics of the ranking,
+// look-back, staging - with 24 warps per SM: long_scoreboard and short_scoreboard lead the stalls.
+// Eighty registers for three blocks per SM are too few for sixteen 4-byte items: the pass spills
+// 324 bytes of stores and 392 of loads per thread (the first pass 108-168 and 108-112), which stay
+// in L1.
 // 32 graphs of 8192 positions, 11.5 M raw edges: 0.61 ms (105-115 us a pass, 85 us the runs);
 // five passes over enumerated 12-byte items with separate count and scan kernels took 1.1 ms.
 
@@ -214,11 +222,10 @@ __device__ __forceinline__ uint32_t look_back(const uint64_t* words, uint32_t ti
 // ---- one stable radix pass: digit = byte `pass` of the key ----
 // Item order inside a tile: warp w holds items [32 kItems w, 32 kItems (w + 1)), round i of the
 // warp 32 consecutive ones.  An item's rank among the tile's items of its digit is the count of
-// the warps before it, the rounds before it and the lanes before it.  The pass is bound by its
-// instructions once the traffic is down to 16 bytes per item, so the lanes of a warp that share a
-// digit find one another by OR-ing their lane bits into a word of shared memory (about 15
-// instructions whatever the digit's width; eight ballots take 40), and a full tile runs without
-// bounds checks.
+// the warps before it, the rounds before it and the lanes before it.  The lanes of a warp that
+// share a digit find one another by OR-ing their lane bits into a word of shared memory (a match
+// by atomics: about 15 instructions whatever the digit's width; eight ballots take 40), and a
+// full tile runs without bounds checks.
 template <typename Key>
 __device__ __forceinline__ uint32_t digit_of(Key key, int pass) {
   if constexpr (sizeof(Key) == 4) {

@@ -139,7 +139,8 @@ __device__ __forceinline__ float centroid_mean(float old_value, int old_size, fl
   return __fdiv_rn(numerator, denominator);
 }
 
-// Optional phase timestamps of the single-launch decode path (see ckv_layer_args).
+// Optional phase timestamps of the single-launch decode path (see ckv_layer_args): the array has
+// room for eight CTAs of a unit.
 __device__ __forceinline__ void phase_stamp(const ckv_layer_args& a, int flat, int rank, int slot) {
   if (a.phase_times != nullptr && threadIdx.x == 0 && rank < 8) {
     unsigned long long now;

@@ -637,8 +637,9 @@ __global__ void __launch_bounds__(kPfThreads, 1)
 
 // ---- exact top-m from the candidate lists (mode 2, second kernel) ----
 // One warp per (batch, KV head, position).  The 16 candidate keys of each of its lists (two
-// from edge_candidates_kernel, one per head of the group otherwise) are re-scored as max over the group of scale * (q . k) in the fixed fp32 order
-// and ranked by (score descending, key index ascending).  A row is flagged when
+// from edge_candidates_kernel, one per head of the group otherwise) are re-scored as max over
+// the group of scale * (q . k) in the fixed fp32 order and ranked by (score descending, key
+// index ascending).  A row is flagged when
 // a key that was turned away could still belong to the top-m: the best
 // approximate score among the dropped keys is within `slack` of the exact m-th.
 __global__ void __launch_bounds__(128) exact_edges_kernel(const ckv_prefill_args a, int group, int lists) {

@@ -195,8 +195,9 @@ typedef struct ckv_layer_args {
                                   peer_wait_expected, so that the launch completes only when the
                                   gathered tensor is complete: no separate wait is needed */
   uint64_t* phase_times;       /* optional diagnostic [batch*R, 8, 16]: nanosecond timestamps
-                                  (%globaltimer) that thread 0 of every CTA of the single-launch
-                                  path writes at its phase boundaries: 0 start, 1 scored,
+                                  (%globaltimer) that thread 0 of CTAs 0..7 of a unit's cluster
+                                  (with more CTAs the others write none) writes at the phase
+                                  boundaries of the single-launch path: 0 start, 1 scored,
                                   2..4 after the selection's three cluster exchanges, 5 descriptors
                                   known, 6 cache rows resolved, 7 attended, 8 partials of the whole
                                   cluster visible (rank 0), 9 merged and updated (rank 0) */
@@ -371,7 +372,8 @@ int ckv_assemble_modularity32(const int32_t* labels, int32_t graphs, int32_t len
 
 /* Edge list -> coalesced adjacency: what the host partitioner consumes.  topk_indices int32 and
  * topk_scores fp32 are [graphs, rows, kappa] (neighbour position per row, -1 or >= seq_len:
- * none), query_positions int64 [graphs, rows] the position a row belongs to.  A row contributes
+ * none), query_positions int64 [graphs, rows] the position a row belongs to (outside [0, seq_len):
+ * the row has no direct edges, those between its neighbours stay).  A row contributes
  * kappa direct edges (weight score * lam / 2) and, for lam < 1, kappa (kappa + 1) / 2
  * co-attention edges between its neighbours (weight score_a * score_b * (1 - lam)); edges are
  * stored as (min, max) over vertices graph * seq_len + position, duplicates merged by adding
