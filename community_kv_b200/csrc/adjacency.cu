@@ -432,9 +432,8 @@ __global__ void __launch_bounds__(kSortThreads, 3)
 template <typename Key>
 __global__ void __launch_bounds__(kSortThreads)
     run_edges_kernel(const Key* keys, const float* weights, const uint32_t* valid, int position_bits, int seq_len,
-                     int64_t capacity, uint64_t* words, uint32_t* ticket, uint32_t polls, uint32_t* fault,
-                     uint32_t* finished, int32_t* edge_src, int32_t* edge_dst, float* edge_weight,
-                     int64_t* edge_count) {
+                     int64_t capacity, uint64_t* words, uint32_t* ticket, uint32_t polls, const uint32_t* fault,
+                     int32_t* edge_src, int32_t* edge_dst, float* edge_weight, unsigned long long* edge_count) {
   constexpr int kItems = Runs<Key>::kItems;
   constexpr int kTile = Runs<Key>::kTile;
   __shared__ alignas(16) Key key_in[kTile];
@@ -495,7 +494,7 @@ __global__ void __launch_bounds__(kSortThreads)
       const unsigned wanted = reach == 32 ? 0xffffffffu : (1u << reach) - 1u;
       if ((ready & wanted) != wanted) {
         if (++polled > polls) {
-          if (lane == 0) atomicOr(fault, 1u);
+          if (lane == 0) atomicExch(edge_count, ~0ull);
           break;
         }
         continue;
@@ -510,13 +509,15 @@ __global__ void __launch_bounds__(kSortThreads)
     if (lane == 0) {
       ahead_s = static_cast<uint32_t>(sum);
       if (tile > 0) publish(words + tile, kComplete | (sum + total));
-      if (base + kTile >= n) *edge_count = static_cast<int64_t>(sum + total);
-      // Any tile may be the one whose wait ran out, also after the last tile has its sum: the tile
-      // that comes through last has every other's word on it behind the fences, and passes it on.
-      __threadfence();
-      if (atomicAdd(finished, 1u) == (n - 1u) / kTile) {
-        __threadfence();
-        if (atomicOr(fault, 0u) != 0u) *edge_count = -1;
+      // The count starts at 0.  Any tile may be the one whose wait ran out, before or after the last
+      // tile has its sum: that tile's -1 replaces a count, and no count replaces a -1.  The earlier
+      // kernels' waits are reported by the fault word.
+      if (base + kTile >= n) {
+        if (*fault != 0u) {
+          atomicExch(edge_count, ~0ull);
+        } else {
+          atomicCAS(edge_count, 0ull, sum + total);
+        }
       }
     }
   }
@@ -588,11 +589,11 @@ int64_t align256(int64_t bytes) { return (bytes + 255) / 256 * 256; }
 struct Scratch {
   void* keys[2];
   float* weights[2];
-  uint32_t* control;  // cleared: digit totals [kMaxPasses][256], valid, fault, finished, a ticket per kernel
+  uint32_t* control;  // cleared: digit totals [kMaxPasses][256], valid, fault, a ticket per kernel
   uint64_t* words;    // cleared: look-back words, [pass][tile][256], then [tile] of the runs
   int64_t bytes;
 };
-constexpr int64_t kControlWords = kMaxPasses * kDigits + 3 + kMaxPasses + 1;
+constexpr int64_t kControlWords = kMaxPasses * kDigits + 2 + kMaxPasses + 1;
 
 template <typename Key>
 int64_t look_words(int64_t raw, int passes) {
@@ -631,8 +632,7 @@ cudaError_t sort_and_merge(const EdgeRows& e, const Scratch& s, int bits, uint32
   uint32_t* totals = s.control;
   uint32_t* valid = totals + kMaxPasses * kDigits;
   uint32_t* fault = valid + 1;
-  uint32_t* finished = fault + 1;
-  uint32_t* tickets = finished + 1;
+  uint32_t* tickets = fault + 1;
   cudaError_t err = cudaMemsetAsync(
       s.control, 0, align256(kControlWords * 4) + static_cast<size_t>(look_words<Key>(e.raw, passes)) * 8, stream);
   if (err != cudaSuccess) return err;
@@ -655,8 +655,8 @@ cudaError_t sort_and_merge(const EdgeRows& e, const Scratch& s, int bits, uint32
   const int last = (passes - 1) & 1;
   run_edges_kernel<Key><<<run_tiles, kSortThreads, 0, stream>>>(
       static_cast<const Key*>(s.keys[last]), s.weights[last], valid, e.position_bits, e.seq_len, capacity,
-      s.words + static_cast<int64_t>(passes) * tiles * kDigits, tickets + kMaxPasses, polls, fault, finished, edge_src,
-      edge_dst, edge_weight, edge_count);
+      s.words + static_cast<int64_t>(passes) * tiles * kDigits, tickets + kMaxPasses, polls, fault, edge_src, edge_dst,
+      edge_weight, reinterpret_cast<unsigned long long*>(edge_count));
   return cudaGetLastError();
 }
 

@@ -480,7 +480,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         }
         if (block > 0) {
           // P.V of the last block is done: this block's S was committed after it.  Rare, so
-          // rolled and in narrow steps: 32 columns at a time spilled registers of the loop.
+          // rolled and in narrow steps, which take few registers beside the row of scores.
 #pragma unroll 1
           for (int part = 0; part < 8; ++part) {
             uint32_t o[16];
