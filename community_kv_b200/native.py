@@ -188,6 +188,7 @@ ENTRY_POINTS = (
     "ckv_wait_peers",
     "ckv_nearest_centroid",
     "ckv_append_kv",
+    "ckv_append_kv_advance",
     "ckv_merge_partials",
     "ckv_assemble_member_csr",
     "ckv_assemble_centroids",
@@ -233,6 +234,9 @@ def library() -> ctypes.CDLL:
     lib.ckv_append_kv.restype = ctypes.c_int
     lib.ckv_append_kv.argtypes = [ctypes.c_void_p] * 4 + [ctypes.c_int64, ctypes.c_int64, ctypes.c_void_p,
                                   ctypes.c_int64, ctypes.c_int64, ctypes.c_void_p]
+    lib.ckv_append_kv_advance.restype = ctypes.c_int
+    lib.ckv_append_kv_advance.argtypes = [ctypes.c_void_p] * 4 + [ctypes.c_int64, ctypes.c_int64, ctypes.c_void_p,
+                                          ctypes.c_void_p]
     _p, _i, _l = ctypes.c_void_p, ctypes.c_int32, ctypes.c_int64
     lib.ckv_assemble_member_csr.restype = ctypes.c_int
     lib.ckv_assemble_member_csr.argtypes = [_p, _i, _i, _i, _i, _p, _p, _p, _i, _p]

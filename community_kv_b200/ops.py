@@ -662,6 +662,8 @@ def append_kv(
     new_key: torch.Tensor,
     new_value: torch.Tensor,
     row: int | torch.Tensor,
+    *,
+    advance: bool = False,
 ) -> None:
     """``cache[..., row, :] = new[..., :]`` for both caches in one small launch.
 
@@ -669,6 +671,7 @@ def append_kv(
     with the same leading shape; ``row`` is one index for all of them, an int32 tensor
     with one element (a device-side cursor shared by all of them, read by the kernel: no
     host round trip), or an int32 tensor with one index per leading entry (negative: skip).
+    ``advance``: a shared cursor is also incremented, behind the rows and in the same launch.
     """
 
     if key_cache.shape != value_cache.shape or new_key.shape != new_value.shape:
@@ -688,14 +691,24 @@ def append_kv(
             raise ValueError("row must be an int32 device tensor with one entry, or one per cache row to write")
         index = row.contiguous()
         stride = 0 if row.numel() == 1 else 1
+        if advance and row.numel() != 1:
+            raise ValueError("only a cursor shared by all rows can be advanced")
     elif not 0 <= int(row) < key_cache.shape[-2]:
         raise ValueError("row is outside the cache")
+    elif advance:
+        raise ValueError("only a device-side cursor can be advanced")
     keep = (new_key.contiguous(), new_value.contiguous())
-    status = native.library().ckv_append_kv(
-        key_cache.data_ptr(), value_cache.data_ptr(), keep[0].data_ptr(), keep[1].data_ptr(), units,
-        key_cache.shape[-2] * HEAD_DIM, native.pointer(index), stride, 0 if index is not None else int(row),
-        native.current_stream(device),
-    )
+    if advance:
+        status = native.library().ckv_append_kv_advance(
+            key_cache.data_ptr(), value_cache.data_ptr(), keep[0].data_ptr(), keep[1].data_ptr(), units,
+            key_cache.shape[-2] * HEAD_DIM, row.data_ptr(), native.current_stream(device),
+        )
+    else:
+        status = native.library().ckv_append_kv(
+            key_cache.data_ptr(), value_cache.data_ptr(), keep[0].data_ptr(), keep[1].data_ptr(), units,
+            key_cache.shape[-2] * HEAD_DIM, native.pointer(index), stride, 0 if index is not None else int(row),
+            native.current_stream(device),
+        )
     if status:
         raise native.NativeError(native.library().ckv_status_string(status).decode())
 

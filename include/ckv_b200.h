@@ -27,7 +27,7 @@
  *   ckv_prefill_topk         torch.ops.flash_attn_3.fwd(..., exclude_sink_tokens=n)
  *                            community_kv/attention/flash_attention.py:23-51
  *                            (third_party/flash_attention/community-kv.patch)
- *   ckv_append_kv            the cache layer's index_copy_ of the decoded token
+ *   ckv_append_kv, ckv_append_kv_advance   the cache layer's index_copy_ of the decoded token
  *                            community_kv/attention/cache.py:29-36
  *   ckv_assemble_member_csr, ckv_assemble_centroids, ckv_assemble_modularity
  *                            build_member_csr, compute_centroids, init_modularity_state
@@ -296,6 +296,11 @@ int ckv_decode_layer(const ckv_layer_args* args, void* cuda_stream);
 int ckv_append_kv(void* key_cache, void* value_cache, const void* new_key, const void* new_value,
                   int64_t units, int64_t unit_stride, const int32_t* row_index,
                   int64_t row_index_stride, int64_t row, void* cuda_stream);
+
+/* The same with one device-side cursor shared by all units (int32[1], the row to write;
+ * negative: nothing is written), which is incremented behind the rows, in the same launch. */
+int ckv_append_kv_advance(void* key_cache, void* value_cache, const void* new_key, const void* new_value,
+                          int64_t units, int64_t unit_stride, int32_t* cursor, void* cuda_stream);
 
 /* Waits (on the stream, in a one-thread kernel with a bounded number of polls)
  * until *flag >= expected, then subtracts `expected` from it.  `flag` is this GPU's

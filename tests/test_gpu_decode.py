@@ -517,6 +517,29 @@ def test_append_kv_rows():
         ops.append_kv(key, value, new_key, new_value, 40)
 
 
+@pytest.mark.parametrize("units", [1, 4, 5, 33, 70])
+def test_append_kv_moves_the_cursor(units):
+    """One launch writes the rows and moves the cursor on: four warps, a warp per unit, several units per warp."""
+
+    device = torch.device("cuda", 0)
+    torch.manual_seed(units)
+    key = torch.randn((units, 9, 128), device=device).to(torch.bfloat16)
+    value = torch.randn_like(key)
+    want_key, want_value = key.clone(), value.clone()
+    cursor = torch.tensor([5], dtype=torch.int32, device=device)
+    for row in (5, 6, 7):
+        new_key = torch.randn((units, 128), device=device).to(torch.bfloat16)
+        new_value = torch.randn_like(new_key)
+        want_key[:, row], want_value[:, row] = new_key, new_value
+        ops.append_kv(key, value, new_key, new_value, cursor, advance=True)
+    assert int(cursor) == 8
+    assert torch.equal(key, want_key) and torch.equal(value, want_value)
+    with pytest.raises(ValueError):
+        ops.append_kv(key, value, new_key, new_value, 3, advance=True)
+    with pytest.raises(ValueError):
+        ops.append_kv(key[:4], value[:4], new_key[:4], new_value[:4], cursor.repeat(4), advance=True)
+
+
 def test_full_size_batch_one_launch_equals_four_kernels():
     """The batched long-context configuration as far as one layer goes (8 sequences x 8 KV heads at ctx 131072,
     1024-4096 Zipf communities, budget 2048): the single cluster launch and the four
