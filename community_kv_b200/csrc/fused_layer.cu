@@ -22,10 +22,10 @@
 //      graph update; the other CTAs have already left.
 //
 // The result is bit for bit the one of the four stand-alone kernels: the same
-// device functions run in the same order on the same data.  The path needs one
-// graph per retrieval head (a graph shared by several heads is updated by its
-// leader while followers may still be reading it, which only a kernel boundary
-// orders) and per-CTA community slices that fit the selection's shared-memory stash.
+// device functions run in the same order on the same data.  The path needs per-CTA
+// community slices that fit the selection's shared-memory stash.  A graph shared by several
+// retrieval heads is updated by its leader while followers may still be reading it, which only a
+// kernel boundary orders: step 4 then ends with the outputs, and the update is a second launch.
 
 #include <atomic>
 
@@ -245,7 +245,7 @@ int wide_ctas(const ckv_layer_args& a) {
 
 // CTAs per unit of the one launch; 0: the stand-alone kernels run.
 int fused_layer_ctas(const ckv_layer_args& a) {
-  if (a.graphs != a.retrieval_heads || a.splits < 1 || a.splits > 2 * kMaxCluster ||
+  if (a.splits < 1 || a.splits > 2 * kMaxCluster ||
       (a.flags & (CKV_FLAG_ATTENTION_ONLY | CKV_FLAG_UPDATE_ONLY | CKV_FLAG_UNFUSED | CKV_FLAG_FP32_CENTROIDS))) {
     return 0;
   }

@@ -10,64 +10,88 @@
 
 namespace ckv {
 
+// The other heads of a graph shared by several retrieval heads take the leader's assignment over into
+// their own tables.  The CTA that has just updated the graph does it, four heads in flight: what it
+// needs of the decision is still in shared memory, and a launch of its own (2.7 us and the gap in
+// front of it) is saved.  Nothing else of the launch reads those tables.
+__device__ __forceinline__ void sync_followers(const ckv_layer_args& a, int flat, const UpdateDecision& decision) {
+  constexpr int kInFlight = 4;
+  const Unit u = make_unit(a, flat);
+  if (u.head != u.graph || decision.overflow != 0) {
+    return;
+  }
+  const int d = threadIdx.x;
+  const int capacity = a.community_capacity;
+  const bool wide = (a.flags & CKV_FLAG_FP32_CENTROIDS) != 0;
+  const bool reference_division = (a.flags & CKV_FLAG_REFERENCE_DIVISION) != 0;
+  for (int base = 0; base < a.retrieval_heads; base += kInFlight) {
+    int64_t index[kInFlight];  // of the community in the head's tables, -1: not a follower
+    int size[kInFlight];
+    float key_value[kInFlight], old_value[kInFlight];
+#pragma unroll
+    for (int i = 0; i < kInFlight; ++i) {
+      const int head = base + i;
+      index[i] = -1;
+      size[i] = 0;
+      key_value[i] = old_value[i] = 0.f;
+      if (head >= a.retrieval_heads || head == u.head || a.retrieval_to_graph[head] != u.graph) {
+        continue;
+      }
+      const int other = u.batch * a.retrieval_heads + head;
+      index[i] = static_cast<int64_t>(other) * capacity + decision.assigned;
+      size[i] = a.community_sizes[index[i]];
+      if (d < kHeadDim) {
+        const __nv_bfloat16* key_row =
+            a.current_key != nullptr
+                ? reinterpret_cast<const __nv_bfloat16*>(a.current_key) + static_cast<int64_t>(other) * kHeadDim
+                : reinterpret_cast<const __nv_bfloat16*>(a.key) + u.batch * a.key_batch_stride +
+                      a.retrieval_to_kv[head] * a.key_head_stride +
+                      static_cast<int64_t>(decision.current) * a.key_row_stride;
+        key_value[i] = __bfloat162float(key_row[d]);
+        if (wide) {
+          old_value[i] = reinterpret_cast<const float*>(a.centroids)[index[i] * kHeadDim + d];
+        } else {
+          const __half_raw raw = __nv_cvt_fp8_to_halfraw(
+              reinterpret_cast<const __nv_fp8_storage_t*>(a.centroids)[index[i] * kHeadDim + d], __NV_E4M3);
+          old_value[i] = __half2float(*reinterpret_cast<const __half*>(&raw));
+        }
+      }
+    }
+    __syncthreads();  // every thread has read the sizes
+#pragma unroll
+    for (int i = 0; i < kInFlight; ++i) {
+      if (index[i] < 0) {
+        continue;
+      }
+      if (d == 0) {
+        a.community_sizes[index[i]] = size[i] + 1;
+        a.community_counts[u.batch * a.retrieval_heads + base + i] = decision.count;
+      }
+      if (d < kHeadDim) {
+        const float updated =
+            size[i] > 0 ? centroid_mean(old_value[i], size[i], key_value[i], reference_division) : key_value[i];
+        if (wide) {
+          reinterpret_cast<float*>(a.centroids)[index[i] * kHeadDim + d] = updated;
+        } else {
+          reinterpret_cast<__nv_fp8_storage_t*>(a.centroids)[index[i] * kHeadDim + d] =
+              __nv_cvt_float_to_fp8(updated, __NV_SATFINITE, __NV_E4M3);
+        }
+      }
+    }
+  }
+}
+
 __global__ void __launch_bounds__(kMergeThreads + 32) merge_update_kernel(const ckv_layer_args a) {
   __shared__ UpdateDecision decision;
   __shared__ float lse_s;
   pdl_release_dependents();
   pdl_wait_for_predecessor();  // partials and candidates come from the attention kernel
   merge_update_unit<8>(a, blockIdx.x, kMergeThreads / 32, decision, lse_s);
+  if (a.retrieval_heads != a.graphs && !(a.flags & CKV_FLAG_SKIP_UPDATE)) {
+    sync_followers(a, blockIdx.x, decision);
+  }
   if (blockIdx.x == 0) {
     wait_for_peer_rows(a);
-  }
-}
-
-// Follower heads of a graph shared by several retrieval heads: apply the
-// leader's assignment to their own centroid table.
-__global__ void __launch_bounds__(kMergeThreads) sync_shared_kernel(const ckv_layer_args a) {
-  const int flat = blockIdx.x;
-  const Unit u = make_unit(a, flat);
-  if (u.head == u.graph) {
-    return;
-  }
-  const int d = threadIdx.x;
-  const int capacity = a.community_capacity;
-  const int64_t graph_slot = static_cast<int64_t>(u.batch) * a.graphs + u.graph;
-  const int community = a.assigned[graph_slot];
-  if (a.overflow[graph_slot] != 0 || community < 0) {
-    return;
-  }
-  const int current = a.current_position[graph_slot] - 1;
-  const int64_t size_index = static_cast<int64_t>(flat) * capacity + community;
-  const int old_size = a.community_sizes[size_index];
-  __syncthreads();
-  if (d == 0) {
-    a.community_sizes[size_index] = old_size + 1;
-    a.community_counts[flat] =
-        a.community_counts[static_cast<int64_t>(u.batch) * a.retrieval_heads + u.graph];
-  }
-  if (current >= 0 && current < a.sequence_capacity) {
-    __nv_fp8_storage_t* centroid = reinterpret_cast<__nv_fp8_storage_t*>(a.centroids) +
-                                   size_index * kHeadDim;
-    const __nv_bfloat16* key_row =
-        a.current_key != nullptr
-            ? reinterpret_cast<const __nv_bfloat16*>(a.current_key) + static_cast<int64_t>(flat) * kHeadDim
-            : reinterpret_cast<const __nv_bfloat16*>(a.key) + u.batch * a.key_batch_stride +
-                  u.kv * a.key_head_stride + static_cast<int64_t>(current) * a.key_row_stride;
-    const float key_value = __bfloat162float(key_row[d]);
-    if (a.flags & CKV_FLAG_FP32_CENTROIDS) {
-      float* wide = reinterpret_cast<float*>(a.centroids) + size_index * kHeadDim + d;
-      *wide = old_size > 0 ? centroid_mean(*wide, old_size, key_value,
-                                           (a.flags & CKV_FLAG_REFERENCE_DIVISION) != 0)
-                           : key_value;
-      return;
-    }
-    float updated = key_value;
-    if (old_size > 0) {
-      const __half_raw raw = __nv_cvt_fp8_to_halfraw(centroid[d], __NV_E4M3);
-      const float old_value = __half2float(*reinterpret_cast<const __half*>(&raw));
-      updated = centroid_mean(old_value, old_size, key_value, (a.flags & CKV_FLAG_REFERENCE_DIVISION) != 0);
-    }
-    centroid[d] = __nv_cvt_float_to_fp8(updated, __NV_SATFINITE, __NV_E4M3);
   }
 }
 
@@ -319,16 +343,8 @@ cudaError_t launch_nearest_centroid(const ckv_layer_args& a, int32_t* forced, cu
 }
 
 cudaError_t launch_merge_update(const ckv_layer_args& a, cudaStream_t stream) {
-  cudaError_t err = launch_dependent(merge_update_kernel, dim3(a.batch * a.retrieval_heads),
-                                     dim3(kMergeThreads + 32), 0, stream, a);
-  if (err != cudaSuccess) {
-    return err;
-  }
-  if (a.retrieval_heads != a.graphs && !(a.flags & CKV_FLAG_SKIP_UPDATE)) {
-    sync_shared_kernel<<<a.batch * a.retrieval_heads, kMergeThreads, 0, stream>>>(a);
-    err = cudaGetLastError();
-  }
-  return err;
+  return launch_dependent(merge_update_kernel, dim3(a.batch * a.retrieval_heads), dim3(kMergeThreads + 32), 0, stream,
+                          a);
 }
 
 }  // namespace ckv

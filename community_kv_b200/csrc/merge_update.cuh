@@ -14,6 +14,8 @@ struct UpdateDecision {
   int current;       // cache row of the new token
   int apply;         // 1 when sizes/centroid/labels are to be written
   int valid_position;
+  int overflow;      // the graph's overflow bits of this step
+  int count;         // communities of the graph after the update
   int candidates[kKappa + 1];  // communities the token may join (-1: none), known before the decision
 };
 
@@ -464,6 +466,8 @@ __device__ __forceinline__ void merge_update_unit(const ckv_layer_args& a, int f
       decision.current = current;
       decision.apply = community_overflow ? 0 : 1;
       decision.valid_position = valid_position ? 1 : 0;
+      decision.overflow = overflow;
+      decision.count = active + (join ? 0 : 1);
     }
   }
   if (!leader) {

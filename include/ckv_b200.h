@@ -275,11 +275,11 @@ int ckv_select_descriptors(const ckv_layer_args* args, void* cuda_stream);
  * CKV_FLAG_SKIP_UPDATE) performs the online assignment and state update. */
 int ckv_segmented_attention(const ckv_layer_args* args, void* cuda_stream);
 
-/* A1..A5 back to back: the whole per-layer decode transition.  With one graph per
- * retrieval head, at most eight splits and communities that fit the selection's
- * shared-memory stash, this is ONE launch: a thread-block cluster per (sequence,
- * retrieval head) scores, selects, attends, merges and updates, synchronising
- * through cluster barriers.  With more splits it is one launch of up to sixteen CTAs
+/* A1..A5 back to back: the whole per-layer decode transition.  With at most eight
+ * splits and communities that fit the selection's shared-memory stash, this is ONE
+ * launch: a thread-block cluster per (sequence, retrieval head) scores, selects,
+ * attends, merges and updates, synchronising through cluster barriers (graphs shared
+ * by several retrieval heads are updated by a second kernel behind it).  With more splits it is one launch of up to sixteen CTAs
  * per unit where that was measured to be the faster route.  Otherwise (or with
  * CKV_FLAG_UNFUSED) the four stand-alone kernels run back to back.  Results are
  * identical either way. */
@@ -320,7 +320,7 @@ int ckv_wait_peers(uint32_t* flag, uint32_t expected, uint32_t* status, void* cu
  * ckv_decode_layer / ckv_online_update. */
 int ckv_nearest_centroid(const ckv_layer_args* args, int32_t* forced_community, void* cuda_stream);
 
-/* How many kernels ckv_decode_layer launches for these arguments (1, 4 or 5);
+/* How many kernels ckv_decode_layer launches for these arguments (1, 2 or 4);
  * no reference counterpart, used for launch accounting. */
 int ckv_decode_layer_kernels(const ckv_layer_args* args);
 

@@ -540,6 +540,44 @@ def test_append_kv_moves_the_cursor(units):
         ops.append_kv(key[:4], value[:4], new_key[:4], new_value[:4], cursor.repeat(4), advance=True)
 
 
+@pytest.mark.parametrize("kv_heads,group,fp32,deferred", [(2, 4, False, False), (5, 2, False, True), (9, 1, False, False),
+                                                          (6, 2, True, False)])
+def test_shared_graph_in_two_launches(monkeypatch, kv_heads, group, fp32, deferred):
+    """One graph for all heads: the cluster launch and the update behind it (or beside the next step) leave the
+    bits of the four stand-alone kernels, the followers' tables included (four of them at a time, and remainders)."""
+
+    device = torch.device("cuda", 0)
+    config = CommunityKVConfig(token_budget=512, num_sink=10, lam=0.5, aggregation="layer_wise",
+                               centroid_dtype="fp32" if fp32 else "e4m3")
+    layer = make_layer(seed=90 + kv_heads, seq_len=3001, communities=60, kv_heads=kv_heads, group_size=group,
+                       max_decode_tokens=8, aggregation="layer_wise")
+    if fp32:
+        layer.assembled.centroids = layer.assembled.centroids.float()
+    layer = layer.to(device)
+    key, value = layer.key[None], layer.value[None]
+
+    def run(unfused):
+        monkeypatch.setenv("CKV_UNFUSED", unfused)
+        runtime = DecodeRuntime(config, defer_update=deferred)
+        state = runtime.prepare_layer(0, **{k: v.clone() if isinstance(v, torch.Tensor) else v
+                                            for k, v in layer.prepare_kwargs().items()})
+        outputs = []
+        for step in range(6):
+            query = make_query(seed=900 + step, query_heads=kv_heads * group).to(device)
+            outputs.append(runtime.decode(layer_idx=0, query=query.view(1, kv_heads * group, 1, 128), key=key,
+                                          value=value, softmax_scale=SCALE).clone())
+        runtime.assert_no_overflow()
+        launched = native.library().ckv_decode_layer_kernels(ctypes.byref(state.args))
+        ws = state.workspace.attention
+        return launched, [*outputs, ws.lse, ws.topk_scores, ws.topk_positions, *state.converted.mutable.tensors()]
+
+    four, want = run("1")
+    launched, got = run("0")
+    assert (four, launched) == (4, 4 if fp32 else 2)
+    for first, second in zip(got, want):
+        assert torch.equal(first.contiguous().view(torch.uint8), second.contiguous().view(torch.uint8))
+
+
 def test_full_size_batch_one_launch_equals_four_kernels():
     """The batched long-context configuration as far as one layer goes (8 sequences x 8 KV heads at ctx 131072,
     1024-4096 Zipf communities, budget 2048): the single cluster launch and the four
