@@ -1,7 +1,8 @@
 // Prefill attention with the reference's top-8 rule, two heads per CTA (sm_100a).
 //
-// One CTA owns 128 consecutive positions of TWO query heads of one KV group (two
-// 128-row tiles that share every K/V tile) and is split into roles:
+// An item is 128 consecutive positions of TWO query heads of one KV group (two 128-row tiles
+// that share every K/V tile).  One CTA per SM works through its items, the longest first (see
+// PairItem), and is split into roles:
 //   warps 0-3  softmax of tile 0, one thread per row (all 128 columns of a key block);
 //   warps 4-7  softmax of tile 1;
 //   warp 8     one lane feeds the K and V rings (and Q) with bulk tensor copies;
@@ -17,6 +18,9 @@
 // the whole row; a row's running maximum only moves when the new one is more than 2^8
 // above it, and the row of O is then rescaled in place by its own thread.
 // Every wait is bounded; a wait that runs out sets the status word and the CTA drains.
+// Between two items nothing waits for the whole CTA: the next Q is fetched when the last S
+// of the item is done, its first S is issued behind the item's last P.V, and the softmax
+// threads write the item's output meanwhile.
 //
 // The top-8 rule is the one of prefill_topk.cu (community-kv.patch,
 // hopper/topk_warpselect.h): per row, four classes of columns (class = (j % 8) / 2)
@@ -28,6 +32,7 @@ namespace ckv {
 
 namespace {
 
+constexpr int kPairCtas = 148;     // one per SM
 constexpr int kPairThreads = 384;  // three warpgroups: two of softmax rows, one of helpers
 
 struct PairSmem {
@@ -123,6 +128,21 @@ __device__ __forceinline__ bool pair_wait(uint32_t bar, uint32_t parity, volatil
   return false;
 }
 
+// One look at a barrier.  The answer takes about 200 cycles; what follows may run meanwhile.
+__device__ __forceinline__ bool pair_test(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return done != 0u;
+}
+
 // The same for a whole warp: lane 0 polls, the others take its word.  The barrier's
 // completion is made visible to the waiting lanes by one successful test of their own.
 __device__ __forceinline__ bool pair_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t* abort) {
@@ -165,6 +185,13 @@ __device__ __forceinline__ void sorted_insert(uint32_t (&queue)[kDepth], uint32_
     queue[k] = max(queue[k], min(queue[k - 1], candidate));
   }
   queue[0] = max(queue[0], candidate);
+}
+
+// Largest of three in one operation
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float y;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+  return y;
 }
 
 // Minimum that does not lose a NaN
@@ -227,6 +254,38 @@ __device__ __forceinline__ void take_candidates(const float (&s)[128], float gat
   }
 }
 
+// The items of the launch in descending length: all head pairs' last tiles, then all tiles before
+// them.  CTA i takes item i of the first gridDim.x, item i from the end of the next, and so on.
+// Causal items differ in length: with one CTA per item and one head's items behind another's, the
+// last head's longest item started when the rest of the chip was nearly done (SMs busy for 82 % of
+// a call of 8192 tokens), and every item paid for filling its pipeline (about 20000 cycles of
+// launch, Q and first K, output, against 3700 per key block).  32 query on 8 KV heads, us a call,
+// before / now, attention alone and with neighbours: 1500 tokens 97 / 88 and 150 / 128, 6001 tokens
+// 375 / 327 and 588 / 526, 16384 tokens 1870 / 1790 and 2690 (2850 in some runs) / 2680 to 2860.
+struct PairItem {
+  int pos0, blocks, head0, kv_head, batch;
+
+  // The CTA's item `n`; false behind its last one.
+  __device__ __forceinline__ bool set(const ckv_prefill_args& a, int n) {
+    const int pairs = (a.query_heads / a.kv_heads) >> 1;
+    const int lanes = a.kv_heads * pairs * a.batch;  // head pairs of all sequences
+    const int tiles = (a.seq_len + kPfRows - 1) / kPfRows;
+    const int ctas = static_cast<int>(gridDim.x), cta = static_cast<int>(blockIdx.x);
+    const int64_t item = static_cast<int64_t>(n) * ctas + ((n & 1) ? ctas - 1 - cta : cta);
+    if (item >= static_cast<int64_t>(lanes) * tiles) {
+      return false;
+    }
+    const int tile = tiles - 1 - static_cast<int>(item / lanes);
+    const int pair = static_cast<int>(item % lanes);
+    batch = pair / (a.kv_heads * pairs);
+    kv_head = pair / pairs % a.kv_heads;
+    head0 = 2 * (pair - batch * a.kv_heads * pairs);
+    pos0 = tile * kPfRows;
+    blocks = tile + 1;  // key blocks 0 .. tile; the last one holds the diagonal
+    return true;
+  }
+};
+
 template <int kMode>
 __global__ void __launch_bounds__(kPairThreads, 1)
     prefill_pair_kernel(const ckv_prefill_args a, const __grid_constant__ CUtensorMap map_q,
@@ -240,15 +299,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
-  const int group = a.query_heads / a.kv_heads;
-  const int pairs = group >> 1;
-  const int tile = gridDim.x - 1 - blockIdx.x;  // longest rows first
-  const int kv_head = blockIdx.y / pairs;
-  const int head0 = kv_head * group + 2 * (blockIdx.y % pairs);
-  const int batch = blockIdx.z;
   const int length = a.seq_len;
-  const int pos0 = tile * kPfRows;
-  const int blocks = tile + 1;  // key blocks 0 .. tile; the last one holds the diagonal
 
   const uint32_t q_addr = smem_u32(smem + PairSmem::kQ);
   const uint32_t k_addr = smem_u32(smem + PairSmem::kK);
@@ -260,6 +311,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   const uint32_t bar_s_full = smem_u32(bars + 9);   // per tile: S written
   const uint32_t bar_p_full = smem_u32(bars + 11);  // per tile: P written by its four warps
   const uint32_t bar_o_full = smem_u32(bars + 13);  // per tile: P.V folded into O
+  const uint32_t bar_q_free = smem_u32(bars + 7);   // the item's last S of both tiles done
 
   // a wait already ran out somewhere in this launch: drain the grid quickly
   const bool drained = a.status != nullptr &&
@@ -295,36 +347,46 @@ __global__ void __launch_bounds__(kPairThreads, 1)
 
   // Register hand-over between the warpgroups.  setmaxnreg.inc blocks until the registers
   // are free, without any bound: the totals must never exceed what the launch allocated
-  // (384 threads x 168 registers = 256 x 216 + 128 x 72).
-  static_assert(256 * 216 + 128 * 72 <= kPairThreads * 168, "register hand-over exceeds the launch allocation");
+  // (384 threads x 168 registers = 256 x 208 + 128 x 88).
+  static_assert(256 * 208 + 128 * 88 <= kPairThreads * 168, "register hand-over exceeds the launch allocation");
   if (warp >= 8) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
   }
   if (warp >= 10) {
     // nothing to do
   } else if (warp == 8) {
     // ---- producer ----
     if (lane == 0) {
-      mbar_expect_tx(bar_q, 2 * kTileBytes);
-      tma_issue_tile(q_addr, &map_q, bar_q, pos0, head0, batch);
-      tma_issue_tile(q_addr + kTileBytes, &map_q, bar_q, pos0, head0 + 1, batch);
-      for (int block = 0; block < blocks; ++block) {
-        const int stage = block & 1;
-        // K(block) goes where K(block - 2) was: free once both tiles' S(block - 2) is done
-        if (block >= 2 && !pair_wait(bar_k_free + 8 * stage, ((block >> 1) - 1) & 1, abort)) {
-          failed = true;
-          break;
+      int step = 0;  // key blocks so far, over all items
+      PairItem item;
+      for (int n = 0; !failed && item.set(a, n); ++n) {
+        for (int block = 0; block < item.blocks; ++block, ++step) {
+          const int stage = step & 1;
+          // K goes where K(step - 2) was: free once both tiles' S(step - 2) is done
+          if (step >= 2 && !pair_wait(bar_k_free + 8 * stage, ((step >> 1) - 1) & 1, abort)) {
+            failed = true;
+            break;
+          }
+          tma_load_tile(k_addr + stage * kTileBytes, &map_k, bar_k_full + 8 * stage, block * kPfKeys,
+                        item.kv_head, item.batch);
+          if (block == 0) {
+            if (n > 0 && !pair_wait(bar_q_free, (n - 1) & 1, abort)) {
+              failed = true;
+              break;
+            }
+            mbar_expect_tx(bar_q, 2 * kTileBytes);
+            tma_issue_tile(q_addr, &map_q, bar_q, item.pos0, item.head0, item.batch);
+            tma_issue_tile(q_addr + kTileBytes, &map_q, bar_q, item.pos0, item.head0 + 1, item.batch);
+          }
+          // V goes where V(step - 2) was.  S(step - 1) is committed after both
+          // P.V(step - 2) were issued, so that barrier covers the products that read the stage.
+          if (step >= 2 && !pair_wait(bar_k_free + 8 * (stage ^ 1), ((step - 1) >> 1) & 1, abort)) {
+            failed = true;
+            break;
+          }
+          tma_load_tile(v_addr + stage * kTileBytes, &map_v, bar_v_full + 8 * stage, block * kPfKeys,
+                        item.kv_head, item.batch);
         }
-        tma_load_tile(k_addr + stage * kTileBytes, &map_k, bar_k_full + 8 * stage, block * kPfKeys,
-                      kv_head, batch);
-        // V(block) goes where V(block - 2) was.  S(block - 1) is committed after both
-        // P.V(block - 2) were issued, so that barrier covers the products that read the stage.
-        if (block >= 2 && !pair_wait(bar_k_free + 8 * (stage ^ 1), ((block - 1) >> 1) & 1, abort)) {
-          failed = true;
-          break;
-        }
-        tma_load_tile(v_addr + stage * kTileBytes, &map_v, bar_v_full + 8 * stage, block * kPfKeys,
-                      kv_head, batch);
       }
     }
   } else if (warp == 9) {
@@ -365,53 +427,88 @@ __global__ void __launch_bounds__(kPairThreads, 1)
                         desc_high, idesc_pv, true);
         }
       };
-      if (pair_wait(bar_q, 0, abort) && pair_wait(bar_k_full, 0, abort)) {
+      // S(step) behind P.V(step - 1), of the same item or of the one before.  This lane sets the
+      // pace of the CTA where there are no neighbours to keep: 32 products of 64 cycles per key
+      // block, and the products wait while it waits.  So it asks for the barriers that are usually
+      // complete by then (K, V, the second tile's P) one group of products ahead; a barrier asked
+      // for when it is needed costs 200 cycles, complete or not.
+      int step = 0;
+      PairItem item, next;
+      bool any = item.set(a, 0);
+      failed = any && !(pair_wait(bar_q, 0, abort) && pair_wait(bar_k_full, 0, abort));
+      if (any && !failed) {
         tc_fence_after();
         issue_qk(0, 0);
         issue_qk(1, 0);
-        for (int block = 0; block < blocks && !failed; ++block) {
-          const int stage = block & 1;
-          const bool more = block + 1 < blocks;
-          if (!pair_wait(bar_v_full + 8 * stage, (block >> 1) & 1, abort)) {
+        if (item.blocks == 1) {
+          umma_commit(bar_q_free);
+        }
+      }
+      bool v_ready = false;
+      for (int n = 0; any && !failed; ++n) {
+        const bool another = next.set(a, n + 1);
+        for (int block = 0; block < item.blocks; ++block, ++step) {
+          const int stage = step & 1;
+          const bool last = block + 1 == item.blocks;
+          const bool more = !last || another;
+          const uint32_t next_parity = ((step + 1) >> 1) & 1;
+          if (!pair_wait(bar_p_full, step & 1, abort) ||
+              (!v_ready && !pair_wait(bar_v_full + 8 * stage, (step >> 1) & 1, abort))) {
             failed = true;
             break;
           }
-#pragma unroll
-          for (int t = 0; t < 2; ++t) {
-            if (!pair_wait(bar_p_full + 8 * t, block & 1, abort)) {
-              failed = true;
-              break;
-            }
+          tc_fence_after();
+          const bool k_ready = pair_test(bar_k_full + 8 * (stage ^ 1), next_parity);
+          issue_pv(0, stage, block > 0);
+          if (last) {
+            umma_commit(bar_o_full);
+          }
+          if (more && ((!k_ready && !pair_wait(bar_k_full + 8 * (stage ^ 1), next_parity, abort)) ||
+                       (last && !pair_wait(bar_q, (n + 1) & 1, abort)))) {
+            failed = true;
+            break;
+          }
+          const bool p_ready = pair_test(bar_p_full + 8, step & 1);
+          if (more) {
             tc_fence_after();
-            issue_pv(t, stage, block > 0);
-            if (!more) {
-              umma_commit(bar_o_full + 8 * t);
-            } else {
-              if (t == 0 && !pair_wait(bar_k_full + 8 * (stage ^ 1), ((block + 1) >> 1) & 1, abort)) {
-                failed = true;
-                break;
-              }
-              tc_fence_after();
-              issue_qk(t, stage ^ 1);
+            issue_qk(0, stage ^ 1);
+          }
+          if (!p_ready && !pair_wait(bar_p_full + 8, step & 1, abort)) {
+            failed = true;
+            break;
+          }
+          tc_fence_after();
+          v_ready = pair_test(bar_v_full + 8 * (stage ^ 1), next_parity);
+          issue_pv(1, stage, block > 0);
+          if (last) {
+            umma_commit(bar_o_full + 8);
+          }
+          if (more) {
+            issue_qk(1, stage ^ 1);
+            // the S just issued is its item's last: Q may be overwritten once it is done
+            if (last ? next.blocks == 1 : block + 2 == item.blocks) {
+              umma_commit(bar_q_free);
             }
           }
         }
-      } else {
-        failed = true;
+        item = next;
+        any = another;
       }
     }
   } else {
     // ---- softmax of tile t, one thread per row ----
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
     const int t = warp >> 2;
     const int row = tid & (kPfRows - 1);
-    const int row_pos = pos0 + row;
-    const int row_head = head0 + t;
-    const bool row_live = row_pos < length;
     const uint32_t lane_base = tmem + (((warp & 3) * 32u) << 16);
     const uint32_t s_addr = lane_base + t * 128u;
     const uint32_t o_addr = lane_base + 256u + t * 128u;
     const float scale_log2 = a.softmax_scale * kLog2e;
+    int step = 0;  // key blocks so far, over all items
+    PairItem item;
+    for (int n = 0; !failed && item.set(a, n); ++n) {
+    const int blocks = item.blocks;
+    const bool live = item.pos0 + row < length;
     float run_max = -INFINITY;  // of the raw (unscaled) scores
     float run_sum = 0.f;
     uint32_t q32[4][kLocalK];
@@ -425,9 +522,9 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       }
     }
 
-    for (int block = 0; block < blocks; ++block) {
+    for (int block = 0; block < blocks; ++block, ++step) {
       const int key0 = block * kPfKeys;
-      if (!pair_wait_warp(bar_s_full + 8 * t, block & 1, abort)) {
+      if (!pair_wait_warp(bar_s_full + 8 * t, step & 1, abort)) {
         failed = true;
         break;
       }
@@ -454,17 +551,15 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       float part_max[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        part_max[i] = fmaxf(s[i], s[i + 8]);
-      }
+        part_max[i] = max3(s[i], s[i + 8], s[i + 16]);
 #pragma unroll
-      for (int c = 16; c < 128; c += 16) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          part_max[i] = fmaxf(part_max[i], fmaxf(s[c + i], s[c + i + 8]));
+        for (int c = 24; c < 120; c += 16) {
+          part_max[i] = max3(part_max[i], s[c + i], s[c + i + 8]);
         }
+        part_max[i] = fmaxf(part_max[i], s[120 + i]);
       }
-      const float tile_max = fmaxf(fmaxf(fmaxf(part_max[0], part_max[1]), fmaxf(part_max[2], part_max[3])),
-                                   fmaxf(fmaxf(part_max[4], part_max[5]), fmaxf(part_max[6], part_max[7])));
+      const float tile_max = max3(max3(part_max[0], part_max[1], part_max[2]),
+                                  max3(part_max[3], part_max[4], part_max[5]), fmaxf(part_max[6], part_max[7]));
 
       // The running maximum only moves when the new one lies more than 2^8 above it
       // (probabilities up to 256 are harmless in bf16 / fp32); moving it means rescaling
@@ -568,7 +663,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
                          ? -3.0e38f
                          : (static_cast<float>(floor_key) - 0.75f) * (1.0f / 256.0f) - 48.0f;
         // rows behind the end of a ragged prompt score 0 everywhere: ties that all reach the gate
-        gate = row_live ? gate : INFINITY;
+        gate = live ? gate : INFINITY;
         // (no vote in front of a class: in most blocks some row of the warp has a taker)
         take_candidates<0>(s, gate, key0, sinks, q32[0]);
         take_candidates<1>(s, gate, key0, sinks, q32[1]);
@@ -578,14 +673,21 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     }
 
     if (!failed) {
-      if (!pair_wait_warp(bar_o_full + 8 * t, 0, abort)) {
+      if (!pair_wait_warp(bar_o_full + 8 * t, n & 1, abort)) {
         failed = true;
       }
     }
     if (!failed) {
       tc_fence_after();
+      // where the rows go is worked out again: through the loop it would cost registers
+      int again = n;
+      asm volatile("" : "+r"(again));
+      item.set(a, again);
+      const int row_pos = item.pos0 + row;
+      const int row_head = item.head0 + t;
+      const bool row_live = row_pos < length;
       const float inverse = 1.f / run_sum;
-      __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.output) + batch * a.o_batch_stride +
+      __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.output) + item.batch * a.o_batch_stride +
                            static_cast<int64_t>(row_live ? row_pos : 0) * a.o_row_stride +
                            row_head * a.o_head_stride;
 #pragma unroll
@@ -608,14 +710,14 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       if (row_live) {
         const float lse = run_max * a.softmax_scale + logf(run_sum);
         const int64_t heads_total = a.query_heads;
-        a.lse[(batch * heads_total + row_head) * length + row_pos] = lse;
+        a.lse[(item.batch * heads_total + row_head) * length + row_pos] = lse;
         if constexpr (kMode == 1) {
           const int skip = a.num_sink + kKappa - 1;
           if (row_pos >= skip) {
             // merge the four sorted class queues: eight times the largest head, which then
             // leaves its queue (a cursor per queue would put the queues into local memory)
             const int64_t base =
-                ((batch * heads_total + row_head) * (length - skip) + (row_pos - skip)) * kKappa;
+                ((item.batch * heads_total + row_head) * (length - skip) + (row_pos - skip)) * kKappa;
             const float lse_log2 = lse * kLog2e;
 #pragma unroll
             for (int rank = 0; rank < kKappa; ++rank) {
@@ -635,6 +737,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
           }
         }
       }
+    }
     }
   }
 
@@ -663,7 +766,8 @@ cudaError_t launch_prefill_pair(const ckv_prefill_args& a, cudaStream_t stream) 
       !tile_map(&map_v, a.value, a, a.kv_heads, a.v_row_stride, a.v_head_stride, a.v_batch_stride, true)) {
     return cudaErrorInvalidValue;
   }
-  const dim3 grid((a.seq_len + kPfRows - 1) / kPfRows, a.kv_heads * (group / 2), a.batch);
+  const int64_t items = static_cast<int64_t>((a.seq_len + kPfRows - 1) / kPfRows) * a.kv_heads * (group / 2) * a.batch;
+  const unsigned grid = static_cast<unsigned>(items < kPairCtas ? items : kPairCtas);
   auto run = [&](auto kernel) -> cudaError_t {
     cudaError_t err =
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem::kTotal);

@@ -131,9 +131,11 @@ __global__ void __launch_bounds__(kPfThreads, 1)
   const int row = tid & (kPfRows - 1);
   const int half = tid >> 7;            // which 64 of the 128 columns / output dims
   const int col0 = half * 64;
-  const int tile = gridDim.x - 1 - blockIdx.x;  // longest rows first
-  const int kv_head = blockIdx.y;
-  const int batch = blockIdx.z;
+  // all heads' longest tiles first, then the tiles before them
+  const int lanes = a.kv_heads * a.batch;
+  const int tile = (gridDim.x - 1 - blockIdx.x) / lanes;
+  const int kv_head = blockIdx.x % lanes % a.kv_heads;
+  const int batch = blockIdx.x % lanes / a.kv_heads;
   const int pos0 = tile * kPositions;
   const int length = a.seq_len;
   const int row_pos = pos0 + row / kGroup;
@@ -562,7 +564,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
     return;
   }
   const float lse = run_max * a.softmax_scale + logf(total);
-  const int64_t heads_total = static_cast<int64_t>(gridDim.y) * kGroup;
+  const int64_t heads_total = static_cast<int64_t>(a.kv_heads) * kGroup;
   a.lse[(batch * heads_total + row_head) * length + row_pos] = lse;
 
   if constexpr (kMode == 1) {
@@ -624,7 +626,7 @@ __global__ void __launch_bounds__(kPfThreads, 1)
     }
     // [batch, kv head, position, G lanes, 16 kept + best dropped] for the second kernel
     uint64_t* list = a.candidates +
-                     (((static_cast<int64_t>(batch) * gridDim.y + kv_head) * length + row_pos) * kGroup +
+                     (((static_cast<int64_t>(batch) * a.kv_heads + kv_head) * length + row_pos) * kGroup +
                       row % kGroup) * (kExactKeep + 1);
 #pragma unroll
     for (int k = 0; k < kExactKeep; ++k) {
@@ -969,9 +971,10 @@ __global__ void __launch_bounds__(kEdgeThreads, 1)
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
-  const int tile = gridDim.x - 1 - blockIdx.x;  // longest tiles first
-  const int kv_head = blockIdx.y;
-  const int batch = blockIdx.z;
+  const int lanes = a.kv_heads * a.batch;
+  const int tile = (gridDim.x - 1 - blockIdx.x) / lanes;  // all heads' longest tiles first (see tile_grid)
+  const int kv_head = blockIdx.x % lanes % a.kv_heads;
+  const int batch = blockIdx.x % lanes / a.kv_heads;
   const int length = a.seq_len;
   const int pos0 = tile * kPfRows;
   const int last_pos = min(length, pos0 + kPfRows) - 1;
@@ -1179,7 +1182,7 @@ __global__ void __launch_bounds__(kEdgeThreads, 1)
     if (row_live && !failed) {
       // [batch, kv head, position, 2 lists, 16 kept + best dropped]: this thread's is list `wg`
       uint64_t* out = a.candidates +
-                      ((static_cast<int64_t>(batch) * gridDim.y + kv_head) * length + row_pos) *
+                      ((static_cast<int64_t>(batch) * a.kv_heads + kv_head) * length + row_pos) *
                           2 * (kExactKeep + 1);
 #pragma unroll
       for (int k = 0; k < kKeep; ++k) {
@@ -1252,6 +1255,16 @@ bool tile_map(CUtensorMap* map, const void* base, const ckv_prefill_args& a, int
 
 namespace {
 
+// CTAs of a launch with one tile of `positions` positions of one KV head each.  Causal tiles differ
+// in length, so the kernels number them with all heads' longest tiles first: with one head's tiles
+// behind another's, the last head's longest tile started when the rest of the chip was nearly done
+// (8192 tokens, 32 query on 8 KV heads: SMs busy for 82 % of the candidate and the attention kernel).
+unsigned tile_grid(const ckv_prefill_args& a, int positions) {
+  const int64_t tiles = (a.seq_len + positions - 1) / positions;
+  const int64_t ctas = tiles * a.kv_heads * a.batch;
+  return ctas <= 0x7fffffff ? static_cast<unsigned>(ctas) : 0u;
+}
+
 template <int kGroup>
 cudaError_t launch_for_group(const ckv_prefill_args& a, cudaStream_t stream) {
   if constexpr (kGroup % 2 == 0) {
@@ -1259,7 +1272,8 @@ cudaError_t launch_for_group(const ckv_prefill_args& a, cudaStream_t stream) {
     if (a.mode != 2) return launch_prefill_pair(a, stream);
   }
   constexpr int kSmem = PrefillSmem::kTotal;
-  const dim3 grid((a.seq_len + kPfRows / kGroup - 1) / (kPfRows / kGroup), a.kv_heads, a.batch);
+  const unsigned grid = tile_grid(a, kPfRows / kGroup);
+  if (grid == 0u) return cudaErrorInvalidConfiguration;
   CUtensorMap map_k, map_v;
   if (!tile_map(&map_k, a.key, a, a.kv_heads, a.k_row_stride, a.k_head_stride, a.k_batch_stride) ||
       !tile_map(&map_v, a.value, a, a.kv_heads, a.v_row_stride, a.v_head_stride, a.v_batch_stride)) {
@@ -1295,7 +1309,8 @@ cudaError_t launch_candidates(const ckv_prefill_args& a, cudaStream_t stream) {
   err = cudaFuncSetAttribute(edge_candidates_kernel<kGroup>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
   if (err != cudaSuccess) return err;
-  const dim3 grid((a.seq_len + kPfRows - 1) / kPfRows, a.kv_heads, a.batch);
+  const unsigned grid = tile_grid(a, kPfRows);
+  if (grid == 0u) return cudaErrorInvalidConfiguration;
   edge_candidates_kernel<kGroup><<<grid, kEdgeThreads, kSmem, stream>>>(a, map_q, map_k);
   return cudaGetLastError();
 }

@@ -342,3 +342,32 @@ def test_plugin_prefill_reads_the_cache_where_it_lies(room, shift):
         SimpleNamespace(layer_idx=0), placed(q, length), placed(k, length + room), placed(v, length + room), None, SCALE)
     assert torch.equal(out, want[0])
     assert torch.equal(edges["topk_indices"], want[5][0]) and torch.equal(edges["topk_scores"], want[4][0])
+
+
+@pytest.mark.parametrize("kv_heads,batch,length", [(149, 1, 120), (33, 9, 120), (74, 1, 200), (75, 1, 200), (25, 6, 300)])
+def test_prefill_items_over_the_ctas(kv_heads, batch, length):
+    """One or several tiles per CTA of the head-pair kernel (148 of them), tiles of one key block next to longer ones:
+    the bits do not depend on which tiles a CTA works through."""
+
+    generator = torch.Generator(device="cuda").manual_seed(length + kv_heads)
+
+    def rows(heads):
+        return torch.randn((batch, length, heads, 128), generator=generator, device="cuda").to(torch.bfloat16)
+
+    q, k, v = rows(2 * kv_heads), rows(kv_heads), rows(kv_heads)
+    k = k * 0.3
+    out, lse, _, _, val, idx = prefill_attention_topk(q, k, v, softmax_scale=SCALE, num_sink=3)
+    plain, plain_lse = prefill_attention(q, k, v, softmax_scale=SCALE)
+    for b in {0, batch // 2, batch - 1}:
+        for h in {0, 1, kv_heads // 2, kv_heads - 1}:
+            alone = prefill_attention_topk(q[b : b + 1, :, 2 * h : 2 * h + 2].contiguous(), k[b : b + 1, :, h : h + 1].contiguous(),
+                                           v[b : b + 1, :, h : h + 1].contiguous(), softmax_scale=SCALE, num_sink=3)
+            pair = slice(2 * h, 2 * h + 2)
+            assert torch.equal(out[b, :, pair], alone[0][0]) and torch.equal(lse[b, pair], alone[1][0])
+            assert torch.equal(val[b, pair], alone[4][0]) and torch.equal(idx[b, pair], alone[5][0])
+            want = torch.nn.functional.scaled_dot_product_attention(
+                q[b, :, pair].float().transpose(0, 1), k[b, :, h].float().expand(2, -1, -1),
+                v[b, :, h].float().expand(2, -1, -1), is_causal=True, scale=SCALE).transpose(0, 1)
+            assert float((out[b, :, pair].float() - want).abs().max()) <= 2e-2
+    # the plain kernel works through the same tiles; its sums are those of the other
+    assert torch.equal(plain, out) and torch.equal(plain_lse, lse)
