@@ -644,6 +644,12 @@ __global__ void __launch_bounds__(kPfThreads, 1)
 // index ascending).  A row is flagged when
 // a key that was turned away could still belong to the top-m: the best
 // approximate score among the dropped keys is within `slack` of the exact m-th.
+// The candidates' key rows lie anywhere in the cache, and a lane needs a whole one: the warp
+// copies 32 of them together, two full rows per instruction, into a tile of shared memory whose
+// 16-byte chunks are XOR-ed with the row's low bits, from which every lane reads its own without
+// a conflict (every lane loading its own row from global memory touched 32 lines per instruction).
+// Up to 32 candidates are ranked by a sort over the lanes.  32 query on 8 KV heads, sixteen edges, a
+// whole call: 6001 tokens 991 -> 910 us, 1500 tokens 279 -> 254 us.
 __global__ void __launch_bounds__(128) exact_edges_kernel(const ckv_prefill_args a, int group, int lists) {
   const int warps_per_block = 4;
   const int warp = threadIdx.x >> 5;
@@ -670,6 +676,8 @@ __global__ void __launch_bounds__(128) exact_edges_kernel(const ckv_prefill_args
   const int candidates = lists * kExactKeep;  // <= 128
   // the position's query rows, staged once per warp (every candidate reuses them)
   __shared__ uint4 q_stage[4][8 * 16];
+  __shared__ __align__(16) uint4 k_stage[4][32 * 16];
+  const uint32_t k_tile = smem_u32(k_stage[warp]);
   for (int index = lane; index < group * 16; index += 32) {
     q_stage[warp][index] = *reinterpret_cast<const uint4*>(q_base + (index >> 4) * a.q_head_stride +
                                                            (index & 15) * 8);
@@ -686,23 +694,36 @@ __global__ void __launch_bounds__(128) exact_edges_kernel(const ckv_prefill_args
 #pragma unroll
   for (int slot = 0; slot < 4; ++slot) {
     best_key[slot] = 0ull;
+    if (32 * slot >= candidates) {
+      continue;  // the same for the whole warp
+    }
     const int index = lane + 32 * slot;
-    if (index >= candidates) {
+    int j = -1;
+    if (index < candidates) {
+      const uint64_t packed = list[(index / kExactKeep) * (kExactKeep + 1) + index % kExactKeep];
+      // the lists of a launch that gave up a wait may hold anything
+      j = packed == 0ull ? -1 : static_cast<int>(0xffffffffu - static_cast<uint32_t>(packed));
+      j = j > pos ? -1 : j;
+    }
+    __syncwarp();  // the last slot's rows have been read
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int row = 2 * i + (lane >> 4);
+      const int chunk = lane & 15;
+      const int from = __shfl_sync(0xffffffffu, j, row);
+      cp_async16(k_tile + row * 256 + ((chunk ^ (row & 7)) << 4),
+                 k_base + static_cast<int64_t>(max(from, 0)) * a.k_row_stride + chunk * 8, from >= 0 ? 16u : 0u);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncwarp();
+    if (j < 0) {
       continue;
     }
-    const uint64_t packed = list[(index / kExactKeep) * (kExactKeep + 1) + index % kExactKeep];
-    if (packed == 0ull) {
-      continue;
-    }
-    const int j = static_cast<int>(0xffffffffu - static_cast<uint32_t>(packed));
-    if (j < 0 || j > pos) {
-      continue;  // the lists of a launch that gave up a wait may hold anything
-    }
-    const uint4* k_row = reinterpret_cast<const uint4*>(k_base + static_cast<int64_t>(j) * a.k_row_stride);
     uint4 k_reg[16];
 #pragma unroll
     for (int piece = 0; piece < 16; ++piece) {
-      k_reg[piece] = k_row[piece];
+      k_reg[piece] = k_stage[warp][lane * 16 + (piece ^ (lane & 7))];
     }
     float score = -INFINITY;
     for (int g = 0; g < group; ++g) {
@@ -740,24 +761,44 @@ __global__ void __launch_bounds__(128) exact_edges_kernel(const ckv_prefill_args
   const int64_t out_base = ((static_cast<int64_t>(batch) * a.kv_heads + kv_head) * rows + (pos - skip)) *
                            a.edges_per_row;
   float last_score = 0.f;
-  for (int rank = 0; rank < a.edges_per_row; ++rank) {
-    uint64_t local = 0ull;
+  if (candidates <= 32) {
+    // bitonic sort over the lanes, the largest first
+    uint64_t key = best_key[0];
 #pragma unroll
-    for (int slot = 0; slot < 4; ++slot) {
-      local = best_key[slot] > local ? best_key[slot] : local;
-    }
-    const uint64_t winner = warp_max_u64(local);
-    if (winner != 0ull) {
+    for (int width = 2; width <= 32; width <<= 1) {
 #pragma unroll
-      for (int slot = 0; slot < 4; ++slot) {
-        best_key[slot] = best_key[slot] == winner ? 0ull : best_key[slot];
+      for (int step = width >> 1; step > 0; step >>= 1) {
+        const uint64_t other = __shfl_xor_sync(0xffffffffu, key, step);
+        const bool larger = ((lane & width) == 0) == ((lane & step) == 0);
+        key = (other > key) == larger ? other : key;
       }
     }
-    last_score = key32_to_float(static_cast<uint32_t>(winner >> 32));
-    if (lane == 0) {
-      a.edge_idx[out_base + rank] =
-          winner == 0ull ? -1 : static_cast<int32_t>(0xffffffffu - static_cast<uint32_t>(winner));
-      a.edge_score[out_base + rank] = winner == 0ull ? -INFINITY : last_score;
+    if (lane < a.edges_per_row) {
+      a.edge_idx[out_base + lane] =
+          key == 0ull ? -1 : static_cast<int32_t>(0xffffffffu - static_cast<uint32_t>(key));
+      a.edge_score[out_base + lane] = key == 0ull ? -INFINITY : key32_to_float(static_cast<uint32_t>(key >> 32));
+    }
+    last_score = key32_to_float(__shfl_sync(0xffffffffu, static_cast<uint32_t>(key >> 32), a.edges_per_row - 1));
+  } else {
+    for (int rank = 0; rank < a.edges_per_row; ++rank) {
+      uint64_t local = 0ull;
+#pragma unroll
+      for (int slot = 0; slot < 4; ++slot) {
+        local = best_key[slot] > local ? best_key[slot] : local;
+      }
+      const uint64_t winner = warp_max_u64(local);
+      if (winner != 0ull) {
+#pragma unroll
+        for (int slot = 0; slot < 4; ++slot) {
+          best_key[slot] = best_key[slot] == winner ? 0ull : best_key[slot];
+        }
+      }
+      last_score = key32_to_float(static_cast<uint32_t>(winner >> 32));
+      if (lane == 0) {
+        a.edge_idx[out_base + rank] =
+            winner == 0ull ? -1 : static_cast<int32_t>(0xffffffffu - static_cast<uint32_t>(winner));
+        a.edge_score[out_base + rank] = winner == 0ull ? -INFINITY : last_score;
+      }
     }
   }
   if (lane == 0 && a.edge_flags != nullptr) {
