@@ -269,11 +269,14 @@ def pointer(tensor: torch.Tensor | None) -> int | None:
 
 
 def current_stream(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    """The current stream's handle (without the stream object around it, which takes 2 us to make)."""
+
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 def call(name: str, args: ctypes.Structure, stream: int) -> None:
-    status = getattr(library(), name)(ctypes.byref(args), ctypes.c_void_p(stream))
+    status = getattr(library(), name)(ctypes.byref(args), stream)
     if status != 0:
         message = library().ckv_status_string(status).decode()
         raise NativeError(f"{name} failed with status {status}: {message}")

@@ -674,9 +674,10 @@ def append_kv(
     ``advance``: a shared cursor is also incremented, behind the rows and in the same launch.
     """
 
-    if key_cache.shape != value_cache.shape or new_key.shape != new_value.shape:
+    shape, fresh = key_cache.shape, new_key.shape
+    if shape != value_cache.shape or fresh != new_value.shape:
         raise ValueError("key and value must have the same shapes")
-    if key_cache.shape[-1] != HEAD_DIM or tuple(key_cache.shape[:-2]) != tuple(new_key.shape[:-1]):
+    if shape[-1] != HEAD_DIM or shape[:-2] != fresh[:-1]:
         raise ValueError("caches must be [..., rows, 128] and the new rows [..., 128]")
     if not (key_cache.is_contiguous() and value_cache.is_contiguous()):
         raise ValueError("the caches must be contiguous")
@@ -693,7 +694,7 @@ def append_kv(
         stride = 0 if row.numel() == 1 else 1
         if advance and row.numel() != 1:
             raise ValueError("only a cursor shared by all rows can be advanced")
-    elif not 0 <= int(row) < key_cache.shape[-2]:
+    elif not 0 <= int(row) < shape[-2]:
         raise ValueError("row is outside the cache")
     elif advance:
         raise ValueError("only a device-side cursor can be advanced")
@@ -701,12 +702,12 @@ def append_kv(
     if advance:
         status = native.library().ckv_append_kv_advance(
             key_cache.data_ptr(), value_cache.data_ptr(), keep[0].data_ptr(), keep[1].data_ptr(), units,
-            key_cache.shape[-2] * HEAD_DIM, row.data_ptr(), native.current_stream(device),
+            shape[-2] * HEAD_DIM, row.data_ptr(), native.current_stream(device),
         )
     else:
         status = native.library().ckv_append_kv(
             key_cache.data_ptr(), value_cache.data_ptr(), keep[0].data_ptr(), keep[1].data_ptr(), units,
-            key_cache.shape[-2] * HEAD_DIM, native.pointer(index), stride, 0 if index is not None else int(row),
+            shape[-2] * HEAD_DIM, native.pointer(index), stride, 0 if index is not None else int(row),
             native.current_stream(device),
         )
     if status:

@@ -325,26 +325,25 @@ class DecodeRuntime:
         layer = self.layers.get(layer_idx)
         if layer is None:
             raise RuntimeError(f"decode layer {layer_idx} is not prepared")
-        if query.ndim != 4 or query.shape[0] != 1 or query.shape[2] != 1 or query.shape[3] != HEAD_DIM:
+        shape = query.shape
+        if len(shape) != 4 or shape[0] != 1 or shape[2] != 1 or shape[3] != HEAD_DIM:
             raise ValueError("decode requires query shape [1, Hq, 1, 128]")
         heads = layer.converted.query_heads
-        if query.shape[1] != heads:
-            raise ValueError(f"decode expected {heads} query heads, found {query.shape[1]}")
-        if key.ndim != 4 or key.shape[0] != 1 or value.shape != key.shape:
+        if shape[1] != heads:
+            raise ValueError(f"decode expected {heads} query heads, found {shape[1]}")
+        shape = key.shape
+        if len(shape) != 4 or shape[0] != 1 or value.shape != shape:
             raise ValueError("decode requires key/value shape [1, Hkv, S, 128]")
-        if key.shape[1] != layer.converted.kv_heads:
-            raise ValueError(
-                f"decode expected {layer.converted.kv_heads} KV heads, found {key.shape[1]}"
-            )
-        flat_query = query[0, :, 0, :]
-        if not flat_query.is_contiguous():
-            flat_query = flat_query.contiguous()
+        if shape[1] != layer.converted.kv_heads:
+            raise ValueError(f"decode expected {layer.converted.kv_heads} KV heads, found {shape[1]}")
+        # [Hq, 128] row after row: two of the four extents are one, so this is the query's memory
+        query = query.contiguous()
         # The state and workspaces never move; the packed argument block is
         # rebuilt only when the caller hands in different K/V storage.
         cache_key = (key.data_ptr(), value.data_ptr(), *key.stride(), float(softmax_scale))
         if layer.args is None or layer.cache_key != cache_key:
             layer.args = ops.build_layer_args(
-                query=flat_query,
+                query=query[0, :, 0, :],
                 key=key[0],
                 value=value[0],
                 csr=layer.converted.csr,
@@ -356,18 +355,20 @@ class DecodeRuntime:
                 workspace=layer.workspace,
             )
             layer.cache_key = cache_key
-        layer.args.query = flat_query.data_ptr()
+        layer.args.query = query.data_ptr()
+        pending = layer.update_done
         if self.config.online_assignment == "nearest_centroid":
-            self._nearest_centroid(layer, key[0])
+            self._nearest_centroid(layer)
+            pending = None  # waited for there, on the same stream
         if self.defer_update:
             if self._deferred is None:
                 self._deferred = ops.DeferredUpdate(query.device)
-            layer.update_done = self._deferred.launch(layer.args, pending=layer.update_done)
+            layer.update_done = self._deferred.launch(layer.args, pending=pending)
         else:
             native.call("ckv_decode_layer", layer.args, native.current_stream(query.device))
         return layer.workspace.attention.output.view(1, 1, heads, HEAD_DIM)
 
-    def _nearest_centroid(self, layer: DecodeLayerState, key: torch.Tensor) -> None:
+    def _nearest_centroid(self, layer: DecodeLayerState) -> None:
         """The variant of the online assignment that is not in the reference: the token joins
         the live community whose centroid has the largest inner product with its key.
 
@@ -387,9 +388,7 @@ class DecodeRuntime:
             # the previous step's deferred update still reads `forced`
             torch.cuda.current_stream(device).wait_event(layer.update_done)
         status = native.library().ckv_nearest_centroid(
-            ctypes.byref(layer.args), ctypes.c_void_p(layer.forced.data_ptr()),
-            ctypes.c_void_p(native.current_stream(device)),
-        )
+            ctypes.byref(layer.args), layer.forced.data_ptr(), native.current_stream(device))
         if status:
             raise native.NativeError(native.library().ckv_status_string(status).decode())
 
