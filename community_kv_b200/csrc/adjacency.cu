@@ -29,10 +29,12 @@
 // What bounds a pass now is not the traffic (16 bytes an item, 28 us of 11.5 M items at the copy
 // rate; DRAM is busy 15-20 %) but the latency of its chain - shared-memory atomics of the ranking,
 // look-back, staging - with 24 warps per SM: long_scoreboard and short_scoreboard lead the stalls.
-// Eighty registers for three blocks per SM are too few for sixteen 4-byte items: the pass spills
-// 324 bytes of stores and 392 of loads per thread (the first pass 108-168 and 108-112), which stay
-// in L1.
-// 32 graphs of 8192 positions, 11.5 M raw edges: 0.61 ms (105-115 us a pass, 85 us the runs);
+// Three blocks per SM leave a thread eighty registers.  A tile's items therefore take their places in
+// shared memory before the look-back, which then holds only counts, and ranks are kept as halves:
+// with the items held across the look-back the 4-byte pass spilled 324 bytes of stores and 392 of
+// loads per thread, now 8 (the first pass none, 36 where the neighbours per row are not eight).  Of a layer of 32
+// graphs of 8192 positions, 11.5 M raw edges, from its neighbours to its decode state: 1680 -> 1586 us
+// (halves alone 1651).  The sort takes a good half millisecond of it;
 // five passes over enumerated 12-byte items with separate count and scan kernels took 1.1 ms.
 
 #include <cuda_runtime.h>
@@ -345,7 +347,7 @@ __global__ void __launch_bounds__(kSortThreads, 3)
       }
     }
 
-    uint32_t rank[kItems];
+    uint32_t rank[kItems / 2];  // of two items, below 32 kItems each
 #pragma unroll
     for (int i = 0; i < kItems; ++i) {
       const bool here = kFull || ((live >> i) & 1u);
@@ -361,14 +363,14 @@ __global__ void __launch_bounds__(kSortThreads, 3)
         my_lanes[digit] = 0u;
       }
       __syncwarp();
-      rank[i] = before + below;
+      rank[i / 2] = (i & 1) ? rank[i / 2] | ((before + below) << 16) : before + below;
     }
     __syncthreads();
 
     // thread d looks after digit d
+    const int d = threadIdx.x;
+    uint32_t count = 0u, start, total;
     {
-      const int d = threadIdx.x;
-      uint32_t count = 0u;
 #pragma unroll
       for (int w = 0; w < kSortWarps; ++w) count += warp_count[w][d];
       publish(words + static_cast<uint64_t>(tile) * kDigits + d, (tile == 0 ? kComplete : kPartial) | count);
@@ -378,8 +380,7 @@ __global__ void __launch_bounds__(kSortThreads, 3)
           if (kFull || ((live >> i) & 1u)) weight[i] = weights[item0 + i * 32];
         }
       }
-      uint32_t total;
-      const uint32_t start = block_prefix(count, warp_total, &total);
+      start = block_prefix(count, warp_total, &total);
       uint32_t running = start;  // counts become places in the tile
 #pragma unroll
       for (int w = 0; w < kSortWarps; ++w) {
@@ -387,21 +388,25 @@ __global__ void __launch_bounds__(kSortThreads, 3)
         warp_count[w][d] = running;
         running += c;
       }
+    }
+    __syncthreads();
+    // the items take their places in the tile first: nothing but the counts is then held in
+    // registers across the look-back, whose predecessors gain the time
+#pragma unroll
+    for (int i = 0; i < kItems; ++i) {
+      if (kFull || ((live >> i) & 1u)) {
+        const uint32_t slot = my_count[digit_of(key[i], pass)] + ((i & 1) ? rank[i / 2] >> 16 : rank[i / 2] & 0xffffu);
+        stage.out.key[slot] = key[i];
+        stage.out.weight[slot] = weight[i];
+      }
+    }
+    {
       const uint32_t ahead = look_back(words + d, tile, kDigits, polls, fault);
       if (tile > 0) {
         publish(words + static_cast<uint64_t>(tile) * kDigits + d, kComplete | (static_cast<uint64_t>(ahead) + count));
       }
       target_base[d] = digit_base[d] + ahead - start;
       if (d == 0) tile_s = total;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < kItems; ++i) {
-      if (kFull || ((live >> i) & 1u)) {
-        const uint32_t slot = my_count[digit_of(key[i], pass)] + rank[i];
-        stage.out.key[slot] = key[i];
-        stage.out.weight[slot] = weight[i];
-      }
     }
     __syncthreads();
     const uint32_t here = kFull ? kTile : tile_s;
