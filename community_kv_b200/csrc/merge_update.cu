@@ -4,7 +4,8 @@
 // warps merges the split partials of one query head at a time with independent
 // 16-byte loads.  The fifth warp of the CTA whose head leads its graph merges the per-split
 // neighbour candidates into the global top-8, applies the modularity-gain rule
-// and updates the graph state in place; it is the single writer of that graph.
+// and updates the graph state in place; it is the single writer of that graph.  Where several
+// heads share the graph the same CTA then updates the other heads' tables.
 
 #include "merge_update.cuh"
 
