@@ -92,7 +92,8 @@ __global__ void __launch_bounds__(kScoreThreads, 2) score_kernel(const ckv_layer
 // fp32 centroid table (CKV_FLAG_FP32_CENTROIDS).  Eight lanes share one centroid row, 16
 // dimensions each; every product and every sum is rounded on its own (multiply, then add),
 // in the order of the e4m3 path - 16 sequential terms per lane, then lanes (j, j^4),
-// (j, j^2), (j, j^1) - so that a CPU reproduces the fp16 score bit for bit.
+// (j, j^2), (j, j^1) - so that a CPU reproduces the fp16 score bit for bit.  A launch's latency long
+// where the table is small, so it is launched under the kernel before it and lets the selection start.
 constexpr int kScoreFp32Threads = 256;
 
 __global__ void __launch_bounds__(kScoreFp32Threads) score_fp32_kernel(const ckv_layer_args a) {
@@ -101,6 +102,8 @@ __global__ void __launch_bounds__(kScoreFp32Threads) score_fp32_kernel(const ckv
   const int limit = score_limit(a, flat);
   const int row = blockIdx.x * (kScoreFp32Threads / 8) + (threadIdx.x >> 3);
   const int slice = threadIdx.x & 7;
+  pdl_release_dependents();
+  pdl_wait_for_predecessor();  // the query and last step's centroids come from upstream
   const int safe_row = min(row, capacity - 1);  // every lane takes part in the shuffles below
   const float4* source = reinterpret_cast<const float4*>(
       reinterpret_cast<const float*>(a.centroids) +
@@ -180,8 +183,7 @@ cudaError_t launch_score(const ckv_layer_args& a, cudaStream_t stream) {
   const int units = a.batch * a.retrieval_heads;
   if (a.flags & CKV_FLAG_FP32_CENTROIDS) {
     const dim3 grid((a.community_capacity + kScoreFp32Threads / 8 - 1) / (kScoreFp32Threads / 8), units);
-    score_fp32_kernel<<<grid, kScoreFp32Threads, 0, stream>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(score_fp32_kernel, grid, dim3(kScoreFp32Threads), 0, stream, a);
   }
   if (units > kScoreMaxUnits) {
     return cudaErrorInvalidConfiguration;

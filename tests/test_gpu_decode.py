@@ -578,6 +578,16 @@ def test_shared_graph_in_two_launches(monkeypatch, kv_heads, group, fp32, deferr
         assert torch.equal(first.contiguous().view(torch.uint8), second.contiguous().view(torch.uint8))
 
 
+@pytest.mark.parametrize("communities", [5, 32, 33, 992, 1025])
+def test_selection_over_few_communities(monkeypatch, communities):
+    """The stand-alone selection keeps a histogram per warp that has a community: one, some and all of the 32 warps."""
+
+    monkeypatch.setenv("CKV_UNFUSED", "1")
+    layer = make_layer(seed=60 + communities, seq_len=8192, communities=communities, kv_heads=2, max_decode_tokens=6)
+    config = CommunityKVConfig(token_budget=512, num_sink=10, lam=0.5, aggregation="query_group")
+    _run_sequence(layer, config, steps=3, seed=6100)
+
+
 def test_full_size_batch_one_launch_equals_four_kernels():
     """The batched long-context configuration as far as one layer goes (8 sequences x 8 KV heads at ctx 131072,
     1024-4096 Zipf communities, budget 2048): the single cluster launch and the four
