@@ -225,6 +225,7 @@ def library() -> ctypes.CDLL:
         "ckv_decode_layer",
         "ckv_segmented_attention_static",
         "ckv_online_update",
+        "ckv_merge_partials",
     ):
         function = getattr(lib, name)
         function.restype = ctypes.c_int

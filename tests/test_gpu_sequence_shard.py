@@ -65,6 +65,37 @@ def test_four_shards_match_the_unsharded_layer(aggregation):
             assert torch.equal(shard.converted.current_position.cpu(), twin.current), where
 
 
+@pytest.mark.parametrize("aggregation", ["query_group", "layer_wise"])
+def test_shards_on_a_stream_of_their_own(aggregation):
+    """Every launch of a step goes to the current stream, whose handle is a full pointer: same bits as on the default."""
+
+    device = torch.device("cuda", 0)
+    config = CommunityKVConfig(token_budget=512, num_sink=10, lam=0.5, aggregation=aggregation)
+    layer = make_layer(seed=61, kv_heads=2, seq_len=4096, communities=100, max_decode_tokens=4, aggregation=aggregation)
+    total_rows = layer.key.shape[1]
+    results = []
+    for stream in (torch.cuda.default_stream(device), torch.cuda.Stream(device)):
+        with torch.cuda.stream(stream):
+            shards = []
+            for rank in range(2):
+                begin, end = ckv_dist.sequence_shard(total_rows, 2, rank)
+                shards.append(SequenceShardedLayer(
+                    converted=convert_prefill_tensors(**layer.to(device).prepare_kwargs()),
+                    key_shard=layer.key[:, begin:end].contiguous().to(device),
+                    value_shard=layer.value[:, begin:end].contiguous().to(device),
+                    row_begin=begin, total_rows=total_rows, config=config))
+            outputs = []
+            for step in range(3):
+                current = int(shards[0].converted.current_position[0])
+                outputs.append(decode_emulated(shards, make_query(seed=1100 + step, query_heads=8).to(device),
+                                               layer.key[:, current].to(device), SCALE).clone())
+            state = [tensor.clone() for shard in shards for tensor in shard.converted.mutable.tensors()]
+        stream.synchronize()
+        results.append([*outputs, *state])
+    for first, second in zip(*results):
+        assert torch.equal(first.contiguous().view(torch.uint8), second.contiguous().view(torch.uint8))
+
+
 def test_large_context_shards_agree_with_one_gpu():
     """The sequence-sharded stress configuration (scaled to 262144 tokens so that two replicas fit comfortably):
     16384 planted clusters per head, budget 8192.  Two row shards against the whole cache in one

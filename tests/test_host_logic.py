@@ -285,6 +285,21 @@ def test_library_exports_every_declared_symbol():
     assert lib.ckv_attention_smem_bytes(4) > 60_000
 
 
+def test_every_entry_point_declares_its_arguments():
+    """Without ``argtypes`` ctypes passes an integer as a 32-bit int: a stream handle would lose its upper half."""
+
+    header = re.sub(r"/\*.*?\*/", "", (ROOT / "include" / "ckv_b200.h").read_text(), flags=re.S)
+    declared = re.findall(r"^(?:int|int64_t|const char\*)\s+(ckv_\w+)\s*\(([^)]*)\)\s*;", header, flags=re.M)
+    assert {name for name, _ in declared} == set(native.ENTRY_POINTS)
+    lib = native.library()
+    for name, parameters in declared:
+        parameters = [] if parameters.strip() == "void" else parameters.split(",")
+        types = getattr(lib, name).argtypes or []
+        assert len(types) == len(parameters), name
+        for kind, parameter in zip(types, parameters):
+            assert not ("*" in parameter and kind in (ctypes.c_int, ctypes.c_int32, ctypes.c_uint32)), (name, parameter)
+
+
 def test_ctypes_struct_matches_the_header(tmp_path):
     source = tmp_path / "layout.c"
     fields = [name for name, _ in native.LayerArgs._fields_]
