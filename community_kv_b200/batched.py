@@ -240,6 +240,8 @@ class BatchedDecodeRuntime:
                 workspace=layer.workspace,
             )
             layer.cache_key = cache_key
+        if not query.is_cuda:  # a block that is already there does not look at the tensors again
+            raise ValueError("batched decode requires a CUDA query")
         layer.args.query = query.data_ptr()
         return layer.args
 

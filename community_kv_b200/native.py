@@ -272,6 +272,8 @@ def pointer(tensor: torch.Tensor | None) -> int | None:
 def current_stream(device: torch.device) -> int:
     """The current stream's handle (without the stream object around it, which takes 2 us to make)."""
 
+    if device.type != "cuda":
+        raise ValueError(f"expected a CUDA device, found {device}")
     index = device.index
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 

@@ -355,6 +355,8 @@ class DecodeRuntime:
                 workspace=layer.workspace,
             )
             layer.cache_key = cache_key
+        if not query.is_cuda:  # a block that is already there does not look at the tensors again
+            raise ValueError("decode requires a CUDA query")
         layer.args.query = query.data_ptr()
         pending = layer.update_done
         if self.config.online_assignment == "nearest_centroid":

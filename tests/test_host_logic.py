@@ -14,7 +14,7 @@ import torch
 import community_kv_b200 as ckv
 from community_kv_b200 import native, ops
 from community_kv_b200.assembly import aggregation_mappings, build_member_csr, compute_centroids
-from community_kv_b200.batched import stack_sequences
+from community_kv_b200.batched import BatchedDecodeRuntime, stack_sequences
 from community_kv_b200.config import CommunityKVConfig, GraphAggregation, PartitionConfig
 from community_kv_b200.runtime import (
     CommunityKVRuntime,
@@ -270,6 +270,70 @@ def test_batched_stack_pads_and_views():
         assert int(current[0]) == 512
         mutable.community_counts[0] += 1          # a view: writes land in the stacked tensor
         assert int(state.mutable.community_counts[b, 0]) == converted[b].initial_community_counts[0] + 1
+
+
+class _NoLibrary:
+    """In place of the CUDA library: keeps the names of the entry points that a call reached."""
+
+    def __init__(self):
+        self.launched = []
+
+    def __getattr__(self, name):
+        return lambda *args: self.launched.append(name) or 0
+
+
+class _NoStream:
+    """In place of the deferred update's stream and events."""
+
+    cuda_stream = 0
+    device = torch.device("cuda", 0)
+
+    def __init__(self, *args, **kwargs):
+        pass
+
+    def record(self, stream=None):
+        pass
+
+    def wait_event(self, event):
+        pass
+
+    def synchronize(self):
+        pass
+
+
+@pytest.mark.parametrize("deferred", [False, True])
+@pytest.mark.parametrize("batched,assignment", [(False, "modularity"), (False, "nearest_centroid"), (True, "modularity")])
+def test_a_host_query_never_reaches_a_launch(monkeypatch, batched, deferred, assignment):
+    """Also not where the argument block is already there, as from the second call with the same K/V on."""
+
+    config = CommunityKVConfig(token_budget=128, num_sink=4, aggregation="query_group", online_assignment=assignment)
+    layer = make_layer(seed=8, kv_heads=2, seq_len=512, communities=12, max_decode_tokens=6)
+    if batched:
+        runtime = BatchedDecodeRuntime(config, defer_update=deferred)
+        state = runtime.prepare_layer(0, [convert_prefill_tensors(**layer.prepare_kwargs())])
+        query = torch.zeros(1, 8, 128, dtype=torch.bfloat16)
+    else:
+        runtime = DecodeRuntime(config, defer_update=deferred)
+        state = runtime.prepare_layer(0, **layer.prepare_kwargs())
+        query = torch.zeros(1, 8, 1, 128, dtype=torch.bfloat16)
+    key, value = layer.key[None], layer.value[None]
+    found = _NoLibrary()
+    monkeypatch.setattr(native, "library", lambda: found)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda index: 0, raising=False)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: _NoStream())
+    monkeypatch.setattr(torch.cuda, "Stream", _NoStream)
+    monkeypatch.setattr(torch.cuda, "Event", _NoStream)
+    call = dict(layer_idx=0, query=query, key=key, value=value, softmax_scale=1.0)
+    with pytest.raises(RuntimeError, match="only on CUDA tensors"):
+        runtime.decode(**call)
+    state.args = native.LayerArgs()
+    state.cache_key = (key.data_ptr(), value.data_ptr(), *key.stride(), 1.0)
+    with pytest.raises(ValueError, match="CUDA"):
+        runtime.decode(**call)
+    assert found.launched == [] and not state.args.query
+    with pytest.raises(ValueError, match="CUDA"):
+        native.current_stream(query.device)
 
 
 # ---- the C ABI surface ---------------------------------------------------------------------
