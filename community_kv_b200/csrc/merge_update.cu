@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kMergeThreads + 32) merge_update_kernel(const 
 // of the layer still running (32 heads: 309 us; one layer of a million tokens: 75 instead of 66 us).
 __global__ void append_kv_kernel(uint4* key_cache, uint4* value_cache, const uint4* new_key, const uint4* new_value,
                                  int64_t units, int64_t unit_stride_vec, const int32_t* row_index,
-                                 int64_t row_index_stride, int64_t row, int32_t* cursor) {
+                                 int64_t row_index_stride, int64_t row, int64_t rows, int32_t* cursor) {
   pdl_wait_for_predecessor();  // the fresh rows and the cursor come from upstream, earlier reads of the row too
   pdl_release_dependents();
   const int lane = threadIdx.x & 31;
@@ -119,7 +119,7 @@ __global__ void append_kv_kernel(uint4* key_cache, uint4* value_cache, const uin
     const uint4 held = fresh[unit * (kHeadDim * 2 / 16) + piece];
     const int64_t target =
         cursor != nullptr ? *cursor : (row_index != nullptr ? row_index[unit * row_index_stride] : row);
-    if (target >= 0) {
+    if (target >= 0 && target < rows) {
       cache[unit * unit_stride_vec + target * (kHeadDim * 2 / 16) + piece] = held;
     }
   }
@@ -134,6 +134,8 @@ __global__ void append_kv_kernel(uint4* key_cache, uint4* value_cache, const uin
 cudaError_t launch_append_kv(void* key_cache, void* value_cache, const void* new_key, const void* new_value,
                              int64_t units, int64_t unit_stride, const int32_t* row_index,
                              int64_t row_index_stride, int64_t row, int32_t* cursor, cudaStream_t stream) {
+  // a row that only the device knows may lie behind the unit's last; the caller has seen any other
+  const int64_t rows = cursor != nullptr || row_index != nullptr ? unit_stride / kHeadDim : row + 1;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(cursor != nullptr ? 1u : static_cast<unsigned>((units + 3) / 4));
   config.blockDim = dim3(cursor != nullptr && units > 4 ? 32u * static_cast<unsigned>(units < 32 ? units : 32) : 128u);
@@ -146,7 +148,7 @@ cudaError_t launch_append_kv(void* key_cache, void* value_cache, const void* new
   return cudaLaunchKernelEx(&config, append_kv_kernel, static_cast<uint4*>(key_cache),
                             static_cast<uint4*>(value_cache), static_cast<const uint4*>(new_key),
                             static_cast<const uint4*>(new_value), units, unit_stride / 8, row_index, row_index_stride,
-                            row, cursor);
+                            row, rows, cursor);
 }
 
 // One thread polls this GPU's counter a bounded number of times.

@@ -670,8 +670,10 @@ def append_kv(
     The caches are bf16 ``[..., rows, 128]`` (contiguous), the new rows bf16 ``[..., 128]``
     with the same leading shape; ``row`` is one index for all of them, an int32 tensor
     with one element (a device-side cursor shared by all of them, read by the kernel: no
-    host round trip), or an int32 tensor with one index per leading entry (negative: skip).
-    ``advance``: a shared cursor is also incremented, behind the rows and in the same launch.
+    host round trip), or an int32 tensor with one index per leading entry.  An index on the
+    device that lies outside the cache writes nothing.
+    ``advance``: a shared cursor is also incremented, behind the rows and in the same launch;
+    it runs on behind the last row.
     """
 
     shape, fresh = key_cache.shape, new_key.shape

@@ -290,15 +290,16 @@ int ckv_decode_layer(const ckv_layer_args* args, void* cuda_stream);
  * elements between units and the new rows are contiguous bf16 [units, 128].  The row
  * is `row_index[u * row_index_stride]` when row_index is given (int32, device;
  * stride 0: one device-side cursor shared by all units, stride 1: one row per unit;
- * a negative row skips the unit) and `row` otherwise.  One small launch instead of the
+ * a row outside [0, unit_stride / 128) skips the unit) and `row` otherwise.  One small launch instead of the
  * arange + two index_copy_ calls of the reference's cache layer
  * (community_kv/attention/cache.py:39-47). */
 int ckv_append_kv(void* key_cache, void* value_cache, const void* new_key, const void* new_value,
                   int64_t units, int64_t unit_stride, const int32_t* row_index,
                   int64_t row_index_stride, int64_t row, void* cuda_stream);
 
-/* The same with one device-side cursor shared by all units (int32[1], the row to write;
- * negative: nothing is written), which is incremented behind the rows, in the same launch. */
+/* The same with one device-side cursor shared by all units (int32[1], the row to write; outside
+ * [0, unit_stride / 128) nothing is written), which is incremented behind the rows, in the same
+ * launch.  It runs on behind the last row, so that a reader sees how many tokens came. */
 int ckv_append_kv_advance(void* key_cache, void* value_cache, const void* new_key, const void* new_value,
                           int64_t units, int64_t unit_stride, int32_t* cursor, void* cuda_stream);
 

@@ -540,6 +540,31 @@ def test_append_kv_moves_the_cursor(units):
         ops.append_kv(key[:4], value[:4], new_key[:4], new_value[:4], cursor.repeat(4), advance=True)
 
 
+@pytest.mark.parametrize("units", [1, 3, 40])
+def test_append_kv_past_the_last_row(units):
+    """A row that only the device knows and that lies outside the cache writes nothing: not into the next head's rows,
+    not behind the last head's.  The caches lie inside larger buffers that must stay as they were."""
+
+    device = torch.device("cuda", 0)
+    rows = 9
+    torch.manual_seed(units)
+    buffers = [torch.randn((units + 2, rows, 128), device=device).to(torch.bfloat16) for _ in range(2)]
+    key, value = (buffer[1:-1] for buffer in buffers)
+    want = [buffer.clone() for buffer in buffers]
+    new = [torch.randn((units, 128), device=device).to(torch.bfloat16) for _ in range(2)]
+    cursor = torch.tensor([rows - 1], dtype=torch.int32, device=device)
+    for _ in range(3):
+        ops.append_kv(key, value, *new, cursor, advance=True)
+    for buffer, row in zip(want, new):
+        buffer[1:-1, rows - 1] = row
+    assert int(cursor) == rows + 2
+    assert all(torch.equal(buffer, expected) for buffer, expected in zip(buffers, want))
+    for outside in (rows, rows + 1, -1):
+        ops.append_kv(key, value, *new, torch.full((1,), outside, dtype=torch.int32, device=device))
+        ops.append_kv(key, value, *new, torch.full((units,), outside, dtype=torch.int32, device=device))
+    assert all(torch.equal(buffer, expected) for buffer, expected in zip(buffers, want))
+
+
 @pytest.mark.parametrize("kv_heads,group,fp32,deferred", [(2, 4, False, False), (5, 2, False, True), (9, 1, False, False),
                                                           (6, 2, True, False)])
 def test_shared_graph_in_two_launches(monkeypatch, kv_heads, group, fp32, deferred):
