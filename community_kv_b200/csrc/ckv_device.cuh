@@ -164,9 +164,9 @@ __device__ __forceinline__ void pdl_wait_for_predecessor() {
 }
 
 // Host side: launch with the programmatic-serialisation attribute.
-template <typename Kernel>
+template <typename Kernel, typename... Args>
 inline cudaError_t launch_dependent(Kernel kernel, dim3 grid, dim3 block, size_t smem,
-                                    cudaStream_t stream, const ckv_layer_args& a) {
+                                    cudaStream_t stream, const Args&... args) {
   cudaLaunchConfig_t config = {};
   config.gridDim = grid;
   config.blockDim = block;
@@ -177,7 +177,7 @@ inline cudaError_t launch_dependent(Kernel kernel, dim3 grid, dim3 block, size_t
   attribute[0].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attribute;
   config.numAttrs = 1;
-  return cudaLaunchKernelEx(&config, kernel, a);
+  return cudaLaunchKernelEx(&config, kernel, args...);
 }
 
 // 16-byte asynchronous global -> shared copy (L2 only); src_bytes 0 zero-fills.

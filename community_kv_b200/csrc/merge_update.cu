@@ -99,7 +99,8 @@ __global__ void __launch_bounds__(kMergeThreads + 32) merge_update_kernel(const 
 // One warp per unit and pass: lanes 0-15 copy the 256-byte key row, lanes 16-31 the value row.
 // Bound by launches and latency (a few kilobytes move), so it is launched early under the kernel
 // before it, and with `cursor` it also moves the shared cursor on, which was a launch of its own: one
-// CTA then does all the units, so that every row is placed before the cursor changes.  Six layers of
+// CTA then does all the units, so that every row is placed before the cursor changes.  That holds up to
+// kOneCtaUnits units; more take the rows and the cursor in two launches.  Six layers of
 // 32 heads, budget 4096, a token through the plug-in: 328 -> 292 us; of 8 heads, budget 2048: 245 ->
 // 214 us; the launch early alone, four layers of 3 sequences: 138 -> 128 us.  Dependents are
 // released behind the wait: released in front of it, the next layer's clusters settle between those
@@ -131,24 +132,30 @@ __global__ void append_kv_kernel(uint4* key_cache, uint4* value_cache, const uin
   }
 }
 
+// Us a call in a captured graph, one CTA for rows and cursor / two launches: 8 units 1.6, 64 2.4,
+// 128 3.1, 256 4.6 / 2.2, 512 7.3 / 2.4, 4096 45 / 3.1.  The second launch costs the host 2 us.
+constexpr int64_t kOneCtaUnits = 128;
+
 cudaError_t launch_append_kv(void* key_cache, void* value_cache, const void* new_key, const void* new_value,
                              int64_t units, int64_t unit_stride, const int32_t* row_index,
                              int64_t row_index_stride, int64_t row, int32_t* cursor, cudaStream_t stream) {
   // a row that only the device knows may lie behind the unit's last; the caller has seen any other
   const int64_t rows = cursor != nullptr || row_index != nullptr ? unit_stride / kHeadDim : row + 1;
-  cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(cursor != nullptr ? 1u : static_cast<unsigned>((units + 3) / 4));
-  config.blockDim = dim3(cursor != nullptr && units > 4 ? 32u * static_cast<unsigned>(units < 32 ? units : 32) : 128u);
-  config.stream = stream;
-  cudaLaunchAttribute attribute[1];
-  attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attribute[0].val.programmaticStreamSerializationAllowed = 1;
-  config.attrs = attribute;
-  config.numAttrs = 1;
-  return cudaLaunchKernelEx(&config, append_kv_kernel, static_cast<uint4*>(key_cache),
+  auto run = [&](unsigned ctas, unsigned warps, int64_t count, const int32_t* index, int32_t* moved) {
+    return launch_dependent(append_kv_kernel, dim3(ctas), dim3(32u * warps), 0, stream, static_cast<uint4*>(key_cache),
                             static_cast<uint4*>(value_cache), static_cast<const uint4*>(new_key),
-                            static_cast<const uint4*>(new_value), units, unit_stride / 8, row_index, row_index_stride,
-                            row, rows, cursor);
+                            static_cast<const uint4*>(new_value), count, unit_stride / 8, index, row_index_stride, row,
+                            rows, moved);
+  };
+  const unsigned ctas = static_cast<unsigned>((units + 3) / 4);
+  if (cursor == nullptr) {
+    return run(ctas, 4u, units, row_index, nullptr);
+  }
+  if (units <= kOneCtaUnits) {
+    return run(1u, units < 4 ? 4u : static_cast<unsigned>(units < 32 ? units : 32), units, nullptr, cursor);
+  }
+  const cudaError_t err = run(ctas, 4u, units, cursor, nullptr);
+  return err == cudaSuccess ? run(1u, 1u, 0, nullptr, cursor) : err;
 }
 
 // One thread polls this GPU's counter a bounded number of times.

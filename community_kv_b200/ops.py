@@ -672,8 +672,8 @@ def append_kv(
     with one element (a device-side cursor shared by all of them, read by the kernel: no
     host round trip), or an int32 tensor with one index per leading entry.  An index on the
     device that lies outside the cache writes nothing.
-    ``advance``: a shared cursor is also incremented, behind the rows and in the same launch;
-    it runs on behind the last row.
+    ``advance``: a shared cursor is also incremented, behind the rows (and, up to 128 of
+    them, in the same launch); it runs on behind the last row.
     """
 
     shape, fresh = key_cache.shape, new_key.shape

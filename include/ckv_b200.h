@@ -298,8 +298,9 @@ int ckv_append_kv(void* key_cache, void* value_cache, const void* new_key, const
                   int64_t row_index_stride, int64_t row, void* cuda_stream);
 
 /* The same with one device-side cursor shared by all units (int32[1], the row to write; outside
- * [0, unit_stride / 128) nothing is written), which is incremented behind the rows, in the same
- * launch.  It runs on behind the last row, so that a reader sees how many tokens came. */
+ * [0, unit_stride / 128) nothing is written), which is incremented behind the rows: in the same
+ * launch up to 128 units, in a second one from there on.  It runs on behind the last row, so that a
+ * reader sees how many tokens came. */
 int ckv_append_kv_advance(void* key_cache, void* value_cache, const void* new_key, const void* new_value,
                           int64_t units, int64_t unit_stride, int32_t* cursor, void* cuda_stream);
 

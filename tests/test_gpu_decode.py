@@ -540,6 +540,61 @@ def test_append_kv_moves_the_cursor(units):
         ops.append_kv(key[:4], value[:4], new_key[:4], new_value[:4], cursor.repeat(4), advance=True)
 
 
+@pytest.mark.parametrize("units", [128, 129, 700])
+def test_append_kv_moves_the_cursor_behind_many_rows(units):
+    """On both sides of the line between one CTA for rows and cursor, and two launches; also replayed from a graph."""
+
+    device = torch.device("cuda", 0)
+    torch.manual_seed(units)
+    key = torch.randn((units, 9, 128), device=device).to(torch.bfloat16)
+    value = torch.randn_like(key)
+    new = [torch.randn((units, 128), device=device).to(torch.bfloat16) for _ in range(2)]
+    want = [key.clone(), value.clone()]
+    cursor = torch.tensor([5], dtype=torch.int32, device=device)
+    ops.append_kv(key, value, *new, cursor, advance=True)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ops.append_kv(key, value, *new, cursor, advance=True)
+    for row in (5, 6, 7):
+        if row > 5:
+            for tensor in new:
+                tensor.copy_(torch.randn_like(tensor))
+            graph.replay()
+        want[0][:, row], want[1][:, row] = new
+    assert int(cursor) == 8
+    assert torch.equal(key, want[0]) and torch.equal(value, want[1])
+
+
+def test_append_kv_of_many_rows_uses_the_chip():
+    """A cursor that moves does not leave 4096 rows to one CTA (25 times as long as over the chip)."""
+
+    device = torch.device("cuda", 0)
+    key = torch.zeros((4096, 130, 128), dtype=torch.bfloat16, device=device)
+    value = torch.zeros_like(key)
+    new = [torch.ones((4096, 128), dtype=torch.bfloat16, device=device) for _ in range(2)]
+    cursor = torch.zeros(1, dtype=torch.int32, device=device)
+
+    def microseconds(advance):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            cursor.zero_()
+            for _ in range(100):
+                ops.append_kv(key, value, *new, cursor, advance=advance)
+        spans = []
+        for _ in range(5):
+            begin, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            torch.cuda.synchronize()
+            begin.record()
+            graph.replay()
+            end.record()
+            end.synchronize()
+            spans.append(begin.elapsed_time(end) * 10)
+        return min(spans)
+
+    ops.append_kv(key, value, *new, cursor)
+    assert microseconds(True) < 4 * microseconds(False) + 5
+
+
 @pytest.mark.parametrize("units", [1, 3, 40])
 def test_append_kv_past_the_last_row(units):
     """A row that only the device knows and that lies outside the cache writes nothing: not into the next head's rows,
