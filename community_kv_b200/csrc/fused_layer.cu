@@ -25,7 +25,7 @@
 // device functions run in the same order on the same data.  The path needs per-CTA
 // community slices that fit the selection's shared-memory stash.  A graph shared by several
 // retrieval heads is updated by its leader while followers may still be reading it, which only a
-// kernel boundary orders: step 4 then ends with the outputs, and the update is a second launch.
+// kernel boundary orders: step 4 is then a second launch, the merge kernel of the stand-alone path.
 
 #include <atomic>
 
@@ -126,6 +126,9 @@ __global__ void __launch_bounds__(kFusedThreads, 3) decode_cluster_kernel(const 
     attention_split<kBlocks>(a, flat, rank, smem);
   }
   phase_stamp(a, flat, rank, 7);
+  if (a.flags & CKV_FLAG_ATTENTION_ONLY) {
+    return;  // the launch behind this one merges; nothing reads another CTA's shared memory any more
+  }
   cluster_arrive();  // release at cluster scope: the partials above are visible to rank 0
   if (rank != 0) {
     return;
@@ -243,6 +246,20 @@ int wide_ctas(const ckv_layer_args& a) {
 
 }  // namespace
 
+// Graphs shared by several heads take two launches, merge and update in the second.  Beside four they
+// save the host two launches and win with more than eight splits; up to eight the scores of few
+// communities are faster over the whole chip, and from about one cluster CTA per SM on the merge's CTAs
+// find their place late.  One graph for all heads, a row appended and a layer decoded, us in a captured
+// graph (eager), four kernels / two launches:
+//    4 heads, budget 512, 4 splits, 100 communities   26.0 (27.4) / 28.4 (28.9)
+//    4 heads, budget 1024, 8 splits, 1000 communities 32.1 (34.3) / 31.8 (32.3)
+//    8 heads, budget 2048, 8 splits, 2000 communities 35.8 (38.0) / 35.8 (36.7)
+//   12 heads, budget 1024, 8 splits, 500 communities  30.1 (31.7) / 30.8 (31.4)
+//   16 heads, the same                                30.6 (33.0) / 33.3 (33.9)
+//   64 heads, the same in 6 splits                    41.0 (42.7) / 46.7 (49.8)
+//    6 heads, budget 8192, 16 splits, 2000 communities 44.2 (46.9) / 37.8 (39.0)
+constexpr int kSharedCtas = 96;
+
 // CTAs per unit of the one launch; 0: the stand-alone kernels run.
 int fused_layer_ctas(const ckv_layer_args& a) {
   if (a.splits < 1 || a.splits > 2 * kMaxCluster ||
@@ -251,6 +268,10 @@ int fused_layer_ctas(const ckv_layer_args& a) {
   }
   const int ctas = a.splits <= 8 ? a.splits : wide_ctas(a);
   if (ctas == 0) {
+    return 0;
+  }
+  if (a.splits <= 8 && a.graphs != a.retrieval_heads && !(a.flags & CKV_FLAG_SKIP_UPDATE) &&
+      a.batch * a.retrieval_heads * ctas > kSharedCtas) {
     return 0;
   }
   // every CTA stages the rows it scores: a 1/ctas share of the 16-row groups

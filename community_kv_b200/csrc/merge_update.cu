@@ -11,70 +11,74 @@
 
 namespace ckv {
 
+constexpr int kFollowersInFlight = 4;
+constexpr int kUpdateMaxThreads = 512;
+
 // The other heads of a graph shared by several retrieval heads take the leader's assignment over into
-// their own tables.  The CTA that has just updated the graph does it, four heads in flight: what it
-// needs of the decision is still in shared memory, and a launch of its own (2.7 us and the gap in
-// front of it) is saved.  Nothing else of the launch reads those tables.
+// their own tables.  The CTA that has just updated the graph does it: what it needs of the decision is
+// still in shared memory, and a launch of its own (2.7 us and the gap in front of it) is saved.  Nothing
+// else of the launch reads those tables.  Bound by the latency of the rows and the divisions behind
+// them: a warp takes a head and has four in flight (eight were slower: 64 heads 18 instead of 12 us),
+// and launch_merge_update adds warps for more than twenty heads.
 __device__ __forceinline__ void sync_followers(const ckv_layer_args& a, int flat, const UpdateDecision& decision) {
-  constexpr int kInFlight = 4;
+  constexpr int kInFlight = kFollowersInFlight;
+  constexpr int kPieces = kHeadDim / 32;  // dimensions lane, lane + 32, ... of a head
   const Unit u = make_unit(a, flat);
   if (u.head != u.graph || decision.overflow != 0) {
     return;
   }
-  const int d = threadIdx.x;
-  const int capacity = a.community_capacity;
+  const int warps = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31;
   const bool wide = (a.flags & CKV_FLAG_FP32_CENTROIDS) != 0;
   const bool reference_division = (a.flags & CKV_FLAG_REFERENCE_DIVISION) != 0;
-  for (int base = 0; base < a.retrieval_heads; base += kInFlight) {
-    int64_t index[kInFlight];  // of the community in the head's tables, -1: not a follower
+  for (int base = threadIdx.x >> 5; base < a.retrieval_heads; base += warps * kInFlight) {
+    bool follows[kInFlight];
+    int64_t index[kInFlight];  // of the community in the head's tables
     int size[kInFlight];
-    float key_value[kInFlight], old_value[kInFlight];
+    float key_value[kInFlight][kPieces], old_value[kInFlight][kPieces];
 #pragma unroll
     for (int i = 0; i < kInFlight; ++i) {
-      const int head = base + i;
-      index[i] = -1;
-      size[i] = 0;
-      key_value[i] = old_value[i] = 0.f;
-      if (head >= a.retrieval_heads || head == u.head || a.retrieval_to_graph[head] != u.graph) {
-        continue;
-      }
+      const int head = min(base + i * warps, a.retrieval_heads - 1);
       const int other = u.batch * a.retrieval_heads + head;
-      index[i] = static_cast<int64_t>(other) * capacity + decision.assigned;
+      follows[i] = base + i * warps < a.retrieval_heads && head != u.head && a.retrieval_to_graph[head] == u.graph;
+      index[i] = static_cast<int64_t>(other) * a.community_capacity + decision.assigned;
       size[i] = a.community_sizes[index[i]];
-      if (d < kHeadDim) {
-        const __nv_bfloat16* key_row =
-            a.current_key != nullptr
-                ? reinterpret_cast<const __nv_bfloat16*>(a.current_key) + static_cast<int64_t>(other) * kHeadDim
-                : reinterpret_cast<const __nv_bfloat16*>(a.key) + u.batch * a.key_batch_stride +
-                      a.retrieval_to_kv[head] * a.key_head_stride +
-                      static_cast<int64_t>(decision.current) * a.key_row_stride;
-        key_value[i] = __bfloat162float(key_row[d]);
+      const __nv_bfloat16* key_row =
+          a.current_key != nullptr
+              ? reinterpret_cast<const __nv_bfloat16*>(a.current_key) + static_cast<int64_t>(other) * kHeadDim
+              : reinterpret_cast<const __nv_bfloat16*>(a.key) + u.batch * a.key_batch_stride +
+                    a.retrieval_to_kv[head] * a.key_head_stride +
+                    static_cast<int64_t>(decision.current) * a.key_row_stride;
+#pragma unroll
+      for (int k = 0; k < kPieces; ++k) {
+        key_value[i][k] = __bfloat162float(key_row[lane + 32 * k]);
         if (wide) {
-          old_value[i] = reinterpret_cast<const float*>(a.centroids)[index[i] * kHeadDim + d];
+          old_value[i][k] = reinterpret_cast<const float*>(a.centroids)[index[i] * kHeadDim + lane + 32 * k];
         } else {
           const __half_raw raw = __nv_cvt_fp8_to_halfraw(
-              reinterpret_cast<const __nv_fp8_storage_t*>(a.centroids)[index[i] * kHeadDim + d], __NV_E4M3);
-          old_value[i] = __half2float(*reinterpret_cast<const __half*>(&raw));
+              reinterpret_cast<const __nv_fp8_storage_t*>(a.centroids)[index[i] * kHeadDim + lane + 32 * k], __NV_E4M3);
+          old_value[i][k] = __half2float(*reinterpret_cast<const __half*>(&raw));
         }
       }
     }
-    __syncthreads();  // every thread has read the sizes
+    __syncwarp();  // every lane has read the sizes
 #pragma unroll
     for (int i = 0; i < kInFlight; ++i) {
-      if (index[i] < 0) {
+      if (!follows[i]) {
         continue;
       }
-      if (d == 0) {
+      if (lane == 0) {
         a.community_sizes[index[i]] = size[i] + 1;
-        a.community_counts[u.batch * a.retrieval_heads + base + i] = decision.count;
+        a.community_counts[u.batch * a.retrieval_heads + base + i * warps] = decision.count;
       }
-      if (d < kHeadDim) {
-        const float updated =
-            size[i] > 0 ? centroid_mean(old_value[i], size[i], key_value[i], reference_division) : key_value[i];
+#pragma unroll
+      for (int k = 0; k < kPieces; ++k) {
+        const float updated = size[i] > 0 ? centroid_mean(old_value[i][k], size[i], key_value[i][k], reference_division)
+                                          : key_value[i][k];
         if (wide) {
-          reinterpret_cast<float*>(a.centroids)[index[i] * kHeadDim + d] = updated;
+          reinterpret_cast<float*>(a.centroids)[index[i] * kHeadDim + lane + 32 * k] = updated;
         } else {
-          reinterpret_cast<__nv_fp8_storage_t*>(a.centroids)[index[i] * kHeadDim + d] =
+          reinterpret_cast<__nv_fp8_storage_t*>(a.centroids)[index[i] * kHeadDim + lane + 32 * k] =
               __nv_cvt_float_to_fp8(updated, __NV_SATFINITE, __NV_E4M3);
         }
       }
@@ -82,7 +86,7 @@ __device__ __forceinline__ void sync_followers(const ckv_layer_args& a, int flat
   }
 }
 
-__global__ void __launch_bounds__(kMergeThreads + 32) merge_update_kernel(const ckv_layer_args a) {
+__global__ void __launch_bounds__(kUpdateMaxThreads) merge_update_kernel(const ckv_layer_args a) {
   __shared__ UpdateDecision decision;
   __shared__ float lse_s;
   pdl_release_dependents();
@@ -352,9 +356,20 @@ cudaError_t launch_nearest_centroid(const ckv_layer_args& a, int32_t* forced, cu
   return cudaLaunchKernelEx(&config, nearest_centroid_kernel, a, forced);
 }
 
+// Warps beyond the five of the merge only serve the followers of a shared graph.  As many as have all of
+// them in flight, but no more than leave every CTA resident at once (16 warps per SM at this kernel's
+// registers).  One graph for all heads, the update alone in a captured graph, us, a launch of its own for
+// the followers / five warps / so: 16 heads 6.8 / 6.3 / 6.1, 32 heads 7.2 / 8.4 / 6.5, 64 heads
+// 7.2 / 12.3 / 7.2.  A whole CTA per head, four heads in flight, took 15.2, 27 and 51.
 cudaError_t launch_merge_update(const ckv_layer_args& a, cudaStream_t stream) {
-  return launch_dependent(merge_update_kernel, dim3(a.batch * a.retrieval_heads), dim3(kMergeThreads + 32), 0, stream,
-                          a);
+  int warps = kMergeThreads / 32 + 1;
+  const int units = a.batch * a.retrieval_heads;
+  if (a.retrieval_heads != a.graphs && !(a.flags & CKV_FLAG_SKIP_UPDATE)) {
+    const int wanted = (a.retrieval_heads + kFollowersInFlight - 1) / kFollowersInFlight;
+    const int most = min(kUpdateMaxThreads / 32, 148 * (kUpdateMaxThreads / 32) / units);
+    warps = max(warps, min(wanted, most));
+  }
+  return launch_dependent(merge_update_kernel, dim3(units), dim3(32 * warps), 0, stream, a);
 }
 
 }  // namespace ckv

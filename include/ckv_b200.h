@@ -279,8 +279,9 @@ int ckv_segmented_attention(const ckv_layer_args* args, void* cuda_stream);
  * splits and communities that fit the selection's shared-memory stash, this is ONE
  * launch: a thread-block cluster per (sequence, retrieval head) scores, selects,
  * attends, merges and updates, synchronising through cluster barriers (graphs shared
- * by several retrieval heads are updated by a second kernel behind it).  With more splits it is one launch of up to sixteen CTAs
- * per unit where that was measured to be the faster route.  Otherwise (or with
+ * by several retrieval heads are merged and updated by a second kernel behind it, where that
+ * was measured to be the faster route).  With more splits it is one launch of up to sixteen
+ * CTAs per unit where that was.  Otherwise (or with
  * CKV_FLAG_UNFUSED) the four stand-alone kernels run back to back.  Results are
  * identical either way. */
 int ckv_decode_layer(const ckv_layer_args* args, void* cuda_stream);

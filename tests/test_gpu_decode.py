@@ -658,6 +658,54 @@ def test_shared_graph_in_two_launches(monkeypatch, kv_heads, group, fp32, deferr
         assert torch.equal(first.contiguous().view(torch.uint8), second.contiguous().view(torch.uint8))
 
 
+@pytest.mark.parametrize("kv_heads,fp32", [(20, False), (21, True), (45, False), (70, False)])
+def test_followers_of_a_shared_graph_match_the_oracle(kv_heads, fp32):
+    """Heads that share one graph, four to a warp: full warps, a remainder, the most warps and more heads than those
+    take at once.  The followers' centroids, sizes and counts are the oracle's."""
+
+    layer = make_layer(seed=30 + kv_heads, kv_heads=kv_heads, group_size=1, seq_len=1031, communities=24,
+                       max_decode_tokens=5, aggregation="layer_wise")
+    if fp32:
+        layer.assembled.centroids = layer.assembled.centroids.float()
+    config = CommunityKVConfig(token_budget=256, num_sink=3, lam=0.5, aggregation="layer_wise",
+                               centroid_dtype="fp32" if fp32 else "e4m3")
+    _run_sequence(layer, config, steps=4, seed=3000 + kv_heads)
+
+
+def test_many_followers_cost_an_update_little():
+    """The followers of a shared graph are updated side by side: 63 of them (head after head 45 us) do not triple
+    the update's time of three."""
+
+    device = torch.device("cuda", 0)
+    config = CommunityKVConfig(token_budget=256, num_sink=3, lam=0.5, aggregation="layer_wise")
+
+    def microseconds(kv_heads):
+        layer = make_layer(seed=70, kv_heads=kv_heads, group_size=1, seq_len=1031, communities=24,
+                           max_decode_tokens=340, aggregation="layer_wise").to(device)
+        runtime = DecodeRuntime(config)
+        state = runtime.prepare_layer(0, **layer.prepare_kwargs())
+        query = make_query(seed=71, query_heads=kv_heads).to(device)
+        runtime.decode(layer_idx=0, query=query.view(1, kv_heads, 1, 128), key=layer.key[None], value=layer.value[None],
+                       softmax_scale=SCALE)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for _ in range(50):
+                native.call("ckv_online_update", state.args, native.current_stream(device))
+        spans = []
+        for _ in range(6):
+            begin, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            torch.cuda.synchronize()
+            begin.record()
+            graph.replay()
+            end.record()
+            end.synchronize()
+            spans.append(begin.elapsed_time(end) * 20)
+        runtime.assert_no_overflow()
+        return min(spans)
+
+    assert microseconds(64) < 3 * microseconds(4)
+
+
 @pytest.mark.parametrize("communities", [5, 32, 33, 992, 1025])
 def test_selection_over_few_communities(monkeypatch, communities):
     """The stand-alone selection keeps a histogram per warp that has a community: one, some and all of the 32 warps."""
