@@ -190,13 +190,6 @@ __device__ __forceinline__ void sorted_insert(uint32_t (&queue)[kDepth], uint32_
   queue[0] = max(queue[0], candidate);
 }
 
-// Largest of three in one operation
-__device__ __forceinline__ float max3(float a, float b, float c) {
-  float y;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
-  return y;
-}
-
 // Minimum that does not lose a NaN
 __device__ __forceinline__ float min_nan(float a, float b) {
   float y;
@@ -664,15 +657,17 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       float part_max[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        part_max[i] = max3(s[i], s[i + 8], s[i + 16]);
-#pragma unroll
-        for (int c = 24; c < 120; c += 16) {
-          part_max[i] = max3(part_max[i], s[c + i], s[c + i + 8]);
-        }
-        part_max[i] = fmaxf(part_max[i], s[120 + i]);
+        part_max[i] = fmaxf(s[i], s[i + 8]);
       }
-      const float tile_max = max3(max3(part_max[0], part_max[1], part_max[2]),
-                                  max3(part_max[3], part_max[4], part_max[5]), fmaxf(part_max[6], part_max[7]));
+#pragma unroll
+      for (int c = 16; c < 128; c += 16) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          part_max[i] = fmaxf(part_max[i], fmaxf(s[c + i], s[c + i + 8]));
+        }
+      }
+      const float tile_max = fmaxf(fmaxf(fmaxf(part_max[0], part_max[1]), fmaxf(part_max[2], part_max[3])),
+                                   fmaxf(fmaxf(part_max[4], part_max[5]), fmaxf(part_max[6], part_max[7])));
 
       // The running maximum only moves when the new one lies more than 2^8 above it
       // (probabilities up to 256 are harmless in bf16 / fp32); moving it means rescaling
