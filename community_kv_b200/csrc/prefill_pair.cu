@@ -613,247 +613,247 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     first.set(a, blockIdx.x);
     int pos0 = first.pos0;
     for (int n = 0; !failed && pos0 >= 0; ++n) {
-    const int blocks = (pos0 >> 7) + 1;
-    const bool live = pos0 + row < length;
-    float run_max = -INFINITY;  // of the raw (unscaled) scores
-    float run_sum = 0.f;
-    uint32_t q32[4][kLocalK];
-    if constexpr (kMode == 1) {
+      const int blocks = (pos0 >> 7) + 1;
+      const bool live = pos0 + row < length;
+      float run_max = -INFINITY;  // of the raw (unscaled) scores
+      float run_sum = 0.f;
+      uint32_t q32[4][kLocalK];
+      if constexpr (kMode == 1) {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < 4; ++c) {
 #pragma unroll
-        for (int k = 0; k < kLocalK; ++k) {
-          q32[c][k] = 0u;
+          for (int k = 0; k < kLocalK; ++k) {
+            q32[c][k] = 0u;
+          }
         }
       }
-    }
 
-    for (int block = 0; block < blocks; ++block, ++step) {
-      const int key0 = block * kPfKeys;
-      if (!pair_wait_warp(bar_s_full + 8 * t, step & 1, abort)) {
-        failed = true;
-        break;
-      }
-      tc_fence_after();
-      uint32_t raw[4][32];
+      for (int block = 0; block < blocks; ++block, ++step) {
+        const int key0 = block * kPfKeys;
+        if (!pair_wait_warp(bar_s_full + 8 * t, step & 1, abort)) {
+          failed = true;
+          break;
+        }
+        tc_fence_after();
+        uint32_t raw[4][32];
 #pragma unroll
-      for (int part = 0; part < 4; ++part) {
-        tmem_load32_issue(s_addr + part * 32u, raw[part]);
-      }
-      tmem_wait_load();
-      float s[128];
-#pragma unroll
-      for (int c = 0; c < 128; ++c) {
-        s[c] = __uint_as_float(raw[c >> 5][c & 31]);
-      }
-      // only the last block of a tile meets the diagonal: key pos0 + c, row pos0 + row
-      if (block == blocks - 1) {
+        for (int part = 0; part < 4; ++part) {
+          tmem_load32_issue(s_addr + part * 32u, raw[part]);
+        }
+        tmem_wait_load();
+        float s[128];
 #pragma unroll
         for (int c = 0; c < 128; ++c) {
-          s[c] = c <= row ? s[c] : -INFINITY;
+          s[c] = __uint_as_float(raw[c >> 5][c & 31]);
         }
-      }
-      // eight independent chains (the compiler keeps the order of a single one)
-      float part_max[8];
+        // only the last block of a tile meets the diagonal: key pos0 + c, row pos0 + row
+        if (block == blocks - 1) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        part_max[i] = fmaxf(s[i], s[i + 8]);
-      }
-#pragma unroll
-      for (int c = 16; c < 128; c += 16) {
+          for (int c = 0; c < 128; ++c) {
+            s[c] = c <= row ? s[c] : -INFINITY;
+          }
+        }
+        // eight independent chains (the compiler keeps the order of a single one)
+        float part_max[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          part_max[i] = fmaxf(part_max[i], fmaxf(s[c + i], s[c + i + 8]));
+          part_max[i] = fmaxf(s[i], s[i + 8]);
         }
-      }
-      const float tile_max = fmaxf(fmaxf(fmaxf(part_max[0], part_max[1]), fmaxf(part_max[2], part_max[3])),
-                                   fmaxf(fmaxf(part_max[4], part_max[5]), fmaxf(part_max[6], part_max[7])));
-
-      // The running maximum only moves when the new one lies more than 2^8 above it
-      // (probabilities up to 256 are harmless in bf16 / fp32); moving it means rescaling
-      // the row of O in tensor memory, once the product that still adds to it is done.
-      const float new_max = fmaxf(run_max, tile_max);
-      const bool move = new_max > run_max && (new_max - run_max) * scale_log2 > 8.0f;
-      if (__any_sync(0xffffffffu, move)) {
-        float corr = 1.f;
-        if (move) {
-          corr = run_max == -INFINITY ? 0.f : exp2_fast((run_max - new_max) * scale_log2);
-          run_max = new_max;
-          run_sum *= corr;
-        }
-        if (block > 0) {
-          // P.V of the last block is done: this block's S was committed after it.  Rare, so
-          // rolled and in narrow steps, which take few registers beside the row of scores.
-#pragma unroll 1
-          for (int part = 0; part < 8; ++part) {
-            uint32_t o[16];
-            tmem_load16_issue(o_addr + part * 16u, o);
-            tmem_wait_load();
 #pragma unroll
-            for (int c = 0; c < 16; ++c) {
-              o[c] = __float_as_uint(__uint_as_float(o[c]) * corr);
-            }
-            tmem_store16_issue(o_addr + part * 16u, o);
-          }
-        }
-      }
-      // ---- probabilities, bf16 pairs, over the first 64 columns of this S buffer ----
-      const float offset = (run_max == -INFINITY ? 0.f : run_max) * scale_log2;
-      const uint64_t scale_pair = pack_pair(scale_log2, scale_log2);
-      const uint64_t offset_pair = pack_pair(-offset, -offset);
-      uint64_t sum_pair[2] = {0ull, 0ull};
-#pragma unroll
-      for (int quarter = 0; quarter < 4; ++quarter) {
-        uint32_t packed[16];
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          const int c = quarter * 32 + 2 * e;
-          float x0, x1;
-          unpack_pair(fma_pair(pack_pair(s[c], s[c + 1]), scale_pair, offset_pair), x0, x1);
-          const float p0 = exp2_fast(x0);
-          const float p1 = exp2_fast(x1);
-          sum_pair[e & 1] = add_pair(sum_pair[e & 1], pack_pair(p0, p1));
-          packed[e] = pack_bf16(p0, p1);
-        }
-        tmem_store16_issue(s_addr + quarter * 16u, packed);
-      }
-      {
-        float a0, a1, b0, b1;
-        unpack_pair(sum_pair[0], a0, a1);
-        unpack_pair(sum_pair[1], b0, b1);
-        run_sum += (a0 + a1) + (b0 + b1);
-      }
-      tmem_wait_store();
-      tc_fence_before();
-      // one arrival per warp: 128 arrivals on one barrier word queue up behind each other
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(bar_p_full + 8 * t);
-      }
-
-      // The candidate bookkeeping is bound by the ALU and by its rounds of insertion, one at least
-      // in most blocks and classes; the gates keep their number down.  32 query on 8 KV heads,
-      // against a gate from the lists alone, rounds with a branch, and the rows behind the
-      // end taking part: 517 tokens 117 -> 39 us, 6001 tokens 1560 -> 530 us, 16384 tokens
-      // 3250 -> 2620 us (attention alone: 20, 326 and 1820 us).
-      // It runs from the scores still in registers while the tensor cores work on this
-      // tile's P.V and next S: it is off the path between two blocks.
-      if constexpr (kMode == 1) {
-        const int sinks = a.num_sink - key0;  // columns of this block that are no candidates
-        if (sinks > 0) {
-          // the groups' maxima without them: the upper 64 columns, if that is far enough
+        for (int c = 16; c < 128; c += 16) {
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
-            part_max[i] = s[64 + i];
-#pragma unroll
-            for (int c = 72 + i; c < 128; c += 8) {
-              part_max[i] = fmaxf(part_max[i], s[c]);
-            }
+            part_max[i] = fmaxf(part_max[i], fmaxf(s[c + i], s[c + i + 8]));
           }
         }
-        // A key that is below two keys of every class can never reach the output (the class
-        // lists then hold at least eight keys above it), nor one below the top four of two
-        // classes.  Two keys of every class: the second-best entries of the lists, or the
-        // maxima of this block's two column groups of every class.
-        const uint32_t third0 = q32[0][3], third1 = q32[1][3], third2 = q32[2][3], third3 = q32[3][3];
-        const uint32_t second_of_fourths =
-            max(min(max(third0, third1), max(third2, third3)),
-                max(min(third0, third1), min(third2, third3)));
-        const uint32_t row_floor = max(min(min(q32[0][1], q32[1][1]), min(q32[2][1], q32[3][1])),
-                                       second_of_fourths);
-        float block_floor =
-            min_nan(min_nan(min_nan(part_max[0], part_max[1]), min_nan(part_max[2], part_max[3])),
-                    min_nan(min_nan(part_max[4], part_max[5]), min_nan(part_max[6], part_max[7])));
-        block_floor = sinks > 64 ? -INFINITY : block_floor;
-        const uint32_t floor_key = max(row_floor >> 17, quantised_key_fma(block_floor));
-        // smallest raw score whose quantised key can reach the floor, a little low
-        float gate = floor_key == 0u
-                         ? -3.0e38f
-                         : (static_cast<float>(floor_key) - 0.75f) * (1.0f / 256.0f) - 48.0f;
-        // rows behind the end of a ragged prompt score 0 everywhere: ties that all reach the gate
-        gate = live ? gate : INFINITY;
-        // (no vote in front of a class: in most blocks some row of the warp has a taker)
-        take_candidates<0>(s, gate, key0, sinks, q32[0]);
-        take_candidates<1>(s, gate, key0, sinks, q32[1]);
-        take_candidates<2>(s, gate, key0, sinks, q32[2]);
-        take_candidates<3>(s, gate, key0, sinks, q32[3]);
-      }
-    }
+        const float tile_max = fmaxf(fmaxf(fmaxf(part_max[0], part_max[1]), fmaxf(part_max[2], part_max[3])),
+                                     fmaxf(fmaxf(part_max[4], part_max[5]), fmaxf(part_max[6], part_max[7])));
 
-    // the next item under the last product; the ring's slots up to it are visible then
-    if (kMany && !failed && !pair_wait_warp(bar_of(n + 1), parity_of(n + 1), abort)) {
-      failed = true;
-    }
-    if (!failed && !pair_wait_warp(bar_o_full + 8 * t, n & 1, abort)) {
-      failed = true;
-    }
-    if (!failed) {
-      tc_fence_after();
-      // not held in registers through the loop
-      PairItem item;
-      if constexpr (kMany) {
-        item = read_item(slot_of(n));
-      } else {
-        uint32_t again = blockIdx.x;
-        asm volatile("" : "+r"(again));
-        item.set(a, again);
-      }
-      const int row_pos = item.pos0 + row;
-      const int row_head = item.head0 + t;
-      const bool row_live = row_pos < length;
-      const float inverse = 1.f / run_sum;
-      __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.output) + item.batch * a.o_batch_stride +
-                           static_cast<int64_t>(row_live ? row_pos : 0) * a.o_row_stride +
-                           row_head * a.o_head_stride;
+        // The running maximum only moves when the new one lies more than 2^8 above it
+        // (probabilities up to 256 are harmless in bf16 / fp32); moving it means rescaling
+        // the row of O in tensor memory, once the product that still adds to it is done.
+        const float new_max = fmaxf(run_max, tile_max);
+        const bool move = new_max > run_max && (new_max - run_max) * scale_log2 > 8.0f;
+        if (__any_sync(0xffffffffu, move)) {
+          float corr = 1.f;
+          if (move) {
+            corr = run_max == -INFINITY ? 0.f : exp2_fast((run_max - new_max) * scale_log2);
+            run_max = new_max;
+            run_sum *= corr;
+          }
+          if (block > 0) {
+            // P.V of the last block is done: this block's S was committed after it.  Rare, so
+            // rolled and in narrow steps, which take few registers beside the row of scores.
+#pragma unroll 1
+            for (int part = 0; part < 8; ++part) {
+              uint32_t o[16];
+              tmem_load16_issue(o_addr + part * 16u, o);
+              tmem_wait_load();
 #pragma unroll
-      for (int part = 0; part < 4; ++part) {
-        uint32_t o[32];
-        tmem_load32_issue(o_addr + part * 32u, o);
-        tmem_wait_load();
-        if (row_live) {
-#pragma unroll
-          for (int d = 0; d < 32; d += 8) {
-            uint4 v;
-            v.x = pack_bf16(__uint_as_float(o[d]) * inverse, __uint_as_float(o[d + 1]) * inverse);
-            v.y = pack_bf16(__uint_as_float(o[d + 2]) * inverse, __uint_as_float(o[d + 3]) * inverse);
-            v.z = pack_bf16(__uint_as_float(o[d + 4]) * inverse, __uint_as_float(o[d + 5]) * inverse);
-            v.w = pack_bf16(__uint_as_float(o[d + 6]) * inverse, __uint_as_float(o[d + 7]) * inverse);
-            *reinterpret_cast<uint4*>(dst + part * 32 + d) = v;
+              for (int c = 0; c < 16; ++c) {
+                o[c] = __float_as_uint(__uint_as_float(o[c]) * corr);
+              }
+              tmem_store16_issue(o_addr + part * 16u, o);
+            }
           }
         }
-      }
-      if (row_live) {
-        const float lse = run_max * a.softmax_scale + logf(run_sum);
-        const int64_t heads_total = a.query_heads;
-        a.lse[(item.batch * heads_total + row_head) * length + row_pos] = lse;
+        // ---- probabilities, bf16 pairs, over the first 64 columns of this S buffer ----
+        const float offset = (run_max == -INFINITY ? 0.f : run_max) * scale_log2;
+        const uint64_t scale_pair = pack_pair(scale_log2, scale_log2);
+        const uint64_t offset_pair = pack_pair(-offset, -offset);
+        uint64_t sum_pair[2] = {0ull, 0ull};
+#pragma unroll
+        for (int quarter = 0; quarter < 4; ++quarter) {
+          uint32_t packed[16];
+#pragma unroll
+          for (int e = 0; e < 16; ++e) {
+            const int c = quarter * 32 + 2 * e;
+            float x0, x1;
+            unpack_pair(fma_pair(pack_pair(s[c], s[c + 1]), scale_pair, offset_pair), x0, x1);
+            const float p0 = exp2_fast(x0);
+            const float p1 = exp2_fast(x1);
+            sum_pair[e & 1] = add_pair(sum_pair[e & 1], pack_pair(p0, p1));
+            packed[e] = pack_bf16(p0, p1);
+          }
+          tmem_store16_issue(s_addr + quarter * 16u, packed);
+        }
+        {
+          float a0, a1, b0, b1;
+          unpack_pair(sum_pair[0], a0, a1);
+          unpack_pair(sum_pair[1], b0, b1);
+          run_sum += (a0 + a1) + (b0 + b1);
+        }
+        tmem_wait_store();
+        tc_fence_before();
+        // one arrival per warp: 128 arrivals on one barrier word queue up behind each other
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(bar_p_full + 8 * t);
+        }
+
+        // The candidate bookkeeping is bound by the ALU and by its rounds of insertion, one at least
+        // in most blocks and classes; the gates keep their number down.  32 query on 8 KV heads,
+        // against a gate from the lists alone, rounds with a branch, and the rows behind the
+        // end taking part: 517 tokens 117 -> 39 us, 6001 tokens 1560 -> 530 us, 16384 tokens
+        // 3250 -> 2620 us (attention alone: 20, 326 and 1820 us).
+        // It runs from the scores still in registers while the tensor cores work on this
+        // tile's P.V and next S: it is off the path between two blocks.
         if constexpr (kMode == 1) {
-          const int skip = a.num_sink + kKappa - 1;
-          if (row_pos >= skip) {
-            // merge the four sorted class queues: eight times the largest head, which then
-            // leaves its queue (a cursor per queue would put the queues into local memory)
-            const int64_t base =
-                ((item.batch * heads_total + row_head) * (length - skip) + (row_pos - skip)) * kKappa;
-            const float lse_log2 = lse * kLog2e;
+          const int sinks = a.num_sink - key0;  // columns of this block that are no candidates
+          if (sinks > 0) {
+            // the groups' maxima without them: the upper 64 columns, if that is far enough
 #pragma unroll
-            for (int rank = 0; rank < kKappa; ++rank) {
-              const uint32_t best = max(max(q32[0][0], q32[1][0]), max(q32[2][0], q32[3][0]));
+            for (int i = 0; i < 8; ++i) {
+              part_max[i] = s[64 + i];
 #pragma unroll
-              for (int c = 0; c < 4; ++c) {
-                const bool leaves = q32[c][0] == best;
-#pragma unroll
-                for (int k = 0; k < kLocalK; ++k) {
-                  q32[c][k] = leaves ? (k + 1 < kLocalK ? q32[c][k + 1] : 0u) : q32[c][k];
-                }
+              for (int c = 72 + i; c < 128; c += 8) {
+                part_max[i] = fmaxf(part_max[i], s[c]);
               }
-              const float dequant = static_cast<float>(best >> 17) / 256.0f - 48.0f;
-              a.topk_val[base + rank] = exp2f(dequant * scale_log2 - lse_log2);
-              a.topk_idx[base + rank] = static_cast<int32_t>(best & 0x1ffffu);
+            }
+          }
+          // A key that is below two keys of every class can never reach the output (the class
+          // lists then hold at least eight keys above it), nor one below the top four of two
+          // classes.  Two keys of every class: the second-best entries of the lists, or the
+          // maxima of this block's two column groups of every class.
+          const uint32_t third0 = q32[0][3], third1 = q32[1][3], third2 = q32[2][3], third3 = q32[3][3];
+          const uint32_t second_of_fourths =
+              max(min(max(third0, third1), max(third2, third3)),
+                  max(min(third0, third1), min(third2, third3)));
+          const uint32_t row_floor = max(min(min(q32[0][1], q32[1][1]), min(q32[2][1], q32[3][1])),
+                                         second_of_fourths);
+          float block_floor =
+              min_nan(min_nan(min_nan(part_max[0], part_max[1]), min_nan(part_max[2], part_max[3])),
+                      min_nan(min_nan(part_max[4], part_max[5]), min_nan(part_max[6], part_max[7])));
+          block_floor = sinks > 64 ? -INFINITY : block_floor;
+          const uint32_t floor_key = max(row_floor >> 17, quantised_key_fma(block_floor));
+          // smallest raw score whose quantised key can reach the floor, a little low
+          float gate = floor_key == 0u
+                           ? -3.0e38f
+                           : (static_cast<float>(floor_key) - 0.75f) * (1.0f / 256.0f) - 48.0f;
+          // rows behind the end of a ragged prompt score 0 everywhere: ties that all reach the gate
+          gate = live ? gate : INFINITY;
+          // (no vote in front of a class: in most blocks some row of the warp has a taker)
+          take_candidates<0>(s, gate, key0, sinks, q32[0]);
+          take_candidates<1>(s, gate, key0, sinks, q32[1]);
+          take_candidates<2>(s, gate, key0, sinks, q32[2]);
+          take_candidates<3>(s, gate, key0, sinks, q32[3]);
+        }
+      }
+
+      // the next item under the last product; the ring's slots up to it are visible then
+      if (kMany && !failed && !pair_wait_warp(bar_of(n + 1), parity_of(n + 1), abort)) {
+        failed = true;
+      }
+      if (!failed && !pair_wait_warp(bar_o_full + 8 * t, n & 1, abort)) {
+        failed = true;
+      }
+      if (!failed) {
+        tc_fence_after();
+        // not held in registers through the loop
+        PairItem item;
+        if constexpr (kMany) {
+          item = read_item(slot_of(n));
+        } else {
+          uint32_t again = blockIdx.x;
+          asm volatile("" : "+r"(again));
+          item.set(a, again);
+        }
+        const int row_pos = item.pos0 + row;
+        const int row_head = item.head0 + t;
+        const bool row_live = row_pos < length;
+        const float inverse = 1.f / run_sum;
+        __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.output) + item.batch * a.o_batch_stride +
+                             static_cast<int64_t>(row_live ? row_pos : 0) * a.o_row_stride +
+                             row_head * a.o_head_stride;
+#pragma unroll
+        for (int part = 0; part < 4; ++part) {
+          uint32_t o[32];
+          tmem_load32_issue(o_addr + part * 32u, o);
+          tmem_wait_load();
+          if (row_live) {
+#pragma unroll
+            for (int d = 0; d < 32; d += 8) {
+              uint4 v;
+              v.x = pack_bf16(__uint_as_float(o[d]) * inverse, __uint_as_float(o[d + 1]) * inverse);
+              v.y = pack_bf16(__uint_as_float(o[d + 2]) * inverse, __uint_as_float(o[d + 3]) * inverse);
+              v.z = pack_bf16(__uint_as_float(o[d + 4]) * inverse, __uint_as_float(o[d + 5]) * inverse);
+              v.w = pack_bf16(__uint_as_float(o[d + 6]) * inverse, __uint_as_float(o[d + 7]) * inverse);
+              *reinterpret_cast<uint4*>(dst + part * 32 + d) = v;
+            }
+          }
+        }
+        if (row_live) {
+          const float lse = run_max * a.softmax_scale + logf(run_sum);
+          const int64_t heads_total = a.query_heads;
+          a.lse[(item.batch * heads_total + row_head) * length + row_pos] = lse;
+          if constexpr (kMode == 1) {
+            const int skip = a.num_sink + kKappa - 1;
+            if (row_pos >= skip) {
+              // merge the four sorted class queues: eight times the largest head, which then
+              // leaves its queue (a cursor per queue would put the queues into local memory)
+              const int64_t base =
+                  ((item.batch * heads_total + row_head) * (length - skip) + (row_pos - skip)) * kKappa;
+              const float lse_log2 = lse * kLog2e;
+#pragma unroll
+              for (int rank = 0; rank < kKappa; ++rank) {
+                const uint32_t best = max(max(q32[0][0], q32[1][0]), max(q32[2][0], q32[3][0]));
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                  const bool leaves = q32[c][0] == best;
+#pragma unroll
+                  for (int k = 0; k < kLocalK; ++k) {
+                    q32[c][k] = leaves ? (k + 1 < kLocalK ? q32[c][k + 1] : 0u) : q32[c][k];
+                  }
+                }
+                const float dequant = static_cast<float>(best >> 17) / 256.0f - 48.0f;
+                a.topk_val[base + rank] = exp2f(dequant * scale_log2 - lse_log2);
+                a.topk_idx[base + rank] = static_cast<int32_t>(best & 0x1ffffu);
+              }
             }
           }
         }
       }
-    }
-    pos0 = kMany ? read_item(slot_of(n + 1)).pos0 : -1;
+      pos0 = kMany ? read_item(slot_of(n + 1)).pos0 : -1;
     }
   }
 
