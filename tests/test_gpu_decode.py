@@ -716,6 +716,48 @@ def test_selection_over_few_communities(monkeypatch, communities):
     _run_sequence(layer, config, steps=3, seed=6100)
 
 
+def test_fp32_layers_back_to_back():
+    """The kernels of a layer with an fp32 table do not stand in the way of the layer before it: back to back it takes
+    about what it takes with a small kernel in between (let go early, an eighth longer)."""
+
+    device = torch.device("cuda", 0)
+    layer = make_layer(seed=7, seq_len=8192, communities=64, max_decode_tokens=1000)
+    layer.assembled.centroids = layer.assembled.centroids.float()
+    layer = layer.to(device)
+    runtime = DecodeRuntime(CommunityKVConfig(token_budget=1024, num_sink=10, lam=0.5, aggregation="query_group",
+                                              centroid_dtype="fp32"))
+    runtime.prepare_layer(0, **layer.prepare_kwargs())
+    query = make_query(seed=900, query_heads=layer.query_heads).to(device)[None, :, None, :]
+    cache = torch.zeros((2, 8, 16, 128), dtype=torch.bfloat16, device=device)
+    row = torch.ones((8, 128), dtype=torch.bfloat16, device=device)
+
+    def microseconds(apart):
+        def step():
+            if apart:
+                ops.append_kv(cache[0], cache[1], row, row, 3)
+            runtime.decode(layer_idx=0, query=query, key=layer.key[None], value=layer.value[None], softmax_scale=SCALE)
+
+        step()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for _ in range(40):
+                step()
+        spans = []
+        for _ in range(6):
+            begin, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            torch.cuda.synchronize()
+            begin.record()
+            graph.replay()
+            end.record()
+            end.synchronize()
+            spans.append(begin.elapsed_time(end) * 25)
+        return min(spans)
+
+    apart = microseconds(True)
+    assert microseconds(False) < 1.08 * apart
+    runtime.assert_no_overflow()
+
+
 def test_full_size_batch_one_launch_equals_four_kernels():
     """The batched long-context configuration as far as one layer goes (8 sequences x 8 KV heads at ctx 131072,
     1024-4096 Zipf communities, budget 2048): the single cluster launch and the four
