@@ -815,10 +815,12 @@ __global__ void __launch_bounds__(128) exact_edges_kernel(const ckv_prefill_args
 // scan of the row's keys.  256 threads per row: every thread scores the keys
 // j = tid, tid + 256, ... in the fixed fp32 order and keeps its own sorted top-m; the
 // 256 lists are then merged m times by a block-wide maximum.  CTAs take rows from the
-// queue exact_edges_kernel filled (or, without a queue, poll every row's flag).
+// queue exact_edges_kernel filled (or, without a queue, look for the flags themselves).
 // Few rows are left to it, so a row's own time counts: a warp copies its 32 key rows of the
 // next step together into shared memory (as exact_edges_kernel does) while it scores this one's.
-// 6001 tokens, 62 of 47808 rows: 904 -> 886 us for the whole call.
+// 6001 tokens, 62 of 47808 rows: 904 -> 886 us for the whole call.  Its registers and stage leave room for
+// one CTA per SM, which costs nothing where every row is scanned: 12.8 -> 10.6 ms (1500 tokens 1357 ->
+// 1296 us; repeated keys, 7317 of 23800 rows, 2018 -> 1613 us).
 constexpr int kRescanStage = 8 * 2 * 32 * 256;  // eight warps, two steps of 32 rows
 
 __global__ void __launch_bounds__(256) exact_rescan_kernel(const ckv_prefill_args a, int group) {
@@ -826,6 +828,7 @@ __global__ void __launch_bounds__(256) exact_rescan_kernel(const ckv_prefill_arg
   extern __shared__ __align__(128) uint8_t rescan_smem[];
   uint64_t* lists = reinterpret_cast<uint64_t*>(rescan_smem);  // once the keys have been scored
   __shared__ uint64_t warp_best[8];
+  __shared__ uint32_t todo[8];
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int warp = tid >> 5;
@@ -833,13 +836,7 @@ __global__ void __launch_bounds__(256) exact_rescan_kernel(const ckv_prefill_arg
   const int skip = a.num_sink + a.edges_per_row - 1;
   const int rows = length - skip;
   const int64_t total = static_cast<int64_t>(a.batch) * a.kv_heads * rows;
-  const bool queued = a.rescan_list != nullptr;
-  const int64_t work = queued ? a.rescan_list[0] : total;
-  for (int64_t w = blockIdx.x; w < work; w += gridDim.x) {
-    const int64_t item = queued ? a.rescan_list[1 + w] : w;
-    if (!queued && a.edge_flags[item] == 0) {
-      continue;
-    }
+  auto scan = [&](int64_t item) {
     const int pos = skip + static_cast<int>(item % rows);
     const int kv_head = static_cast<int>((item / rows) % a.kv_heads);
     const int batch = static_cast<int>(item / (static_cast<int64_t>(rows) * a.kv_heads));
@@ -954,6 +951,31 @@ __global__ void __launch_bounds__(256) exact_rescan_kernel(const ckv_prefill_arg
             winner == 0ull ? -INFINITY : key32_to_float(static_cast<uint32_t>(winner >> 32));
       }
       __syncthreads();
+    }
+  };
+  // A CTA's rows lie gridDim.x apart, in the queue or among all rows; without a queue it looks at the
+  // flags of 256 of them at once (a CTA per row, most of them for the sake of its flag, took one query
+  // head per KV head with 1500 tokens and 438 of 11800 rows A).
+  const int64_t stride = gridDim.x;
+  if (a.rescan_list != nullptr) {
+    const int64_t work = a.rescan_list[0];
+    for (int64_t w = blockIdx.x; w < work; w += stride) {
+      scan(a.rescan_list[1 + w]);
+    }
+    return;
+  }
+  for (int64_t first = blockIdx.x; first < total; first += 256 * stride) {
+    const int64_t own = first + tid * stride;
+    const uint32_t flagged = __ballot_sync(0xffffffffu, own < total && a.edge_flags[own] != 0);
+    __syncthreads();  // the last 256 rows are done
+    if (lane == 0) {
+      todo[warp] = flagged;
+    }
+    __syncthreads();
+    for (int word = 0; word < 8; ++word) {
+      for (uint32_t left = todo[word]; left != 0u; left &= left - 1u) {
+        scan(first + (32 * word + __ffs(left) - 1) * stride);
+      }
     }
   }
 }
@@ -1419,7 +1441,7 @@ cudaError_t launch_prefill(const ckv_prefill_args& a, cudaStream_t stream) {
   if (err != cudaSuccess || a.edge_flags == nullptr) {
     return err;
   }
-  const long long rescan_grid = a.rescan_list != nullptr ? (items < 148 * 4 ? items : 148 * 4) : items;
+  const int64_t rescan_grid = items < 148 * 4 ? items : 148 * 4;
   err = cudaFuncSetAttribute(exact_rescan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRescanStage);
   if (err != cudaSuccess) return err;
   exact_rescan_kernel<<<static_cast<unsigned>(rescan_grid), 256, kRescanStage, stream>>>(a, group);

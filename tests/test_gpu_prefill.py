@@ -6,7 +6,9 @@ import numpy as np
 import pytest
 import torch
 
+from community_kv_b200 import native
 from community_kv_b200.prefill import (
+    _pack,
     check_status,
     prefill_attention,
     prefill_attention_edges,
@@ -151,6 +153,33 @@ def test_exact_edges_rescan_path():
     want_idx, want_score = oracle.exact_edges(q[0].float().numpy(), k[0].float().numpy(), SCALE, sinks, edges)
     assert np.array_equal(edge_idx[0].cpu().numpy(), want_idx)
     assert np.array_equal(edge_score[0].cpu().numpy().view(np.uint32), want_score.view(np.uint32))
+
+
+@pytest.mark.parametrize("batch,kv_heads,length,slack", [(1, 2, 700, 1e-3), (1, 2, 700, 1e9), (2, 32, 2500, 1e-3)])
+def test_exact_edges_without_a_queue(batch, kv_heads, length, slack):
+    """The queue of rows to scan again is optional: without it the flags lead to the same edges, with few rows, with
+    all of them, and with more rows than the launch looks at in one go."""
+
+    generator = torch.Generator(device="cuda").manual_seed(length)
+    q, k = (torch.randn((batch, length, kv_heads, 128), generator=generator, device="cuda").to(torch.bfloat16)
+            for _ in range(2))
+    _, _, want_idx, want_score, want_flags = prefill_attention_edges(
+        q, k, k, softmax_scale=SCALE, num_sink=3, edges_per_row=16, exact_slack=slack)
+    rows = length - 18
+    assert 0 < int(want_flags.sum()) and (slack < 1 or int(want_flags.sum()) > 0.9 * want_flags.numel())
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    args, *keep = _pack(q, k, k, softmax_scale=SCALE, num_sink=3, mode=2, edges_per_row=16, exact_slack=slack,
+                        status=status)
+    candidates = torch.empty((batch, kv_heads, length, 1, 17), dtype=torch.int64, device="cuda")
+    edge_idx = torch.full((batch, kv_heads, rows, 16), -2, dtype=torch.int32, device="cuda")
+    edge_score = torch.zeros((batch, kv_heads, rows, 16), device="cuda")
+    flags = torch.empty((batch, kv_heads, rows), dtype=torch.int32, device="cuda")
+    native.fill(args, candidates=candidates.data_ptr(), edge_idx=edge_idx.data_ptr(), edge_score=edge_score.data_ptr(),
+                edge_flags=flags.data_ptr(), rescan_list=None)
+    native.call("ckv_prefill_topk", args, native.current_stream(q.device))
+    check_status(status)
+    del keep  # the tensors that the launch wrote and read
+    assert torch.equal(edge_idx, want_idx) and torch.equal(edge_score, want_score) and torch.equal(flags, want_flags)
 
 
 def test_batch_and_validation():
