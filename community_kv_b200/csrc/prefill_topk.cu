@@ -131,11 +131,20 @@ __global__ void __launch_bounds__(kPfThreads, 1)
   const int row = tid & (kPfRows - 1);
   const int half = tid >> 7;            // which 64 of the 128 columns / output dims
   const int col0 = half * 64;
-  // all heads' longest tiles first, then the tiles before them
+  // All heads' longest tiles first, then the tiles before them - or head after head, where every tile has
+  // an SM at once and is long: the insertions of equal tiles on the two SMs of a TPC slow each other down
+  // (1500 tokens, 8 heads: 680 thousand cycles for the last tile, 505 where the other SM was done).  Exact
+  // edges of one query head per KV head, us a call, tile after tile / head after head, on two GPUs: 8
+  // heads of 700 tokens 197 / 200, 16 heads of 1000 tokens 305, 325 / 264, 264, 8 of 1500 383, 442 / 345,
+  // 358, 4 of 2500 560, 660 / 467, 491; eight query heads per KV head, 517 tokens 122 / 128, 1500 and 2300
+  // tokens the same.
   const int lanes = a.kv_heads * a.batch;
-  const int tile = (gridDim.x - 1 - blockIdx.x) / lanes;
-  const int kv_head = blockIdx.x % lanes % a.kv_heads;
-  const int batch = blockIdx.x % lanes / a.kv_heads;
+  const int tiles = gridDim.x / lanes;
+  const bool by_head = kMode == 2 && gridDim.x <= 148u && a.seq_len > 7 * kPfKeys;
+  const int lane_of_cta = by_head ? blockIdx.x / tiles : blockIdx.x % lanes;
+  const int tile = tiles - 1 - static_cast<int>(by_head ? blockIdx.x % tiles : blockIdx.x / lanes);
+  const int kv_head = lane_of_cta % a.kv_heads;
+  const int batch = lane_of_cta / a.kv_heads;
   const int pos0 = tile * kPositions;
   const int length = a.seq_len;
   const int row_pos = pos0 + row / kGroup;

@@ -105,6 +105,20 @@ def test_exact_edges_are_bit_exact(length, heads, kv_heads, edges):
     assert int(flags.sum()) <= flags.numel() // 20
 
 
+@pytest.mark.parametrize("length,heads,kv_heads,batch", [(896, 2, 2, 2), (897, 2, 2, 2), (1100, 3, 3, 1), (1000, 8, 1, 2)])
+def test_exact_edges_head_after_head(length, heads, kv_heads, batch):
+    """On both sides of the line between tiles of all heads by length and one head's tiles behind another's."""
+
+    sinks, edges = 4, 16
+    q, k, v = _inputs(17, length, heads, kv_heads, batch=batch)
+    _, _, edge_idx, edge_score, _ = prefill_attention_edges(
+        q.cuda(), k.cuda(), v.cuda(), softmax_scale=SCALE, num_sink=sinks, edges_per_row=edges)
+    for b in range(batch):
+        want_idx, want_score = oracle.exact_edges(q[b].float().numpy(), k[b].float().numpy(), SCALE, sinks, edges)
+        assert np.array_equal(edge_idx[b].cpu().numpy(), want_idx)
+        assert np.array_equal(edge_score[b].cpu().numpy().view(np.uint32), want_score.view(np.uint32))
+
+
 @pytest.mark.parametrize("length,heads,kv_heads,sinks", [(100, 4, 2, 4), (129, 8, 2, 0), (12, 2, 1, 3), (9, 4, 1, 4)])
 def test_reference_topk_rule_short_and_ragged(length, heads, kv_heads, sinks):
     """Rows shorter than one tile, a tile of a single row, a prompt barely longer than the sinks."""
