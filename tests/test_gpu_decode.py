@@ -10,6 +10,7 @@ import torch
 
 from community_kv_b200 import native, ops
 from community_kv_b200.batched import BatchedDecodeRuntime
+from community_kv_b200.cache import StaticCacheLayer
 from community_kv_b200.config import CommunityKVConfig, GraphAggregation
 from community_kv_b200.runtime import DecodeRuntime, convert_prefill_tensors
 from community_kv_b200.state import DecodeLayerWorkspace
@@ -595,6 +596,31 @@ def test_append_kv_of_many_rows_uses_the_chip():
     assert microseconds(True) < 4 * microseconds(False) + 5
 
 
+def test_the_cache_appends_under_capture():
+    """The device phase of the plug-in's cache needs no host: a captured append writes another row at every replay."""
+
+    device = torch.device("cuda", 0)
+    layer = StaticCacheLayer(max_cache_len=12)
+    prompt = torch.randn((1, 6, 4, 128), device=device).to(torch.bfloat16)
+    row_key, row_value = (torch.randn((1, 6, 1, 128), device=device).to(torch.bfloat16) for _ in range(2))
+    with torch.inference_mode():
+        layer.update(prompt, prompt)
+        layer.enable_device_updates()
+        layer.update(row_key, row_value)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            layer.update(row_key, row_value)
+        want_key, want_value = layer.keys.clone(), layer.values.clone()
+        for row in (5, 6, 7):
+            row_key.copy_(torch.randn_like(row_key))
+            row_value.copy_(torch.randn_like(row_value))
+            graph.replay()
+            want_key[:, :, row], want_value[:, :, row] = row_key[:, :, 0], row_value[:, :, 0]
+        layer.sync_valid_length()
+    assert layer.valid_length == 8
+    assert torch.equal(layer.keys, want_key) and torch.equal(layer.values, want_value)
+
+
 @pytest.mark.parametrize("units", [1, 3, 40])
 def test_append_kv_past_the_last_row(units):
     """A row that only the device knows and that lies outside the cache writes nothing: not into the next head's rows,
@@ -670,6 +696,87 @@ def test_followers_of_a_shared_graph_match_the_oracle(kv_heads, fp32):
     config = CommunityKVConfig(token_budget=256, num_sink=3, lam=0.5, aggregation="layer_wise",
                                centroid_dtype="fp32" if fp32 else "e4m3")
     _run_sequence(layer, config, steps=4, seed=3000 + kv_heads)
+
+
+@pytest.mark.parametrize("kv_heads,splits,kernels", [(3, 11, 2), (1, 9, 1), (2, None, 4)])
+def test_shared_graph_with_more_than_eight_splits(kv_heads, splits, kernels):
+    """One graph for all heads in a cluster of more than eight CTAs, and in the four kernels, against the oracle."""
+
+    layer = make_layer(seed=53, seq_len=12007, communities=301, kv_heads=kv_heads, max_decode_tokens=6,
+                       aggregation="layer_wise", zipf_exponent=1.1)
+    config = CommunityKVConfig(token_budget=8192, num_sink=10, lam=0.5, aggregation="layer_wise")
+    state, _ = _run_sequence(layer, config, steps=4, seed=5300, splits=splits)
+    assert native.library().ckv_decode_layer_kernels(ctypes.byref(state.args)) == kernels
+
+
+@pytest.mark.parametrize("kv_heads,kernels", [(12, 2), (13, 4)])
+def test_shared_graph_on_both_sides_of_the_line(kv_heads, kernels):
+    """96 CTAs of the cluster launch are the most that take two launches."""
+
+    layer = make_layer(seed=57, kv_heads=kv_heads, group_size=1, seq_len=2053, communities=40, max_decode_tokens=5,
+                       aggregation="layer_wise")
+    config = CommunityKVConfig(token_budget=1024, num_sink=10, lam=0.5, aggregation="layer_wise")
+    state, _ = _run_sequence(layer, config, steps=3, seed=5700, splits=8)
+    assert native.library().ckv_decode_layer_kernels(ctypes.byref(state.args)) == kernels
+
+
+@pytest.mark.parametrize("batch,kv_heads,deferred", [(3, 5, False), (3, 5, True), (2, 23, False)])
+def test_shared_graphs_in_a_batch(batch, kv_heads, deferred):
+    """Every sequence has a graph of its own that all its heads share: leaders and followers of each are the oracle's."""
+
+    device = torch.device("cuda", 0)
+    config = CommunityKVConfig(token_budget=256, num_sink=3, lam=0.5, aggregation="layer_wise")
+    layers = [make_layer(seed=110 + b, kv_heads=kv_heads, group_size=2, seq_len=1500, communities=30 + 7 * b,
+                         max_decode_tokens=6, aggregation="layer_wise") for b in range(batch)]
+    runtime = BatchedDecodeRuntime(config, splits=2, defer_update=deferred)
+    state = runtime.prepare_layer(0, [convert_prefill_tensors(**layer.to(device).prepare_kwargs()) for layer in layers])
+    twins = []
+    for b in range(batch):
+        twins.append(OracleLayer(*state.sequence_view(b), token_budget=256, num_sink=3,
+                                 cover=state.workspace.selection.score_cover[b].cpu().tolist()))
+    key = torch.stack([layer.key for layer in layers]).to(device)
+    value = torch.stack([layer.value for layer in layers]).to(device)
+    for step in range(4):
+        queries = torch.stack([make_query(seed=1200 + 10 * step + b, query_heads=2 * kv_heads) for b in range(batch)])
+        runtime.decode(layer_idx=0, query=queries.to(device), key=key, value=value, softmax_scale=SCALE)
+        torch.cuda.synchronize()
+        for b in range(batch):
+            twins[b].step(query=queries[b], key=layers[b].key, value=layers[b].value, softmax_scale=SCALE, lam=config.lam,
+                          device_scores=state.workspace.selection.scores[b])
+            _, mutable, current = state.sequence_view(b)
+            assert_state_equal(mutable, twins[b].state, f"step {step} seq {b}")
+            assert torch.equal(current.cpu(), twins[b].current)
+    runtime.assert_no_overflow()
+
+
+def test_overflow_leaves_the_followers_alone():
+    """Beyond the room for decoded tokens a shared graph reports it, and its followers' tables stay as they are."""
+
+    layer = make_layer(seed=43, kv_heads=3, seq_len=1024, communities=16, max_decode_tokens=2, aggregation="layer_wise")
+    config = CommunityKVConfig(token_budget=128, num_sink=2, lam=0.5, aggregation="layer_wise")
+    device = torch.device("cuda", 0)
+    runtime = DecodeRuntime(config, splits=1)
+    state = runtime.prepare_layer(0, **layer.to(device).prepare_kwargs())
+    twin = OracleLayer(state.converted.csr, state.converted.mutable, state.converted.current_position,
+                       token_budget=128, num_sink=2, cover=_cover(state.converted))
+    key, value = layer.key.to(device)[None], layer.value.to(device)[None]
+    flags = []
+    for step in range(5):
+        before = [tensor.clone() for tensor in (state.converted.mutable.centroids.view(torch.uint8),
+                                                state.converted.mutable.community_sizes,
+                                                state.converted.mutable.community_counts)]
+        query = make_query(seed=820 + step, query_heads=layer.query_heads)
+        runtime.decode(layer_idx=0, query=query.to(device)[None, :, None, :], key=key, value=value, softmax_scale=SCALE)
+        want = twin.step(query=query, key=layer.key, value=layer.value, softmax_scale=SCALE, lam=0.5,
+                         device_scores=state.workspace.selection.scores)
+        assert torch.equal(state.workspace.update.overflow.cpu(), want.overflow), step
+        assert_state_equal(state.converted.mutable, twin.state, f"step {step}")
+        flags.append(int(state.workspace.update.overflow.max()))
+        if flags[-1]:
+            after = (state.converted.mutable.centroids.view(torch.uint8), state.converted.mutable.community_sizes,
+                     state.converted.mutable.community_counts)
+            assert all(torch.equal(x[1:], y[1:]) for x, y in zip(before, after))
+    assert flags[0] == 0 and flags[-1] != 0
 
 
 def test_many_followers_cost_an_update_little():
