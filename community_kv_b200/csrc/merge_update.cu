@@ -86,13 +86,16 @@ __device__ __forceinline__ void sync_followers(const ckv_layer_args& a, int flat
   }
 }
 
-__global__ void __launch_bounds__(kUpdateMaxThreads) merge_update_kernel(const ckv_layer_args a) {
+// kFollowers: several heads share a graph (a kernel of its own, so that the other keeps its registers).
+template <bool kFollowers>
+__global__ void __launch_bounds__(kFollowers ? kUpdateMaxThreads : kMergeThreads + 32)
+    merge_update_kernel(const ckv_layer_args a) {
   __shared__ UpdateDecision decision;
   __shared__ float lse_s;
   pdl_release_dependents();
   pdl_wait_for_predecessor();  // partials and candidates come from the attention kernel
   merge_update_unit<8>(a, blockIdx.x, kMergeThreads / 32, decision, lse_s);
-  if (a.retrieval_heads != a.graphs && !(a.flags & CKV_FLAG_SKIP_UPDATE)) {
+  if constexpr (kFollowers) {
     sync_followers(a, blockIdx.x, decision);
   }
   if (blockIdx.x == 0) {
@@ -362,14 +365,15 @@ cudaError_t launch_nearest_centroid(const ckv_layer_args& a, int32_t* forced, cu
 // the followers / five warps / so: 16 heads 6.8 / 6.3 / 6.1, 32 heads 7.2 / 8.4 / 6.5, 64 heads
 // 7.2 / 12.3 / 7.2.  A whole CTA per head, four heads in flight, took 15.2, 27 and 51.
 cudaError_t launch_merge_update(const ckv_layer_args& a, cudaStream_t stream) {
-  int warps = kMergeThreads / 32 + 1;
   const int units = a.batch * a.retrieval_heads;
-  if (a.retrieval_heads != a.graphs && !(a.flags & CKV_FLAG_SKIP_UPDATE)) {
-    const int wanted = (a.retrieval_heads + kFollowersInFlight - 1) / kFollowersInFlight;
-    const int most = min(kUpdateMaxThreads / 32, 148 * (kUpdateMaxThreads / 32) / units);
-    warps = max(warps, min(wanted, most));
+  const int fewest = kMergeThreads / 32 + 1;
+  if (a.retrieval_heads == a.graphs || (a.flags & CKV_FLAG_SKIP_UPDATE)) {
+    return launch_dependent(merge_update_kernel<false>, dim3(units), dim3(32 * fewest), 0, stream, a);
   }
-  return launch_dependent(merge_update_kernel, dim3(units), dim3(32 * warps), 0, stream, a);
+  const int wanted = (a.retrieval_heads + kFollowersInFlight - 1) / kFollowersInFlight;
+  const int most = min(kUpdateMaxThreads / 32, 148 * (kUpdateMaxThreads / 32) / units);
+  const int warps = max(fewest, min(wanted, most));
+  return launch_dependent(merge_update_kernel<true>, dim3(units), dim3(32 * warps), 0, stream, a);
 }
 
 }  // namespace ckv
