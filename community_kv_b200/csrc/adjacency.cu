@@ -32,10 +32,10 @@
 // Three blocks per SM leave a thread eighty registers.  A tile's items therefore take their places in
 // shared memory before the look-back, which then holds only counts, and ranks are kept as halves:
 // with the items held across the look-back the 4-byte pass spilled 324 bytes of stores and 392 of
-// loads per thread, now 8 (the first pass none, 36 where the neighbours per row are not eight).  Of a layer of 32
-// graphs of 8192 positions, 11.5 M raw edges, from its neighbours to its decode state: 1680 -> 1586 us
-// (halves alone 1651).  The sort takes a good half millisecond of it;
-// five passes over enumerated 12-byte items with separate count and scan kernels took 1.1 ms.
+// loads per thread, now 8 (the first pass none, 36 where the neighbours per row are not eight).  The call
+// for 32 graphs of 8192 positions, 11.5 M raw edges of random neighbours: 776 -> 697 us, for 8 such graphs
+// 343 -> 326, for one of 1024 positions 164 -> 150.
+// Five passes over enumerated 12-byte items with separate count and scan kernels took 1.1 ms.
 
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -259,7 +259,7 @@ __device__ __forceinline__ void take_candidates(const float (&s)[128], float gat
 // launch, Q and first K, output (about 20000 cycles against 3700 per key block) each time.  Shares dealt
 // out before the launch save that too, but a CTA whose SM is held by another kernel then keeps its
 // whole share waiting.  32 query on 8 KV heads, us a call, attention alone and with neighbours: a CTA
-// per item / shares / so: 4096 tokens 139, 135, 132 and 248, 247, 245; 16384 tokens 1806, 1770, 1739
+// per item / shares / so: 4096 tokens 139, 135, 133 and 248, 247, 245; 16384 tokens 1806, 1770, 1748
 // and about 2700 each.  Attention alone beside a kernel that holds 16 SMs for 1.7 ms, shares / so:
 // 4096 tokens 291 and 189, 16384 tokens 3270 and 1892.
 struct PairItem {
