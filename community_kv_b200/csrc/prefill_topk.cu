@@ -139,10 +139,15 @@ __global__ void __launch_bounds__(kPfThreads, 1)
   // 358, 4 of 2500 560, 660 / 467, 491; eight query heads per KV head, 517 tokens 122 / 128, 1500 and 2300
   // tokens the same.
   const int lanes = a.kv_heads * a.batch;
-  const int tiles = gridDim.x / lanes;
-  const bool by_head = kMode == 2 && gridDim.x <= 148u && a.seq_len > 7 * kPfKeys;
-  const int lane_of_cta = by_head ? blockIdx.x / tiles : blockIdx.x % lanes;
-  const int tile = tiles - 1 - static_cast<int>(by_head ? blockIdx.x % tiles : blockIdx.x / lanes);
+  int tile = (gridDim.x - 1 - blockIdx.x) / lanes;
+  int lane_of_cta = blockIdx.x % lanes;
+  if constexpr (kMode == 2) {
+    if (gridDim.x <= 148u && a.seq_len > 7 * kPfKeys) {
+      const int tiles = gridDim.x / lanes;
+      tile = tiles - 1 - static_cast<int>(blockIdx.x % tiles);
+      lane_of_cta = blockIdx.x / tiles;
+    }
+  }
   const int kv_head = lane_of_cta % a.kv_heads;
   const int batch = lane_of_cta / a.kv_heads;
   const int pos0 = tile * kPositions;
