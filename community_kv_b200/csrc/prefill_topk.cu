@@ -664,7 +664,12 @@ __global__ void __launch_bounds__(kPfThreads, 1)
 // a conflict (every lane loading its own row from global memory touched 32 lines per instruction).
 // Up to 32 candidates are ranked by a sort over the lanes.  32 query on 8 KV heads, sixteen edges, a
 // whole call: 6001 tokens 991 -> 910 us, 1500 tokens 279 -> 254 us.
-__global__ void __launch_bounds__(128) exact_edges_kernel(const ckv_prefill_args a, int group, int lists) {
+// kSlots: rounds of 32 candidates; the next round's rows come while this one's are scored.  kResident: CTAs
+// per SM that the registers leave room for.  A short prompt has fewer, and its warps hide their own reads the
+// better the more registers they have; eight query heads per KV head, us a call, five / three: 4 KV heads of
+// 64 tokens 59.4 / 52.7, 2 of 300 tokens 101.6 / 94.9, 4 of 1500 tokens 355 / 361, of 6001 tokens 2265 / 2290.
+template <int kSlots, int kResident>
+__global__ void __launch_bounds__(128, kResident) exact_edges_kernel(const ckv_prefill_args a, int group, int lists) {
   const int warps_per_block = 4;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -697,7 +702,7 @@ __global__ void __launch_bounds__(128) exact_edges_kernel(const ckv_prefill_args
                                                            (index & 15) * 8);
   }
   __syncwarp();
-  uint64_t best_key[4];
+  uint64_t best_key[kSlots];
   float best_dropped = -INFINITY;  // best approximate score among the keys turned away
   if (lane < lists) {
     const uint64_t lost = list[lane * (kExactKeep + 1) + kExactKeep];
@@ -705,21 +710,19 @@ __global__ void __launch_bounds__(128) exact_edges_kernel(const ckv_prefill_args
       best_dropped = key32_to_float(static_cast<uint32_t>(lost >> 32));
     }
   }
+  int found[kSlots];  // the lane's candidates, -1: none
 #pragma unroll
-  for (int slot = 0; slot < 4; ++slot) {
-    best_key[slot] = 0ull;
-    if (32 * slot >= candidates) {
-      continue;  // the same for the whole warp
-    }
+  for (int slot = 0; slot < kSlots; ++slot) {
     const int index = lane + 32 * slot;
-    int j = -1;
+    found[slot] = -1;
     if (index < candidates) {
       const uint64_t packed = list[(index / kExactKeep) * (kExactKeep + 1) + index % kExactKeep];
       // the lists of a launch that gave up a wait may hold anything
-      j = packed == 0ull ? -1 : static_cast<int>(0xffffffffu - static_cast<uint32_t>(packed));
-      j = j > pos ? -1 : j;
+      found[slot] = packed == 0ull ? -1 : static_cast<int>(0xffffffffu - static_cast<uint32_t>(packed));
+      found[slot] = found[slot] > pos ? -1 : found[slot];
     }
-    __syncwarp();  // the last slot's rows have been read
+  }
+  auto fetch = [&](int j) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       const int row = 2 * i + (lane >> 4);
@@ -729,15 +732,28 @@ __global__ void __launch_bounds__(128) exact_edges_kernel(const ckv_prefill_args
                  k_base + static_cast<int64_t>(max(from, 0)) * a.k_row_stride + chunk * 8, from >= 0 ? 16u : 0u);
     }
     cp_async_commit();
+  };
+  fetch(found[0]);
+#pragma unroll
+  for (int slot = 0; slot < kSlots; ++slot) {
+    best_key[slot] = 0ull;
+    if (32 * slot >= candidates) {
+      continue;  // the same for the whole warp
+    }
     cp_async_wait<0>();
     __syncwarp();
-    if (j < 0) {
-      continue;
-    }
     uint4 k_reg[16];
 #pragma unroll
     for (int piece = 0; piece < 16; ++piece) {
       k_reg[piece] = k_stage[warp][lane * 16 + (piece ^ (lane & 7))];
+    }
+    if (slot + 1 < kSlots && 32 * (slot + 1) < candidates) {
+      __syncwarp();  // the rows have been read; the next ones come while these are scored
+      fetch(found[slot + 1 < kSlots ? slot + 1 : slot]);
+    }
+    const int j = found[slot];
+    if (j < 0) {
+      continue;
     }
     float score = -INFINITY;
     for (int g = 0; g < group; ++g) {
@@ -775,7 +791,7 @@ __global__ void __launch_bounds__(128) exact_edges_kernel(const ckv_prefill_args
   const int64_t out_base = ((static_cast<int64_t>(batch) * a.kv_heads + kv_head) * rows + (pos - skip)) *
                            a.edges_per_row;
   float last_score = 0.f;
-  if (candidates <= 32) {
+  if constexpr (kSlots == 1) {
     // bitonic sort over the lanes, the largest first
     uint64_t key = best_key[0];
 #pragma unroll
@@ -797,13 +813,13 @@ __global__ void __launch_bounds__(128) exact_edges_kernel(const ckv_prefill_args
     for (int rank = 0; rank < a.edges_per_row; ++rank) {
       uint64_t local = 0ull;
 #pragma unroll
-      for (int slot = 0; slot < 4; ++slot) {
+      for (int slot = 0; slot < kSlots; ++slot) {
         local = best_key[slot] > local ? best_key[slot] : local;
       }
       const uint64_t winner = warp_max_u64(local);
       if (winner != 0ull) {
 #pragma unroll
-        for (int slot = 0; slot < 4; ++slot) {
+        for (int slot = 0; slot < kSlots; ++slot) {
           best_key[slot] = best_key[slot] == winner ? 0ull : best_key[slot];
         }
       }
@@ -1450,7 +1466,14 @@ cudaError_t launch_prefill(const ckv_prefill_args& a, cudaStream_t stream) {
   }
   const int64_t items = static_cast<int64_t>(a.batch) * a.kv_heads * rows;
   const int lists = group == 2 || group == 4 ? 2 : group;
-  exact_edges_kernel<<<static_cast<unsigned>((items + 3) / 4), 128, 0, stream>>>(a, group, lists);
+  const unsigned edge_grid = static_cast<unsigned>((items + 3) / 4);
+  if (lists * kExactKeep <= 32) {
+    exact_edges_kernel<1, 5><<<edge_grid, 128, 0, stream>>>(a, group, lists);
+  } else if (edge_grid <= 3 * 148) {
+    exact_edges_kernel<4, 3><<<edge_grid, 128, 0, stream>>>(a, group, lists);
+  } else {
+    exact_edges_kernel<4, 5><<<edge_grid, 128, 0, stream>>>(a, group, lists);
+  }
   err = cudaGetLastError();
   if (err != cudaSuccess || a.edge_flags == nullptr) {
     return err;

@@ -145,6 +145,19 @@ def test_reference_topk_rule_short_and_ragged(length, heads, kv_heads, sinks):
                 assert abs(int(keys[position, j]) - int(floor_key)) <= 1, (head, row, j)
 
 
+@pytest.mark.parametrize("length,kv_heads", [(35, 1), (462, 4), (463, 4), (700, 4)])
+def test_exact_edges_of_eight_heads_per_group(length, kv_heads):
+    """Four rounds of candidates per row, on both sides of the line between few rows and many (444 CTAs of four)."""
+
+    sinks, edges = 4, 16
+    q, k, v = _inputs(19, length, 8 * kv_heads, kv_heads)
+    _, _, edge_idx, edge_score, _ = prefill_attention_edges(
+        q.cuda(), k.cuda(), v.cuda(), softmax_scale=SCALE, num_sink=sinks, edges_per_row=edges)
+    want_idx, want_score = oracle.exact_edges(q[0].float().numpy(), k[0].float().numpy(), SCALE, sinks, edges)
+    assert np.array_equal(edge_idx[0].cpu().numpy(), want_idx)
+    assert np.array_equal(edge_score[0].cpu().numpy().view(np.uint32), want_score.view(np.uint32))
+
+
 def test_exact_edges_of_a_prompt_shorter_than_the_list():
     q, k, v = _inputs(7, 12, 4, 2)
     out, lse, edge_idx, edge_score, flags = prefill_attention_edges(
